@@ -16,7 +16,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_lib")
 BUILD_DIR = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT_DIR, "libnyles_gb300.so")
-SOURCES = ["nyles_stencil.cu", "nyles_mg.cu", "nyles_model.cu"]
+SOURCES = ["nyles_stencil.cu", "nyles_line.cu", "nyles_mg.cu", "nyles_model.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
          "-I" + os.path.join(os.path.dirname(HERE), "include")]

@@ -63,6 +63,12 @@ template <typename T>
 int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const ProgPtrs<T>& ds, int terms,
                cudaStream_t st, bool interior = false, const Bat& bat = Bat());
 
+// FP64: the WENO tracer and vortex-force tendencies (TERM_TRACER, TERM_VF, TERM_TRDIFF of
+// `terms`), direction by direction (nyles_line.cu). Tracer registers are set, the vortex
+// force is added to the velocity registers.
+int launch_rhs_lines(const NylesDesc* d, const Geom& g, const StencilPtrs<double>& s, const ProgPtrs<double>& ds,
+                     int terms, cudaStream_t st, bool interior);
+
 // time-scheme elementwise updates (core/timescheme.py:113-221)
 enum { UPD_EULER = 0, UPD_RK3_2 = 1, UPD_RK3_3 = 2, UPD_LF_PRED = 3, UPD_LF_FIRST = 4, UPD_LF_CORR = 5 };
 template <typename T>

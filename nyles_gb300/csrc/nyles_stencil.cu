@@ -107,29 +107,6 @@ __device__ __forceinline__ T lap1d(const T* __restrict__ u, const Geom& g, long 
     return fx - fxm;
 }
 
-// -(flux divergence) of one tracer at a cell, accumulated direction by direction in
-// the reference's order (x pass assigns, y and z passes add), core/tracer.py:59-72;
-// with `diff`, each direction's diffusion k[pass]*lap follows its advection
-// (core/tracer.py:74-76)
-template <typename T>
-__device__ __forceinline__ T tracer_rhs(const T* __restrict__ q, const T* const* U, const Geom& g, long long c,
-                                        const int* pos, bool diff, T kx, T ky, T kz) {
-    T acc = T(0);
-    for (int pass = 0; pass < 3; ++pass) {
-        const int d = 2 - pass;            // x, then y, then z
-        const int i = pos[d];
-        const T Fi = tr_flux(U[d], q, g, c, i, d);
-        if (i > 0) {
-            const T Fm = tr_flux(U[d], q, g, c - g.stride(d), i - 1, d);
-            acc = (acc + Fm) - Fi;
-        } else {
-            acc = acc - Fi;
-        }
-        if (diff) acc = acc + (pass == 0 ? kx : (pass == 1 ? ky : kz)) * lap1d(q, g, c, i, d);
-    }
-    return acc;
-}
-
 // ---------------------------------------------------------------- linear vortex force
 // The linear branch of core/fortran_vortex_force.f90 (direc :43-55, flip :121-133) with
 // core/interpolate.f90:3-112, which the reference never takes (`linear = .false.` at
@@ -225,62 +202,18 @@ __device__ __forceinline__ void vortex_force_cell(const RhsArgs<T>& a, long long
     }
 }
 
+// the vortex force alone, added to the velocity registers (FP32; FP64 for the linear branch)
 template <typename T>
-__global__ void __launch_bounds__(128) k_rhs(const RhsArgs<T> a) {
+__global__ void __launch_bounds__(128) k_vortex_force(const RhsArgs<T> a) {
     const Geom& g = a.g;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     const int z = blockIdx.z * blockDim.z + threadIdx.z;
     if (x >= g.N[2] || y >= g.N[1] || z >= g.N[0]) return;
     const long long c = g.at(z, y, x);
-    const int pos[3] = {z, y, x};
-    const bool acc = (a.terms & TERM_ACCUMULATE) != 0;
-
-    // ---- tracers: b first, then t0.. (core/tracer.py:59-72)
-    if (a.terms & TERM_TRACER) {
-        const T* Uxyz[3] = {a.U[2], a.U[1], a.U[0]};   // indexed by geometry axis z, y, x
-        for (int t = 0; t <= a.ntr; ++t) {
-            const T* q = (t == 0) ? a.b : a.tr[t - 1];
-            const int slot = (t == 0) ? 0 : 3 + t;
-            const bool diff = (a.terms & TERM_TRDIFF) && ((a.kmask >> t) & 1);
-            T v = tracer_rhs(q, Uxyz, g, c, pos, diff, a.kcoef[t][0], a.kcoef[t][1], a.kcoef[t][2]);
-            if (a.ds[slot]) a.ds[slot][c] = acc ? a.ds[slot][c] + v : v;
-        }
-    } else if (!acc) {
-        for (int t = 0; t <= a.ntr; ++t) {
-            const int slot = (t == 0) ? 0 : 3 + t;
-            if (a.ds[slot]) a.ds[slot][c] = T(0);
-        }
-    }
-
-    // ---- velocity
-    if (!(a.terms & (TERM_VF | TERM_BERNOULLI | TERM_VISC)) && acc) return;
-    T dux = acc ? a.ds[1][c] : T(0);
-    T duy = acc ? a.ds[2][c] : T(0);
-    T duz = acc ? a.ds[3][c] : T(0);
-    const int Nz = g.N[0], Ny = g.N[1], Nx = g.N[2];
-    if (a.terms & TERM_VF) {
-        if (a.vf_order) vortex_force_cell<T, 2>(a, c, z, y, x, dux, duy, duz);
-        else vortex_force_cell<T, 1>(a, c, z, y, x, dux, duy, duz);
-    }
-    if (a.terms & TERM_BERNOULLI) {   // core/bernoulli.py:14-23
-        const T* ke = a.ke;
-        if (x < Nx - 1) dux = sub_rn(dux, sub_rn(__ldg(ke + c + 1), __ldg(ke + c)));
-        if (y < Ny - 1) duy = sub_rn(duy, sub_rn(__ldg(ke + c + g.sy), __ldg(ke + c)));
-        if (z < Nz - 1) {
-            duz = sub_rn(duz, sub_rn(__ldg(ke + c + g.sz), __ldg(ke + c)));
-            if (!a.euler) duz = add_rn(duz, mul_rn(a.half_dz, add_rn(__ldg(a.b + c + g.sz), __ldg(a.b + c))));
-        }
-    }
-    if (a.terms & TERM_VISC) {   // core/viscosity.py:5-9: direction outer, component inner
-        for (int pass = 0; pass < 3; ++pass) {
-            const int d = 2 - pass;
-            const T cf = a.vcoef[pass];
-            dux = dux + cf * lap1d(a.u[0], g, c, pos[d], d);
-            duy = duy + cf * lap1d(a.u[1], g, c, pos[d], d);
-            duz = duz + cf * lap1d(a.u[2], g, c, pos[d], d);
-        }
-    }
+    T dux = a.ds[1][c], duy = a.ds[2][c], duz = a.ds[3][c];
+    if (sizeof(T) == sizeof(float) && !a.vf_order) vortex_force_cell<T, 1>(a, c, z, y, x, dux, duy, duz);
+    else vortex_force_cell<T, 2>(a, c, z, y, x, dux, duy, duz);
     a.ds[1][c] = dux;
     a.ds[2][c] = duy;
     a.ds[3][c] = duz;
@@ -290,8 +223,8 @@ __global__ void __launch_bounds__(128) k_rhs(const RhsArgs<T> a) {
 // The full right-hand side with tracer face fluxes shared between the two cells of
 // each face: along x through a warp shuffle (one warp = one x row of 32 cells), along
 // y through shared memory, along z carried in a register while the thread marches up
-// its column chunk. One WENO5 per direction and tracer per cell instead of two; same
-// arithmetic and accumulation order as k_rhs.
+// its column chunk. One WENO5 per direction and tracer per cell instead of two. FP32, and
+// in FP64 the terms without WENO reconstructions (those march along lines, nyles_line.cu).
 constexpr int RZ_BX = 32, RZ_BY = 8, RZ_ZC = 16;
 
 template <typename T>
@@ -897,9 +830,14 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
         a.kcoef[q][1] = T(d->tracer_diffusivity[q] * d->idy2);
         a.kcoef[q][2] = T(d->tracer_diffusivity[q] * d->idz2);
     }
+    if constexpr (sizeof(T) == sizeof(double)) {   // WENO in FP64: by lines
+        if ((terms & TERM_ACCUMULATE) && d->vf_order == 0) return launch_rhs_lines(d, g, s, ds, TERM_VF, st, interior);
+        if (d->model == NYLES_MODEL_ADVECTION && d->tracer_order == 0)
+            return launch_rhs_lines(d, g, s, ds, terms, st, false);
+    }
     if (terms & TERM_ACCUMULATE) {   // add into existing registers (vortex force alone)
         dim3 blk(32, 2, 2);
-        k_rhs<T><<<grid3(g, blk), blk, 0, st>>>(a);
+        k_vortex_force<T><<<grid3(g, blk), blk, 0, st>>>(a);
         note_launch();
         return cuda_status(cudaGetLastError(), "rhs kernel");
     }
@@ -921,7 +859,7 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
         // are not touched (the reference never writes them)
         if (order > 0) {
             tracer_linear(a.b, a.ds[0], 0);
-        } else {
+        } else if constexpr (sizeof(T) == sizeof(float)) {
             const T* kc = a.kcoef[0];
             if ((terms & TERM_TRDIFF) && (d->tracer_diffusion & 1))
                 k_tracer_march<T, true><<<grd, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], a.b, a.ds[0], kc[0], kc[1],
@@ -938,6 +876,25 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
     const bool tr = (terms & TERM_TRACER) != 0, vf = (terms & TERM_VF) != 0;
     const bool bdiff = tr && (terms & TERM_TRDIFF) && (d->tracer_diffusion & 1);
     const bool lin = vf && d->vf_order > 0;
+    if constexpr (sizeof(T) == sizeof(double)) {
+        // the terms without a reconstruction (and the linear vortex force) set the
+        // registers, then the lines add theirs
+        if (bat.tab) {
+            set_error("batched right-hand side: single precision only");
+            return NYLES_UNSUPPORTED;
+        }
+        if (lin) k_rhs_march<T, false, 2, false><<<grd_box, blk, 0, st>>>(a);
+        else k_rhs_march<T, false, 0, false><<<grd_box, blk, 0, st>>>(a);
+        note_launch();
+        if (linear_tr) {
+            tracer_linear(a.b, a.ds[0], 0);
+            for (int t = 0; t < d->n_tracers; ++t) tracer_linear(a.tr[t], a.ds[4 + t], t + 1);
+        } else if (!tr) {   // Euler3d: tracers are not advected, their tendency is zero (reset_state)
+            for (int t = 0; t < d->n_tracers; ++t) cudaMemsetAsync(a.ds[4 + t], 0, sizeof(T) * g.vol, st);
+        }
+        const int line_terms = (tr ? terms & (TERM_TRACER | TERM_TRDIFF) : 0) | (vf && !lin ? TERM_VF : 0);
+        return launch_rhs_lines(d, g, s, ds, line_terms, st, interior);
+    } else {
     if (bat.tab) {   // batched: buoyancy advection, WENO vortex force, no buoyancy diffusion
         if (!(tr && vf && !bdiff && !lin && !linear_tr && d->n_tracers == 0 && d->model != NYLES_MODEL_ADVECTION)) {
             set_error("batched right-hand side: only buoyancy advection with the WENO vortex force and no tracers");
@@ -981,6 +938,7 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
         }
     }
     return cuda_status(cudaGetLastError(), "rhs kernel");
+    }
 }
 
 // ---------------------------------------------------------------- time-scheme updates
