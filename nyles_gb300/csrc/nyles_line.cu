@@ -224,11 +224,14 @@ __global__ void __launch_bounds__(LINE_THREADS) k_line(const __grid_constant__ L
 }
 
 // Cells per thread: every chunk starts with the six loads and four nodes of its first face
-// (about 30 FP64 instructions, 3/4 of a flux), so chunks are long, unless they leave the
-// chip without the ~8 warps per SM that keep its FP64 pipe busy.
+// (about 30 FP64 instructions, 3/4 of a flux), so chunks are long, until they leave fewer
+// than 24 warps per SM, which then end unevenly. Measured, chunks of 8 / 16 / 32 / 64: the
+// 109 x 75 x 53 right-hand side 614 / 644 / 706 us (16 cells: 23 warps per SM), a 128 x 64 x 64
+// LFAM3 step 2.53 / 2.50 / 2.65 ms (16 cells: 29 warps per SM), a 256^3 RK3 step - / 86.7 / 85.4 /
+// 85.3 ms; below 8 nothing is gained (64 x 32 x 32: 4, 6, 8, 12 cells within 3%).
 static int line_chunk(long long lines, int n) {
-    int chunk = 32;
-    while (chunk > 4 && lines * ((n + chunk - 1) / chunk) < 152ll * 8 * 32) chunk /= 2;
+    int chunk = 64;
+    while (chunk > 8 && lines * ((n + chunk - 1) / chunk) < 152ll * 24 * 32) chunk /= 2;
     return chunk;
 }
 

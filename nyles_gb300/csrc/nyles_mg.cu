@@ -16,6 +16,7 @@
 // neighbours all lie inside the level takes a fast path with direct strided loads;
 // only blocks touching the level's faces go through the ghost logic.
 #include "nyles_internal.h"
+#include "nyles_fx.cuh"
 #include <cstdlib>
 #include <vector>
 #include <cstring>
@@ -342,7 +343,7 @@ __device__ __forceinline__ void fcg_set_alpha(double pq, double pr, double* sc) 
 // and out per block into `partial` and `partial2` (the Krylov solve: z.q of the new
 // preconditioned residual against the previous direction's image, and the sum of z).
 // BAT: batched launch over the runs of `bat` (pointers shifted to each run's memory)
-template <typename T, int MODE, bool BAT = false>
+template <typename T, int MODE, bool BAT = false, int ZC = MG_ZC>
 __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_jacobi(const MgGeom g, const T* __restrict__ in,
                                                             const T* __restrict__ b, T* __restrict__ out, T omega,
                                                             float2* __restrict__ acc, const T* __restrict__ dot,
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_jacobi(const MgGeom g, con
     const int y = blockIdx.y * MG_BY + threadIdx.y;
     float sdot = 0.f, ssum = 0.f;
     if (x < g.n[2] && y < g.n[1]) {
-        const int nz = g.n[0], z0 = bz * MG_ZC;
+        const int nz = g.n[0], z0 = bz * ZC;
         const long long sy = g.n[2], sz = (long long)g.n[1] * g.n[2];
         const MgNb nx = mg_nb(x, g.n[2], g.per[2], 1), ny = mg_nb(y, g.n[1], g.per[1], sy);
         const int dxy = (int)nx.wm + (int)nx.wp + (int)ny.wm + (int)ny.wp;
@@ -388,23 +389,20 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_jacobi(const MgGeom g, con
                 }
             }
         };
-        if (z0 + MG_ZC <= nz) {
+        if (z0 + ZC <= nz) {
             // full chunk: fixed trip count, fully unrolled, so that every load of the chunk
             // is issued before the first result is needed
-            const MgNb lo = mg_nb(z0, nz, g.per[0], sz), hi = mg_nb(z0 + MG_ZC - 1, nz, g.per[0], sz);
-            T col[MG_ZC + 2];
+            const MgNb lo = mg_nb(z0, nz, g.per[0], sz), hi = mg_nb(z0 + ZC - 1, nz, g.per[0], sz);
+            T col[ZC + 2];
             col[0] = mg_ldw(in, c0 + lo.om, lo.wm);
 #pragma unroll
-            for (int k = 1; k <= MG_ZC; ++k) col[k] = in[c0 + (k - 1) * sz];
-            col[MG_ZC + 1] = mg_ldw(in, c0 + (MG_ZC - 1) * sz + hi.op, hi.wp);
-            const T idg = mg_idiag<T>(g, dxy + 2);
-            const T idg_lo = mg_idiag<T>(g, dxy + 1 + (int)lo.wm);
-            const T idg_hi = mg_idiag<T>(g, dxy + 1 + (int)hi.wp);
+            for (int k = 1; k <= ZC; ++k) col[k] = in[c0 + (k - 1) * sz];
+            col[ZC + 1] = mg_ldw(in, c0 + (ZC - 1) * sz + hi.op, hi.wp);
 #pragma unroll
-            for (int k = 0; k < MG_ZC; ++k) {
+            for (int k = 0; k < ZC; ++k) {
                 const long long c = c0 + k * sz;
-                put(c, cell(c, col[k], col[k + 1], col[k + 2], k == 0 ? idg_lo : (k == MG_ZC - 1 ? idg_hi : idg)),
-                    (MODE == 2) ? dot[c] : T(0));
+                const int dg = dxy + (k == 0 ? (int)lo.wm : 1) + (k == ZC - 1 ? (int)hi.wp : 1);
+                put(c, cell(c, col[k], col[k + 1], col[k + 2], mg_idiag<T>(g, dg)), (MODE == 2) ? dot[c] : T(0));
             }
         } else {
             for (int z = z0; z < nz; ++z) {   // last, partial chunk
@@ -568,7 +566,7 @@ __device__ __forceinline__ T mg_jacobi_from_zero(T b, T omega, T idg) {
 // bc = Rcoef*(sum of the 8 children) with Rcoef = 1/2 (basicoperators.f90:32-60,
 // operators.f90:172-213). The coarse solution is zero at this point (operators.f90:209),
 // so the first half-sweep of the coarse smoothing is written here, into yc.
-template <typename T, bool BAT = false>
+template <typename T, bool BAT = false, int RZC = MG_RZC>
 __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_restrict(const MgGeom gf, const T* __restrict__ xf,
                                                               const T* __restrict__ bf, const MgGeom gc,
                                                               T* __restrict__ bc, T* __restrict__ yc, T omega,
@@ -585,14 +583,14 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_restrict(const MgGeom gf, 
     const int x = blockIdx.x * MG_BX + threadIdx.x;
     const int y = blockIdx.y * MG_BY + threadIdx.y;
     if (x >= gc.n[2] || y >= gc.n[1]) return;
-    const int nzc = gc.n[0], z0 = bz * MG_RZC;
+    const int nzc = gc.n[0], z0 = bz * RZC;
     auto emit = [&](int z, T s) {
         const long long c = mg_at(gc, z, y, x);
         const T bv = T(0.5) * s;
         bc[c] = bv;
         yc[c] = mg_jacobi_from_zero(bv, omega, mg_idiag<T>(gc, mg_diag(gc, z, y, x)));
     };
-    if (z0 + MG_RZC > nzc) {   // last, partial chunk
+    if (z0 + RZC > nzc) {   // last, partial chunk
         for (int z = z0; z < nzc; ++z) emit(z, mg_restrict_cell(gf, xf, bf, z, y, x));
         return;
     }
@@ -604,12 +602,12 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_restrict(const MgGeom gf, 
     const int i0 = 2 * x, j0 = 2 * y, k0 = 2 * z0;
     const MgNb xl = mg_nb(i0, gf.n[2], gf.per[2], 1), xh = mg_nb(i0 + 1, gf.n[2], gf.per[2], 1);
     const MgNb yl = mg_nb(j0, gf.n[1], gf.per[1], sy), yh = mg_nb(j0 + 1, gf.n[1], gf.per[1], sy);
-    const MgNb zl = mg_nb(k0, gf.n[0], gf.per[0], sz), zh = mg_nb(k0 + 2 * MG_RZC - 1, gf.n[0], gf.per[0], sz);
+    const MgNb zl = mg_nb(k0, gf.n[0], gf.per[0], sz), zh = mg_nb(k0 + 2 * RZC - 1, gf.n[0], gf.per[0], sz);
     // wet x/y neighbours of the children (j0,i0), (j0,i1), (j1,i0), (j1,i1)
     const int dxy[4] = {(int)xl.wm + 1 + (int)yl.wm + 1, 1 + (int)xh.wp + (int)yl.wm + 1,
                         (int)xl.wm + 1 + 1 + (int)yh.wp, 1 + (int)xh.wp + 1 + (int)yh.wp};
     const long long cb = mg_at(gf, k0, j0, i0);
-    constexpr int NP = 2 * MG_RZC + 2;   // fine planes k0-1 .. k0+2*RZC
+    constexpr int NP = 2 * RZC + 2;   // fine planes k0-1 .. k0+2*RZC
     T v[NP][4];
     auto ld4 = [&](long long c, bool wet, T* o) {
         o[0] = mg_ldw(xf, c, wet);
@@ -620,7 +618,7 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_restrict(const MgGeom gf, 
     ld4(cb + zl.om, zl.wm, v[0]);
 #pragma unroll
     for (int q = 1; q < NP - 1; ++q) ld4(cb + (q - 1) * sz, true, v[q]);
-    ld4(cb + (2 * MG_RZC - 1) * sz + zh.op, zh.wp, v[NP - 1]);
+    ld4(cb + (2 * RZC - 1) * sz + zh.op, zh.wp, v[NP - 1]);
     // The 8 residuals b + diag*x - sum(x_nb) summed at once: each child's 6 neighbours
     // are 3 siblings and 3 cells outside the 2 x 2 x 2 block, so the sum is
     // sum(b) + sum(w_c x_c) - sum(24 outside cells) with w_c = diag_c - 3, the child's wet
@@ -628,7 +626,7 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_restrict(const MgGeom gf, 
     // to rounding, with 2/3 of their FP64 instructions.
     const T wxy[4] = {T(dxy[0] - 2), T(dxy[1] - 2), T(dxy[2] - 2), T(dxy[3] - 2)};
 #pragma unroll
-    for (int zc = 0; zc < MG_RZC; ++zc) {
+    for (int zc = 0; zc < RZC; ++zc) {
         T sb = T(0), sx = T(0), so = T(0);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -677,7 +675,7 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_prolong(const MgGeom gf, T
         return;
     }
     // Full chunk, unrolled: the in-plane 9-3-3-1 sums of the coarse planes z0/2-1 ..
-    // z0/2+ZC/2 (each used by two fine planes) are formed once; a coarse neighbour
+    // z0/2+MG_ZC/2 (each used by two fine planes) are formed once; a coarse neighbour
     // outside the level is the periodic image or 0.
     const int ic = x >> 1, jc = y >> 1;
     const long long csy = gc.n[2], csz = (long long)gc.n[1] * gc.n[2];
@@ -711,6 +709,77 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_prolong(const MgGeom gf, T
         const T bpl = P[m], opl = P[(k & 1) ? m + 1 : m - 1];
         const T pc = (k == 0) ? pc_lo : (k == MG_ZC - 1 ? pc_hi : pc_wet);
         xf[c0 + k * sz] = xv[k] + pc * (T(3) * bpl + opl);
+    }
+}
+
+// The FP64 prolongation, one coarse column per thread: the 8 fine cells of a coarse cell share
+// the x interpolations of its three coarse rows and the y interpolations of each plane, 26
+// FP64 instructions for 8 cells where the per-fine-column form (k_mg_prolong) takes 40: 215 ->
+// 127 us into 256^3, 28 -> 21 us into 128^3, FP64-bound. CZ coarse planes per thread; fine extents are
+// twice the coarse ones (every FP64 level: only the coarsest may have odd extents).
+template <int CZ>
+__global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_prolong_f64(const MgGeom gf, double* __restrict__ xf,
+                                                                 const MgGeom gc, const double* __restrict__ xc) {
+    const int x = blockIdx.x * MG_BX + threadIdx.x;
+    const int y = blockIdx.y * MG_BY + threadIdx.y;
+    if (x >= gc.n[2] || y >= gc.n[1]) return;
+    const int nzc = gc.n[0], k0 = blockIdx.z * CZ, k1 = min(k0 + CZ, nzc);
+    const long long csy = gc.n[2], csz = (long long)gc.n[1] * gc.n[2];
+    const MgNb cx = mg_nb(x, gc.n[2], gc.per[2], 1), cy = mg_nb(y, gc.n[1], gc.per[1], csy);
+    const double* __restrict__ col = xc + mg_at(gc, 0, y, x);
+    struct Plane { double v[2][2]; };   // [y low/high][x low/high]
+    auto plane = [&](int k) -> Plane {
+        bool wet = true;
+        if (k < 0 || k >= nzc) {
+            wet = gc.per[0] != 0;
+            k = k < 0 ? nzc - 1 : 0;
+        }
+        const double* p = col + (long long)k * csz;
+        double lo[3], hi[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const long long o = j == 0 ? cy.om : (j == 1 ? 0 : cy.op);
+            const bool w = wet && (j == 0 ? cy.wm : (j == 1 ? true : cy.wp));
+            const double a = mg_ldw(p, o, w), l = mg_ldw(p, o + cx.om, w && cx.wm), r = mg_ldw(p, o + cx.op, w && cx.wp);
+            lo[j] = fma(3.0, a, l);
+            hi[j] = fma(3.0, a, r);
+        }
+        Plane q;
+        q.v[0][0] = fma(3.0, lo[1], lo[0]);
+        q.v[0][1] = fma(3.0, hi[1], hi[0]);
+        q.v[1][0] = fma(3.0, lo[1], lo[2]);
+        q.v[1][1] = fma(3.0, hi[1], hi[2]);
+        return q;
+    };
+    const long long fsy = gf.n[2], fsz = (long long)gf.n[1] * gf.n[2];
+    double* __restrict__ f0 = xf + mg_at(gf, 0, 2 * y, 2 * x);
+    Plane m = plane(k0 - 1), c = plane(k0);
+#pragma unroll
+    for (int kk = 0; kk < CZ; ++kk) {
+        const int k = k0 + kk;
+        if (k >= k1) break;
+        double2 old[2][2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                old[h][j] = *reinterpret_cast<const double2*>(f0 + (2 * k + h) * fsz + j * fsy);
+        const Plane p = plane(k + 1);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int wz = (h == 0 ? k > 0 : k < nzc - 1) || gc.per[0] ? 4 : 0;
+            const Plane& o = h == 0 ? m : p;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int wy = (j == 0 ? cy.wm : cy.wp) ? 2 : 0;
+                double2 r = old[h][j];
+                r.x = fma(gf.pcoef[(int)cx.wm | wy | wz], fma(3.0, c.v[j][0], o.v[j][0]), r.x);
+                r.y = fma(gf.pcoef[(int)cx.wp | wy | wz], fma(3.0, c.v[j][1], o.v[j][1]), r.y);
+                *reinterpret_cast<double2*>(f0 + (2 * k + h) * fsz + j * fsy) = r;
+            }
+        }
+        m = c;
+        c = p;
     }
 }
 
@@ -1217,13 +1286,13 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_sumsq(const MgGeom g, cons
 // next V-cycle: both need the same neighbour sum, so one pass gives sum(r^2) (same
 // partials, same order as k_mg_sumsq MODE 1) and y = (1-omega)*x + omega*(sum - b)*idiag.
 // If the solve then stops, y is simply not used.
-template <typename T>
+template <typename T, int ZC = MG_ZC>
 __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_resid_sweep(const MgGeom g, const T* __restrict__ v,
                                                                  const T* __restrict__ b, T* __restrict__ y_out,
                                                                  T omega, double* __restrict__ partial) {
     const int x = blockIdx.x * MG_BX + threadIdx.x;
     const int y = blockIdx.y * MG_BY + threadIdx.y;
-    const int nz = g.n[0], z0 = blockIdx.z * MG_ZC;
+    const int nz = g.n[0], z0 = blockIdx.z * ZC;
     (void)omega;   // the tables hold omega/diag
     double s = 0.0;
     if (x < g.n[2] && y < g.n[1]) {
@@ -1240,17 +1309,17 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_resid_sweep(const MgGeom g
             // (1-omega)x + omega(nsum - b)/diag = x - (omega/diag) r
             y_out[c] = x0 - mg_idiag<T>(g, dg) * r;
         };
-        if (z0 + MG_ZC <= nz) {
-            const MgNb lo = mg_nb(z0, nz, g.per[0], sz), hi = mg_nb(z0 + MG_ZC - 1, nz, g.per[0], sz);
-            T col[MG_ZC + 2];
+        if (z0 + ZC <= nz) {
+            const MgNb lo = mg_nb(z0, nz, g.per[0], sz), hi = mg_nb(z0 + ZC - 1, nz, g.per[0], sz);
+            T col[ZC + 2];
             col[0] = mg_ldw(v, c0 + lo.om, lo.wm);
 #pragma unroll
-            for (int k = 1; k <= MG_ZC; ++k) col[k] = v[c0 + (k - 1) * sz];
-            col[MG_ZC + 1] = mg_ldw(v, c0 + (MG_ZC - 1) * sz + hi.op, hi.wp);
+            for (int k = 1; k <= ZC; ++k) col[k] = v[c0 + (k - 1) * sz];
+            col[ZC + 1] = mg_ldw(v, c0 + (ZC - 1) * sz + hi.op, hi.wp);
 #pragma unroll
-            for (int k = 0; k < MG_ZC; ++k)
+            for (int k = 0; k < ZC; ++k)
                 cell(c0 + k * sz, col[k], col[k + 1], col[k + 2],
-                     dxy + (k == 0 ? 1 + (int)lo.wm : (k == MG_ZC - 1 ? 1 + (int)hi.wp : 2)));
+                     dxy + (k == 0 ? (int)lo.wm : 1) + (k == ZC - 1 ? (int)hi.wp : 1));
         } else {
             for (int z = z0; z < nz; ++z) {
                 const long long c = c0 + (z - z0) * sz;
@@ -1261,6 +1330,196 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_resid_sweep(const MgGeom g
         }
     }
     block_partial(s, partial, blockIdx.z);
+}
+
+// ---------------------------------------------------------------- FP64 levels on the integer pipes
+// What the V-cycle does to a level is a sum over a cell and its neighbours: a half-sweep is
+// (1-omega) x + (omega/diag) (sum(x_nb) - b), the stop test and the restriction need the residual
+// r = b + diag*x - sum(x_nb). In doubles the sum is 6 FP64 instructions of a half-sweep's 8, at
+// 2 lanes per cycle and SM; here it is a sum of 64-bit integers (nyles_fx.cuh), about 110 integer
+// instructions per cell with the conversions, and 2 FP64 instructions are left. Bound by the integer
+// pipe (64% busy; FP64 26%, memory 25%). Measured against the double kernels (k_mg_jacobi,
+// k_mg_resid_sweep, k_mg_restrict in 8-cell columns) per launch: 128^3 38 -> 17, 44 -> 20 and
+// 37 -> 17 us; 256^3 step with the transfer below 142 -> 85.4 ms.
+// A block owns 32 x 8 columns of ZC cells, one column per thread: every value of the tile
+// and of the ring around it is loaded first, the block agrees on the exponent, and the
+// converted columns meet in shared memory. Ghosts: 0 across a wall, else the periodic image.
+// Tiles that the level cuts off are summed in doubles, as those of too wide a range.
+// MODE 0: out = x - (omega/diag) r. MODE 1: also the block's sum of r^2. MODE 2: the coarse
+// right-hand side 0.5 * (sum of r over the 8 children) and its first half-sweep (k_mg_restrict);
+// fine extents are twice the coarse ones.
+
+// r of the thread's column in doubles (any tile); MODE 2: the sums over the pairs in z and x
+// go to `sums` [ZC/2][BY][BX/2] as bit patterns of doubles
+template <int ZC, int MODE>
+__device__ __noinline__ double fx_tile_double(const MgGeom& g, const double* __restrict__ v, const double* __restrict__ b,
+                                              double* __restrict__ out, int x, int y, int zb, long long* sums) {
+    const bool act = x < g.n[2] && y < g.n[1];
+    double s = 0.0, pair = 0.0;
+    for (int k = 0; k < ZC; ++k) {
+        const int z = zb + k;
+        double r = 0.0;
+        if (act && z < g.n[0]) {
+            const long long c = mg_at(g, z, y, x);
+            const double xc = v[c];
+            const int dg = mg_diag(g, z, y, x);
+            r = fma((double)dg, xc, b[c]) - mg_nsum(v, g, z, y, x);
+            if (MODE == 0) out[c] = fma(g.idiag[dg], mg_nsum(v, g, z, y, x) - b[c], (1.0 - g.idiag[1]) * xc);
+            else if (MODE == 1) out[c] = fma(-g.idiag[dg], r, xc);
+            if (MODE == 1) s = fma(r, r, s);
+        }
+        if (MODE == 2) {
+            pair = (k & 1) ? pair + r : r;
+            if (k & 1) {
+                const double w = pair + __shfl_down_sync(0xffffffffu, pair, 1);
+                if ((threadIdx.x & 1) == 0)
+                    sums[((k >> 1) * MG_BY + threadIdx.y) * (MG_BX / 2) + (threadIdx.x >> 1)] = __double_as_longlong(w);
+            }
+        }
+    }
+    return s;
+}
+
+template <int ZC, int MODE>
+__global__ void __launch_bounds__(MG_BX * MG_BY, 3) k_mg_fx(const MgGeom g, const double* __restrict__ v,
+                                                           const double* __restrict__ b, double* __restrict__ out,
+                                                           double* __restrict__ partial, const MgGeom gc,
+                                                           double* __restrict__ bc) {
+    constexpr int BX = MG_BX, BY = MG_BY, NT = BX * BY;
+    __shared__ long long tile[ZC][BY + 2][BX + 2];
+    __shared__ unsigned int swarp[2][BY];
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * BX + tx;
+    const int nx = g.n[2], ny = g.n[1], nz = g.n[0];
+    const int xb = blockIdx.x * BX, yb = blockIdx.y * BY, zb = blockIdx.z * ZC;
+    const int x = xb + tx, y = yb + ty;
+    const long long sy = nx, sz = (long long)ny * nx;
+    long long* const sums = &tile[0][0][0];   // MODE 2: [ZC/2][BY][BX/2], after the tile has been read
+    double s = 0.0;
+    bool fx = xb + BX <= nx && yb + BY <= ny && zb + ZC <= nz;
+    int Eu = 0;
+    if (fx) {
+        const MgNb nlo = mg_nb(zb, nz, g.per[0], sz), nhi = mg_nb(zb + ZC - 1, nz, g.per[0], sz);
+        const MgNb ylo = mg_nb(yb, ny, g.per[1], sy), yhi = mg_nb(yb + BY - 1, ny, g.per[1], sy);
+        const MgNb xlo = mg_nb(xb, nx, g.per[2], 1), xhi = mg_nb(xb + BX - 1, nx, g.per[2], 1);
+        const long long c0 = ((long long)zb * ny + y) * nx + x;
+        const double* __restrict__ pv = v + c0;
+        const double* __restrict__ pb = b + c0;
+        double col[ZC + 2], bcol[ZC];
+#pragma unroll
+        for (int k = 0; k < ZC; ++k) col[k + 1] = pv[k * sz];
+        col[0] = nlo.wm ? pv[nlo.om] : 0.0;
+        col[ZC + 1] = nhi.wp ? pv[(ZC - 1) * sz + nhi.op] : 0.0;
+#pragma unroll
+        for (int k = 0; k < ZC; ++k) bcol[k] = pb[k * sz];
+        // the rows below and above the tile (2 ZC row segments over BY warps) and the
+        // columns beside it
+        constexpr int NHY = (2 * ZC + BY - 1) / BY, NHX = (2 * ZC * BY + NT - 1) / NT;
+        double hy[NHY], hx[NHX];
+#pragma unroll
+        for (int h = 0; h < NHY; ++h) {
+            const int q = ty + h * BY, pl = q >> 1;
+            const double* row = v + ((long long)(zb + pl) * ny + yb) * nx + x;
+            hy[h] = 0.0;
+            if (q < 2 * ZC && ((q & 1) ? yhi.wp : ylo.wm)) hy[h] = row[(q & 1) ? (BY - 1) * sy + yhi.op : ylo.om];
+        }
+#pragma unroll
+        for (int h = 0; h < NHX; ++h) {
+            const int q = tid + h * NT, pl = q / (2 * BY), yr = (q >> 1) % BY;
+            const double* row = v + ((long long)(zb + pl) * ny + yb + yr) * nx + xb;
+            hx[h] = 0.0;
+            if (q < 2 * ZC * BY && ((q & 1) ? xhi.wp : xlo.wm)) hx[h] = row[(q & 1) ? BX - 1 + xhi.op : xlo.om];
+        }
+        // the tile's exponent, and the smallest one among the threads' own values (with the
+        // neighbouring columns': a stencil next to a zero of x is as large as its neighbours)
+        unsigned int own = max(fx_mag(col[0]), fx_mag(col[ZC + 1]));
+#pragma unroll
+        for (int k = 0; k < ZC; ++k) own = max(own, max(fx_mag(col[k + 1]), fx_mag(bcol[k])));
+        unsigned int all = own;
+#pragma unroll
+        for (int h = 0; h < NHY; ++h) all = max(all, fx_mag(hy[h]));
+#pragma unroll
+        for (int h = 0; h < NHX; ++h) all = max(all, fx_mag(hx[h]));
+        own = max(own, max(__shfl_up_sync(0xffffffffu, own, 1), __shfl_down_sync(0xffffffffu, own, 1)));
+        all = __reduce_max_sync(0xffffffffu, all);
+        own = __reduce_min_sync(0xffffffffu, own ? own : 0x7fffffffu);
+        if (tx == 0) {
+            swarp[0][ty] = all;
+            swarp[1][ty] = own;
+        }
+        __syncthreads();
+        const int E = (int)(__reduce_max_sync(0xffffffffu, swarp[0][tx % BY]) >> 20);
+        const int Emin = (int)(__reduce_min_sync(0xffffffffu, swarp[1][tx % BY]) >> 20);
+        fx = E >= FX_EMIN && E < 0x7ff && E - Emin <= FX_RANGE;
+        // MODE 2: eight residuals stay below 2^63 in units eight times as large
+        Eu = MODE == 2 ? E + 3 : E;
+        if (fx) {
+            long long f[ZC + 2];
+#pragma unroll
+            for (int k = 0; k < ZC + 2; ++k) f[k] = fx_from(col[k], Eu);
+#pragma unroll
+            for (int k = 0; k < ZC; ++k) tile[k][ty + 1][tx + 1] = f[k + 1];
+#pragma unroll
+            for (int h = 0; h < NHY; ++h) {
+                const int q = ty + h * BY;
+                if (q < 2 * ZC) tile[q >> 1][(q & 1) ? BY + 1 : 0][tx + 1] = fx_from(hy[h], Eu);
+            }
+#pragma unroll
+            for (int h = 0; h < NHX; ++h) {
+                const int q = tid + h * NT;
+                if (q < 2 * ZC * BY) tile[q / (2 * BY)][((q >> 1) % BY) + 1][(q & 1) ? BX + 1 : 0] = fx_from(hx[h], Eu);
+            }
+            __syncthreads();
+            const int dxy = (int)(x > 0 || g.per[2]) + (int)(x < nx - 1 || g.per[2]) + (int)(y > 0 || g.per[1]) +
+                            (int)(y < ny - 1 || g.per[1]);
+            const double idg = MODE == 2 ? 0.0 : g.idiag[dxy + 2], cff1 = 1.0 - g.idiag[1];   // idiag[1] = omega
+            double* __restrict__ po = MODE == 2 ? nullptr : out + c0;
+            long long acc[MODE == 2 ? ZC / 2 : 1];
+#pragma unroll
+            for (int k = 0; k < ZC; ++k) {
+                const unsigned int dg = dxy + (k == 0 ? (int)nlo.wm : 1) + (k == ZC - 1 ? (int)nhi.wp : 1);
+                const long long sum = tile[k][ty + 1][tx] + tile[k][ty + 1][tx + 2] + tile[k][ty][tx + 1] +
+                                      tile[k][ty + 2][tx + 1] + f[k] + f[k + 2];
+                const long long bk = fx_round(bcol[k], Eu);
+                if (MODE == 0) {
+                    const double w = (k == 0 || k == ZC - 1) ? g.idiag[dg] : idg;
+                    po[k * sz] = fma(w, fx_to_double(sum - bk, Eu), cff1 * col[k + 1]);
+                } else {
+                    const long long r = bk + fx_mul(f[k + 1], dg) - sum;
+                    if (MODE == 2) {
+                        acc[k >> 1] = (k & 1) ? acc[k >> 1] + r : r;
+                    } else {
+                        const double rd = fx_to_double(r, Eu), w = (k == 0 || k == ZC - 1) ? g.idiag[dg] : idg;
+                        po[k * sz] = fma(-w, rd, col[k + 1]);
+                        s = fma(rd, rd, s);
+                    }
+                }
+            }
+            if (MODE == 2) {
+                __syncthreads();   // the tile has been read
+#pragma unroll
+                for (int k = 0; k < ZC / 2; ++k) {
+                    const long long w = acc[k] + __shfl_down_sync(0xffffffffu, acc[k], 1);
+                    if ((tx & 1) == 0) sums[(k * BY + ty) * (BX / 2) + (tx >> 1)] = w;
+                }
+            }
+        }
+    }
+    if (!fx) s = fx_tile_double<ZC, MODE>(g, v, b, out, x, y, zb, sums);
+    if (MODE == 1) block_partial(s, partial, blockIdx.z);
+    if (MODE == 2) {
+        __syncthreads();
+        for (int q = tid; q < (ZC / 2) * (BY / 2) * (BX / 2); q += NT) {
+            const int cx = q % (BX / 2), cy = (q / (BX / 2)) % (BY / 2), cz = q / (BX / 2 * (BY / 2));
+            const int X = xb / 2 + cx, Y = yb / 2 + cy, Z = zb / 2 + cz;
+            if (X >= gc.n[2] || Y >= gc.n[1] || Z >= gc.n[0]) continue;
+            const long long s0 = sums[(cz * BY + 2 * cy) * (BX / 2) + cx], s1 = sums[(cz * BY + 2 * cy + 1) * (BX / 2) + cx];
+            const double t = fx ? fx_to_double(s0 + s1, Eu) : __longlong_as_double(s0) + __longlong_as_double(s1);
+            const double bv = 0.5 * t;
+            const long long c = mg_at(gc, Z, Y, X);
+            bc[c] = bv;
+            out[c] = mg_jacobi_from_zero(bv, 0.0, mg_idiag<double>(gc, mg_diag(gc, Z, Y, X)));
+        }
+    }
 }
 
 // ---------------------------------------------------------------- mixed precision
@@ -1896,6 +2155,17 @@ static inline dim3 bgrid(const MgImpl* mg, dim3 g) {
     return g;
 }
 
+// FP64 levels: the integer-sum kernel where a level's 8-cell columns fill the chip; below,
+// the double kernels with one cell per thread (their launches last as long as one thread's
+// chain of FP64 instructions: 8 cells 9 us, 1 cell 4 us on 32^3 and 16^3). Measured with the line at
+// 2^15 / 2^18 / 2^19 cells / everything in doubles: a 128^3 solve 1.364 / 1.361 / 1.387 / 2.086 ms, a
+// 128 x 64 x 64 LFAM3 step 2.64 / 2.65 / 2.65 / 2.96 ms.
+constexpr int FX_ZC = 8;
+constexpr long long FX_MINVOL = 1ll << 18;
+static inline bool use_fx(const MgImpl* mg, int l) {
+    return mg->precision == NYLES_FP64 && mg->lev[l].vol >= FX_MINVOL;
+}
+
 // the 4-cell vector kernels apply to a level whose x and z extents allow them; zc = the
 // z cells per thread (V4_ZC on level 0 and for the float-pair and Krylov kernels,
 // lvl_zc below)
@@ -2096,7 +2366,7 @@ int mg_init(MgImpl* mg, int nx, int ny, int nz, int topology, int precision, int
         }
     }
     // one partial per block of the largest reduction grid (the float-pair residual's)
-    const dim3 g0 = grid_zc(mg->lev[0].n, MG_DFZC < MG_ZC ? MG_DFZC : MG_ZC);
+    const dim3 g0 = grid_zc(mg->lev[0].n, precision == NYLES_FP64 && !use_fx(mg, 0) ? 1 : (MG_DFZC < MG_ZC ? MG_DFZC : MG_ZC));
     mg->npartial = (int)(g0.x * g0.y * g0.z);
     {
         const char* e = getenv("NYLES_GB300_SCALAR_KERNELS");
@@ -2128,6 +2398,17 @@ static void smooth(MgImpl* mg, int l, cudaStream_t st, int last_mode, bool from_
     const T om = T(mg->omega);
     ProfScope ps(mg->prof, 8, st);
     note_launch(from_y ? 1 : 2);
+    if constexpr (sizeof(T) == sizeof(double)) {   // FP64: always stored (last_mode 0)
+        if (use_fx(mg, l)) {
+            const dim3 gx = grid_zc(g.n, FX_ZC);
+            if (!from_y) k_mg_fx<FX_ZC, 0><<<gx, kBlk, 0, st>>>(g, x, b, y, nullptr, g, nullptr);
+            k_mg_fx<FX_ZC, 0><<<gx, kBlk, 0, st>>>(g, y, b, x, nullptr, g, nullptr);
+        } else {
+            const dim3 gs = grid_zc(g.n, 1);
+            if (!from_y) k_mg_jacobi<T, 0, false, 1><<<gs, kBlk, 0, st>>>(g, x, b, y, om, nullptr, nullptr, nullptr, nullptr);
+            k_mg_jacobi<T, 0, false, 1><<<gs, kBlk, 0, st>>>(g, y, b, x, om, nullptr, nullptr, nullptr, nullptr);
+        }
+    } else {
     if (mg->bat.tab) {   // batched (stationary mixed refinement): modes 0 and 1
         const Bat& bt = mg->bat;
         float2* pdf = last_mode == 1 ? mg_pdf(mg) : nullptr;
@@ -2187,6 +2468,7 @@ static void smooth(MgImpl* mg, int l, cudaStream_t st, int last_mode, bool from_
                                                 reinterpret_cast<double*>(mg->ws + mg->off_partial2));
     else
         k_mg_jacobi<T, 0><<<grd, kBlk, 0, st>>>(g, y, b, x, om, nullptr, nullptr, nullptr, nullptr);
+    }
 }
 
 // solvers.f90:35-55
@@ -2241,7 +2523,16 @@ static void vcycle(MgImpl* mg, cudaStream_t st, int level0_last) {
                     done = true;
                 }
             }
-            if (!done && mg->bat.tab)
+            if constexpr (sizeof(T) == sizeof(double)) {
+                if (use_fx(mg, l))
+                    k_mg_fx<FX_ZC, 2><<<grid_zc(gf.n, FX_ZC), kBlk, 0, st>>>(gf, lvp<T>(mg, l, 1), lvp<T>(mg, l, 2),
+                                                                            lvp<T>(mg, l + 1, 3), nullptr, gc,
+                                                                            lvp<T>(mg, l + 1, 2));
+                else
+                    k_mg_restrict<T, false, 1><<<grid_zc(gc.n, 1), kBlk, 0, st>>>(
+                        gf, lvp<T>(mg, l, 1), lvp<T>(mg, l, 2), gc, lvp<T>(mg, l + 1, 2), lvp<T>(mg, l + 1, 3),
+                        T(mg->omega));
+            } else if (!done && mg->bat.tab)
                 k_mg_restrict<T, true><<<bgrid(mg, grid_zc(gc.n, MG_RZC)), kBlk, 0, st>>>(
                     gf, lvp<T>(mg, l, 1), lvp<T>(mg, l, 2), gc, lvp<T>(mg, l + 1, 2), lvp<T>(mg, l + 1, 3),
                     T(mg->omega), mg->bat);
@@ -2273,7 +2564,12 @@ static void vcycle(MgImpl* mg, cudaStream_t st, int level0_last) {
                     done = true;
                 }
             }
-            if (!done && mg->bat.tab)
+            if constexpr (sizeof(T) == sizeof(double)) {
+                if (use_fx(mg, l))   // enough columns for 4 coarse planes per thread
+                    k_mg_prolong_f64<4><<<grid_zc(gc.n, 4), kBlk, 0, st>>>(gf, lvp<T>(mg, l, 1), gc, lvp<T>(mg, l + 1, 1));
+                else
+                    k_mg_prolong_f64<1><<<grid_zc(gc.n, 1), kBlk, 0, st>>>(gf, lvp<T>(mg, l, 1), gc, lvp<T>(mg, l + 1, 1));
+            } else if (!done && mg->bat.tab)
                 k_mg_prolong<T, true><<<bgrid(mg, grid_zc(gf.n, MG_ZC)), kBlk, 0, st>>>(
                     gf, lvp<T>(mg, l, 1), gc, lvp<T>(mg, l + 1, 1), mg->bat);
             else if (!done)
@@ -2357,11 +2653,16 @@ static void enqueue_resid_sweep(MgImpl* mg, cudaStream_t st) {
     MgGeom g = mgg(mg, 0);
     double* part = reinterpret_cast<double*>(mg->ws + mg->off_partial);
     double* sc = reinterpret_cast<double*>(mg->ws + mg->off_scalars);
-    const dim3 grd = grid_zc(g.n, MG_ZC);
+    const bool fx = use_fx(mg, 0);
+    const dim3 grd = grid_zc(g.n, fx ? FX_ZC : 1);
     ProfScope ps(mg->prof, 11, st);
     note_launch(2);
-    k_mg_resid_sweep<double><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2),
-                                                   lvp<double>(mg, 0, 3), mg->omega, part);
+    if (fx)
+        k_mg_fx<FX_ZC, 1><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2), lvp<double>(mg, 0, 3),
+                                                part, g, nullptr);
+    else
+        k_mg_resid_sweep<double, 1><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2),
+                                                          lvp<double>(mg, 0, 3), mg->omega, part);
     k_mg_final<<<1, 1024, 0, st>>>(part, (int)(grd.x * grd.y * grd.z), sc + SC_RR);
 }
 
