@@ -17,6 +17,8 @@
 // only blocks touching the level's faces go through the ghost logic.
 #include "nyles_internal.h"
 #include "nyles_fx.cuh"
+#include <cooperative_groups.h>
+#include <type_traits>
 #include <cstdlib>
 #include <vector>
 #include <cstring>
@@ -1001,230 +1003,405 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_prolong_v4(const MgGeom gf
     mg_prolong_v4_blk<ZC>(gf, xf, gc, xc, blockIdx.x, blockIdx.y, bz);
 }
 
-// ---------------------------------------------------------------- coarse levels in one block
+// ---------------------------------------------------------------- coarse levels in one cluster
 // Levels l0..L-1 of a V-cycle (solvers.f90:35-55 from level l0 down and back up) run in
-// one thread block: the level arrays live in shared memory, and each half-sweep,
-// restriction and prolongation is one pass of the block over a level followed by a
-// barrier, instead of one grid launch each. Input: b of level l0 (its x is zero after
-// the restriction that produced b); output: x of level l0. The per-cell arithmetic is
-// that of the grid kernels' ghost paths.
+// one cluster of BT_CTAS thread blocks: the level arrays live in shared memory, and each
+// half-sweep, restriction and prolongation is one pass followed by a barrier, instead of
+// one grid launch each. Input: b of level l0 (its x is zero after the restriction that
+// produced b); output: x of level l0. The per-cell arithmetic is that of the grid kernels.
+// The larger of these levels are cut into slabs of z planes, one per block (MgBottomLevel::pp
+// planes, an even number, so that a coarse plane's children are one block's); a pass
+// writes the planes its neighbours need into their shared memory, and the cluster's barrier
+// ends it. The smallest levels, where a pass is one round of loads, live in block 0, whose own
+// barrier ends a pass while the others wait. Every array carries a ring of ghost cells (0 across
+// walls; a pass writes a cell's periodic images with the cell), so that neighbours lie at
+// offsets common to all threads, and a thread's column comes from two multiplications by
+// precomputed reciprocals.
+// Bound by the instructions and barriers of a pass (1.4 us each; a cluster barrier alone is 0.37 us with
+// 512 threads); FP64: by the FP64 pipes of its SMs. Measured against the same levels in one block: 24^3 and
+// below 53 -> 28 us per V-cycle in FP32; with the larger levels now included, a 48^3 mixed step 1464 ->
+// 1224 us, ten steps of eight 64^3 runs 19.0 -> 18.4 ms, a 64 x 32 x 32 FP64 step 1521 -> 1431 us.
 constexpr int MG_BOTTOM_MAXLEV = 12;
 constexpr size_t MG_BOTTOM_SMEM = 200 * 1024;
-constexpr long long MG_BOTTOM_MAXVOL_FP64 = 1024;   // largest level (cells) in the FP64 one-block kernel
-template <typename T> struct MgBottomThreads { static constexpr int n = 1024; };
-template <> struct MgBottomThreads<double> { static constexpr int n = 512; };   // register budget
+constexpr int BT_CTAS = 8, BT_THREADS = 512;
 
+struct MgBottomLevel {
+    int n[3];                // z, y, x
+    int pp, nblk;            // z planes per block, blocks that hold planes (1: block 0 alone)
+    int sy, sz, vol;         // of the padded arrays (pp + 2 planes)
+    int off;                 // elements: x, then y, then b
+    int zg, ng;              // cells of a column per task, tasks per column
+    unsigned int mx, mcol;   // ceil(2^32 / n[2]), ceil(2^32 / (n[1] n[2]))
+    int bychild;             // FP32: roundings of the smallest levels (see bottom_plan)
+};
 template <typename T>
 struct MgBottom {
-    int nlev;                          // levels held: l0..L-1
-    MgGeom g[MG_BOTTOM_MAXLEV];
-    int off[MG_BOTTOM_MAXLEV];         // element offset of each level's x in shared memory; b, y follow
-    T* xg;                             // x of level l0 (global)
-    const T* bg;                       // b of level l0 (global)
-    T omega;
+    int nlev;                // levels held, none of them empty
+    int resmooth;            // the last one lies above an empty level: it is smoothed on the way up too
+    int per[3];
+    T idiag[8], pcoef[8];    // MgGeom's tables
+    MgBottomLevel lev[MG_BOTTOM_MAXLEV];
+    T* xg;                   // x of level l0 (global)
+    const T* bg;             // b of level l0 (global)
 };
 
-__device__ __forceinline__ int mg_vol(const MgGeom& g) { return g.n[0] * g.n[1] * g.n[2]; }
+// quotient by the n of m = ceil(2^32 / n), exact for t, n < 2^16 (n = 1: m wraps to 0)
+__device__ __forceinline__ int bottom_div(int t, unsigned int m) { return m ? (int)__umulhi((unsigned int)t, m) : t; }
 
-// neighbours along one direction with 32-bit offsets (levels held in shared memory)
-struct MgNbI {
-    int om, op;
-    bool wm, wp;
+// a column segment of the block's slab: cells z0 <= z < z1 of the level, p = index of the first
+// one in the padded arrays
+struct BottomTask {
+    int x, y, z0, z1, p;
 };
-__device__ __forceinline__ MgNbI mg_nbi(int c, int n, int per, int stride) {
-    MgNbI r;
-    r.wm = c > 0 || per;
-    r.wp = c < n - 1 || per;
-    r.om = c > 0 ? -stride : (per ? (n - 1) * stride : 0);
-    r.op = c < n - 1 ? stride : (per ? -(n - 1) * stride : 0);
+__device__ __forceinline__ BottomTask bottom_task(const MgBottomLevel& l, int zb, int t) {
+    BottomTask k;
+    const int ncol = l.n[1] * l.n[2], g = bottom_div(t, l.mcol), col = t - g * ncol;
+    k.y = bottom_div(col, l.mx);
+    k.x = col - k.y * l.n[2];
+    k.z0 = zb + g * l.zg;
+    k.z1 = min(k.z0 + l.zg, min(zb + l.pp, l.n[0]));
+    k.p = (k.z0 - zb + 1) * l.sz + (k.y + 1) * l.sy + k.x + 1;
+    return k;
+}
+
+// A block's slab of a level
+template <typename T>
+struct BottomSlab {
+    int zb, ze;              // planes held
+    int zlo, zhi;            // the planes with an image in the slab below, above (-1: none)
+    T *lo, *hi;              // shared memory there, shifted so that an element's index is its image's
+};
+
+// Offsets of a column's images across the x and y faces of a periodic level (0: none; both when n = 1)
+struct BottomRing {
+    int xl, xh, yl, yh;
+    bool any;
+};
+__device__ __forceinline__ BottomRing bottom_ring(const MgBottomLevel& l, const int* per, int y, int x) {
+    BottomRing r;
+    r.xl = per[2] && x == 0 ? l.n[2] : 0;
+    r.xh = per[2] && x == l.n[2] - 1 ? -l.n[2] : 0;
+    r.yl = per[1] && y == 0 ? l.n[1] * l.sy : 0;
+    r.yh = per[1] && y == l.n[1] - 1 ? -l.n[1] * l.sy : 0;
+    r.any = (r.xl | r.xh | r.yl | r.yh) != 0;
     return r;
 }
-template <typename T>
-__device__ __forceinline__ T sm_ldw(const T* a, int c, bool wet) {
-    const T v = a[c];
-    return wet ? v : T(0);
-}
-
-// Visit every cell of a level: threads take (x, y) columns, split in z when the block
-// has more threads than the level has columns; f(z, y, x, nx, ny) gets the column's
-// x/y neighbours.
-template <typename F>
-__device__ __forceinline__ void bottom_cells(const MgGeom& g, F f) {
-    const int ncol = g.n[1] * g.n[2], nz = g.n[0];
-    if (ncol == 0 || nz == 0) return;
-    const int groups = max(1, (int)blockDim.x / ncol);
-    const int zc = (nz + groups - 1) / groups;
-    // power-of-two extents (the usual coarse levels): masks and shifts instead of the
-    // integer divisions, which took a large share of a pass over a small level
-    const int n2 = g.n[2];
-    const bool p2 = ((ncol & (ncol - 1)) | (n2 & (n2 - 1))) == 0;
-    const int lc = __ffs(ncol) - 1, l2 = __ffs(n2) - 1;
-    for (int t = threadIdx.x; t < ncol * groups; t += blockDim.x) {
-        int col, grp, x, y;
-        if (p2) {
-            col = t & (ncol - 1);
-            grp = t >> lc;
-            x = col & (n2 - 1);
-            y = col >> l2;
-        } else {
-            col = t % ncol;
-            grp = t / ncol;
-            x = col % n2;
-            y = col / n2;
-        }
-        const MgNbI nx = mg_nbi(x, g.n[2], g.per[2], 1), ny = mg_nbi(y, g.n[1], g.per[1], g.n[2]);
-        const int ze = min(nz, (grp + 1) * zc);
-        for (int z = grp * zc; z < ze; ++z) f(z, y, x, nx, ny);
+template <bool EDGES, typename T>
+__device__ __forceinline__ void bottom_ring_put(const BottomRing& r, T* q, T v) {
+    if (r.xl) q[r.xl] = v;
+    if (r.xh) q[r.xh] = v;
+    if (r.yl) q[r.yl] = v;
+    if (r.yh) q[r.yh] = v;
+    if (EDGES) {
+        if (r.xl && r.yl) q[r.xl + r.yl] = v;
+        if (r.xl && r.yh) q[r.xl + r.yh] = v;
+        if (r.xh && r.yl) q[r.xh + r.yl] = v;
+        if (r.xh && r.yh) q[r.xh + r.yh] = v;
     }
 }
-
-// one half-sweep in -> out over a level held in shared memory
-template <typename T>
-__device__ __forceinline__ void bottom_sweep(const MgGeom& g, const T* in, const T* b, T* out, T cff1, T om) {
-    const int sz = g.n[1] * g.n[2];
-    bottom_cells(g, [&](int z, int y, int x, const MgNbI& nx, const MgNbI& ny) {
-        const int c = (z * g.n[1] + y) * g.n[2] + x;
-        const MgNbI nzb = mg_nbi(z, g.n[0], g.per[0], sz);
-        const T idg = mg_idiag<T>(g, (int)nx.wm + (int)nx.wp + (int)ny.wm + (int)ny.wp + (int)nzb.wm + (int)nzb.wp);
-        const T s = ((((sm_ldw(in, c + nx.om, nx.wm) + sm_ldw(in, c + nx.op, nx.wp)) + sm_ldw(in, c + ny.om, ny.wm)) +
-                      sm_ldw(in, c + ny.op, ny.wp)) + sm_ldw(in, c + nzb.om, nzb.wm)) + sm_ldw(in, c + nzb.op, nzb.wp);
-        out[c] = cff1 * in[c] + (s - b[c]) * idg;
-    });
-    __syncthreads();
-}
-
-// 1/diag of a cell from its column's x/y neighbours and its z position
-template <typename T>
-__device__ __forceinline__ T bottom_idiag(const MgGeom& g, int z, const MgNbI& nx, const MgNbI& ny) {
-    const MgNbI nzb = mg_nbi(z, g.n[0], g.per[0], 0);
-    return mg_idiag<T>(g, (int)nx.wm + (int)nx.wp + (int)ny.wm + (int)ny.wp + (int)nzb.wm + (int)nzb.wp);
-}
-
-// sum of the residuals of the 8 children of coarse cell (z, y, x), shared-memory level
-// (mg_restrict_cell with direct neighbour offsets)
-template <typename T>
-__device__ __forceinline__ T bottom_restrict(const MgGeom& gf, const T* xf, const T* bf, int z, int y, int x) {
-    const int nx = gf.n[2], ny = gf.n[1], nz = gf.n[0], sy = nx, sz = nx * ny;
-    const int i0 = 2 * x, j0 = 2 * y, k0 = 2 * z;
-    const MgNbI xl = mg_nbi(i0, nx, gf.per[2], 1), xh = mg_nbi(i0 + 1, nx, gf.per[2], 1);
-    const MgNbI yl = mg_nbi(j0, ny, gf.per[1], sy), yh = mg_nbi(j0 + 1, ny, gf.per[1], sy);
-    const MgNbI zl = mg_nbi(k0, nz, gf.per[0], sz), zh = mg_nbi(k0 + 1, nz, gf.per[0], sz);
-    const int dxy[4] = {(int)xl.wm + 1 + (int)yl.wm + 1, 1 + (int)xh.wp + (int)yl.wm + 1,
-                        (int)xl.wm + 1 + 1 + (int)yh.wp, 1 + (int)xh.wp + 1 + (int)yh.wp};
-    const int cb = (k0 * ny + j0) * nx + i0;
-    T v[4][4];   // the 2 x 2 children positions on planes k0-1 .. k0+2
-    auto ld4 = [&](int c, bool wet, T* o) {
-        o[0] = sm_ldw(xf, c, wet);
-        o[1] = sm_ldw(xf, c + 1, wet);
-        o[2] = sm_ldw(xf, c + sy, wet);
-        o[3] = sm_ldw(xf, c + sy + 1, wet);
-    };
-    ld4(cb + zl.om, zl.wm, v[0]);
-    ld4(cb, true, v[1]);
-    ld4(cb + sz, true, v[2]);
-    ld4(cb + sz + zh.op, zh.wp, v[3]);
-    T s = T(0);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int q = h + 1;
-        const int c = cb + h * sz;
-        const int dz = (h == 0 ? (int)zl.wm : 1) + (h == 1 ? (int)zh.wp : 1);
-        const T xm0 = sm_ldw(xf, c + xl.om, xl.wm), xm1 = sm_ldw(xf, c + sy + xl.om, xl.wm);
-        const T xp0 = sm_ldw(xf, c + 1 + xh.op, xh.wp), xp1 = sm_ldw(xf, c + sy + 1 + xh.op, xh.wp);
-        const T ym0 = sm_ldw(xf, c + yl.om, yl.wm), ym1 = sm_ldw(xf, c + 1 + yl.om, yl.wm);
-        const T yp0 = sm_ldw(xf, c + sy + yh.op, yh.wp), yp1 = sm_ldw(xf, c + sy + 1 + yh.op, yh.wp);
-        const T* p = v[q];
-        const T r00 = (bf[c] + T(dxy[0] + dz) * p[0]) - (((((xm0 + p[1]) + ym0) + p[2]) + v[q - 1][0]) + v[q + 1][0]);
-        const T r01 = (bf[c + 1] + T(dxy[1] + dz) * p[1]) -
-                      (((((p[0] + xp0) + ym1) + p[3]) + v[q - 1][1]) + v[q + 1][1]);
-        const T r10 = (bf[c + sy] + T(dxy[2] + dz) * p[2]) -
-                      (((((xm1 + p[3]) + p[0]) + yp0) + v[q - 1][2]) + v[q + 1][2]);
-        const T r11 = (bf[c + sy + 1] + T(dxy[3] + dz) * p[3]) -
-                      (((((p[2] + xp1) + p[1]) + yp1) + v[q - 1][3]) + v[q + 1][3]);
-        s = (h == 0) ? r00 : s + r00;
-        s = s + r01;
-        s = s + r10;
-        s = s + r11;
+// element p of the array at offset o (of shared memory base `s`) = v, a cell of plane z, with its images: in
+// the level's ghost columns, and of the slab's first and last plane in the neighbouring slabs. EDGES: images
+// across edges and corners too (before a prolongation reads the diagonal neighbours).
+template <bool EDGES, typename T>
+__device__ __forceinline__ void bottom_put(const BottomSlab<T>& sl, const BottomRing& r, T* s, int o, int p, int z, T v) {
+    s[o + p] = v;
+    if (z == sl.zlo) sl.lo[o + p] = v;
+    if (z == sl.zhi) sl.hi[o + p] = v;
+    if (r.any) {
+        bottom_ring_put<EDGES>(r, s + o + p, v);
+        if (EDGES && z == sl.zlo) bottom_ring_put<true>(r, sl.lo + o + p, v);
+        if (EDGES && z == sl.zhi) bottom_ring_put<true>(r, sl.hi + o + p, v);
     }
-    return s;
+}
+// damped inverse diagonals of a column: inside, and at the first and last plane of a closed level
+template <typename T>
+struct BottomDiag {
+    T in, end;
+    int z1;                  // last plane with a closed end (-1: periodic)
+    __device__ __forceinline__ T at(int z) const { return (z == 0 || z == z1) && z1 >= 0 ? end : in; }
+};
+
+// wet x and y neighbours of a column, wet z neighbours of a cell
+__device__ __forceinline__ int bottom_wet_xy(const MgBottomLevel& l, const int* per, int y, int x) {
+    return (per[2] ? 2 : (x > 0) + (x < l.n[2] - 1)) + (per[1] ? 2 : (y > 0) + (y < l.n[1] - 1));
+}
+__device__ __forceinline__ int bottom_wet_z(const MgBottomLevel& l, const int* per, int z) {
+    return per[0] ? 2 : (z > 0) + (z < l.n[0] - 1);
+}
+template <typename T>
+__device__ __forceinline__ BottomDiag<T> bottom_diag(const MgBottomLevel& l, const int* per, const T* idiag, int y, int x) {
+    BottomDiag<T> d;
+    const int dxy = bottom_wet_xy(l, per, y, x);
+    d.z1 = per[0] ? -1 : l.n[0] - 1;
+    d.in = idiag[dxy + 2];
+    d.end = idiag[dxy + (l.n[0] > 1 ? 1 : 0)];
+    return d;
 }
 
-// prolongation increment of fine cell (z, y, x) from a shared-memory coarse level
-// (mg_prolong_cell with direct neighbour offsets)
 template <typename T>
-__device__ __forceinline__ T bottom_prolong(const MgGeom& gf, const MgGeom& gc, const T* xc, int z, int y, int x) {
-    const int ic = x >> 1, jc = y >> 1, kc = z >> 1;
-    const int csy = gc.n[2], csz = gc.n[1] * gc.n[2];
-    const MgNbI cx = mg_nbi(ic, gc.n[2], gc.per[2], 1), cy = mg_nbi(jc, gc.n[1], gc.per[1], csy);
-    const MgNbI cz = mg_nbi(kc, gc.n[0], gc.per[0], csz);
-    const int ox = (x & 1) ? cx.op : cx.om, oy = (y & 1) ? cy.op : cy.om, oz = (z & 1) ? cz.op : cz.om;
-    const bool wx = (x & 1) ? cx.wp : cx.wm, wy = (y & 1) ? cy.wp : cy.wm, wz = (z & 1) ? cz.wp : cz.wm;
-    const int c0 = (kc * gc.n[1] + jc) * gc.n[2] + ic;
-    auto plane = [&](int c, bool w) -> T {
-        const T a = sm_ldw(xc, c, w), b = sm_ldw(xc, c + ox, w && wx);
-        const T d = sm_ldw(xc, c + oy, w && wy), e = sm_ldw(xc, c + ox + oy, w && wx && wy);
-        return ((T(9) * a + T(3) * b) + T(3) * d) + e;
-    };
-    const T bpl = plane(c0, true), opl = plane(c0 + oz, wz);
-    const T pcoef = mg_pcoef<T>(gf, (int)wx | ((int)wy << 1) | ((int)wz << 2));
-    return pcoef * (T(3) * bpl + opl);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(MgBottomThreads<T>::n, 1) k_mg_bottom(const MgBottom<T> a, const Bat bat = Bat()) {
+__global__ void __cluster_dims__(BT_CTAS, 1, 1) __launch_bounds__(BT_THREADS, 2)
+    k_mg_bottom(const __grid_constant__ MgBottom<T> a, const Bat bat = Bat()) {
     extern __shared__ __align__(16) unsigned char mg_smem[];
     int bz;
     long long dlt;
-    if (!batch_enter(bat, bz, dlt)) return;
+    if (!batch_enter(bat, bz, dlt)) return;   // (one answer for the whole cluster)
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank();
     // the arguments stay in parameter space (their level table is indexed at run time:
     // a copy of the struct would sit in every thread's local memory); only the two
     // global pointers are shifted to the block's run
     T* const xg = bshift(a.xg, dlt);
     const T* const bg = bshift(a.bg, dlt);
-    T* sm = reinterpret_cast<T*>(mg_smem);
-    const T om = a.omega, cff1 = T(1) - om;
+    T* const sm = reinterpret_cast<T*>(mg_smem);
+    const T cff1 = T(1) - a.idiag[1];   // idiag[1] = omega
     const int L = a.nlev;
-    auto X = [&](int l) { return sm + a.off[l]; };
-    auto Bv = [&](int l) { return sm + a.off[l] + mg_vol(a.g[l]); };
-    auto Y = [&](int l) { return sm + a.off[l] + 2 * mg_vol(a.g[l]); };
-    // level l0 starts from x = 0: its first half-sweep is y = from_zero(b)
-    bottom_cells(a.g[0], [&](int z, int y, int x, const MgNbI& nx, const MgNbI& ny) {
-        const int c = (z * a.g[0].n[1] + y) * a.g[0].n[2] + x;
-        const T bv = bg[c];
-        Bv(0)[c] = bv;
-        Y(0)[c] = mg_jacobi_from_zero(bv, om, bottom_idiag<T>(a.g[0], z, nx, ny));
-    });
-    __syncthreads();
-    for (int l = 0; l < L - 1; ++l) {
-        if (mg_vol(a.g[l]) == 0) break;
-        bottom_sweep(a.g[l], Y(l), Bv(l), X(l), cff1, om);   // second half of the pre-smoothing
-        const MgGeom& gc = a.g[l + 1];
-        if (mg_vol(gc) == 0) break;
-        // restriction; the coarse level starts from zero, so its first half-sweep is written too
-        bottom_cells(gc, [&](int z, int y, int x, const MgNbI& nx, const MgNbI& ny) {
-            const int c = (z * gc.n[1] + y) * gc.n[2] + x;
-            const T bv = T(0.5) * bottom_restrict(a.g[l], X(l), Bv(l), z, y, x);
-            Bv(l + 1)[c] = bv;
-            Y(l + 1)[c] = mg_jacobi_from_zero(bv, om, bottom_idiag<T>(gc, z, nx, ny));
-        });
-        __syncthreads();
-    }
-    if (mg_vol(a.g[L - 1]) > 0) bottom_sweep(a.g[L - 1], Y(L - 1), Bv(L - 1), X(L - 1), cff1, om);
-    for (int l = L - 2; l >= 0; --l) {
-        const MgGeom& gf = a.g[l];
-        if (mg_vol(gf) == 0) continue;
-        if (mg_vol(a.g[l + 1]) > 0) {
-            bottom_cells(gf, [&](int z, int y, int x, const MgNbI&, const MgNbI&) {
-                const int c = (z * gf.n[1] + y) * gf.n[2] + x;
-                X(l)[c] = X(l)[c] + bottom_prolong(gf, a.g[l + 1], X(l + 1), z, y, x);
-            });
-            __syncthreads();
+    // the block's slab of level l as seen from `who` (a block writes block 0's small levels
+    // when it restricts into them); ghosts of the neighbouring slabs lie nz_prev planes up and
+    // the block's own planes down from its first and last plane
+    auto slab = [&](const MgBottomLevel& l, int who) {
+        BottomSlab<T> s;
+        s.zb = who * l.pp;
+        s.ze = min(s.zb + l.pp, l.n[0]);
+        s.zlo = s.zhi = -1;
+        s.lo = s.hi = sm;
+        if (who >= l.nblk) { s.ze = s.zb; return s; }
+        const int prev = who > 0 ? who - 1 : (a.per[0] ? l.nblk - 1 : -1);
+        const int next = who < l.nblk - 1 ? who + 1 : (a.per[0] ? 0 : -1);
+        if (prev >= 0) {
+            s.zlo = s.zb;
+            s.lo = cluster.map_shared_rank(sm, prev) + min(l.pp, l.n[0] - prev * l.pp) * l.sz;
         }
-        bottom_sweep(gf, X(l), Bv(l), Y(l), cff1, om);
-        bottom_sweep(gf, Y(l), Bv(l), X(l), cff1, om);
+        if (next >= 0) {
+            s.zhi = s.ze - 1;
+            s.hi = cluster.map_shared_rank(sm, next) - (s.ze - s.zb) * l.sz;
+        }
+        return s;
+    };
+    // ends a pass over level l (its writers and readers: the cluster, or block 0)
+    auto sync = [&](const MgBottomLevel& l) {
+        if (l.nblk > 1) cluster.sync();
+        else if (rank == 0) __syncthreads();
+    };
+    auto ntasks = [&](const MgBottomLevel& l) { return rank < l.nblk ? l.n[1] * l.n[2] * l.ng : 0; };
+    // offsets of a level's arrays
+    enum { AX = 0, AY = 1, AB = 2 };
+    auto arr = [&](const MgBottomLevel& l, int w) { return l.off + w * l.vol; };
+
+    // ghosts across walls stay 0
+    const MgBottomLevel& last = a.lev[L - 1];
+    for (int q = threadIdx.x; q < last.off + 3 * last.vol; q += BT_THREADS) sm[q] = T(0);
+    cluster.sync();
+    {   // level l0 starts from x = 0: its first half-sweep is y = from_zero(b)
+        const MgBottomLevel& l = a.lev[0];
+        const BottomSlab<T> sl = slab(l, rank);
+        const int nplane = l.n[1] * l.n[2], nt = ntasks(l), ob = arr(l, AB), oy = arr(l, AY);
+        for (int t = threadIdx.x; t < nt; t += BT_THREADS) {
+            const BottomTask k = bottom_task(l, sl.zb, t);
+            const BottomRing ring = bottom_ring(l, a.per, k.y, k.x);
+            const BottomDiag<T> dg = bottom_diag(l, a.per, a.idiag, k.y, k.x);
+            const T* pb = bg + k.z0 * nplane + k.y * l.n[2] + k.x;
+            int p = k.p;
+            for (int z = k.z0; z < k.z1; ++z, pb += nplane, p += l.sz) {
+                const T bv = *pb;
+                sm[ob + p] = bv;
+                bottom_put<false>(sl, ring, sm, oy, p, z, mg_jacobi_from_zero(bv, T(0), dg.at(z)));
+            }
+        }
+        sync(l);
     }
-    const int v0 = mg_vol(a.g[0]);
-    for (int q = threadIdx.x; q < v0; q += blockDim.x) xg[q] = X(0)[q];
+    // one half-sweep from array wi to array wo
+    auto sweep = [&](const MgBottomLevel& l, int wi, int wo, auto edges) {
+        constexpr bool EDGES = decltype(edges)::value;
+        const BottomSlab<T> sl = slab(l, rank);
+        const int nt = ntasks(l), oo = arr(l, wo);
+        const T* in = sm + arr(l, wi);
+        const T* b = sm + arr(l, AB);
+        for (int t = threadIdx.x; t < nt; t += BT_THREADS) {
+            const BottomTask k = bottom_task(l, sl.zb, t);
+            const BottomRing ring = bottom_ring(l, a.per, k.y, k.x);
+            const BottomDiag<T> dg = bottom_diag(l, a.per, a.idiag, k.y, k.x);
+            int p = k.p;
+            T zm = in[p - l.sz], zc = in[p];
+            for (int z = k.z0; z < k.z1; ++z) {
+                const T zp = in[p + l.sz];
+                const T s = ((((in[p - 1] + in[p + 1]) + in[p - l.sy]) + in[p + l.sy]) + zm) + zp;
+                bottom_put<EDGES>(sl, ring, sm, oo, p, z, fma(cff1, zc, mul_rn(s - b[p], dg.at(z))));
+                zm = zc;
+                zc = zp;
+                p += l.sz;
+            }
+        }
+        sync(l);
+    };
+    for (int i = 0; i < L - 1; ++i) {
+        const MgBottomLevel &f = a.lev[i], &c = a.lev[i + 1];
+        sweep(f, AY, AX, std::false_type());   // second half of the pre-smoothing
+        // residuals of the 8 children; the coarse level starts from zero, so its first
+        // half-sweep is written too
+        const BottomSlab<T> fs = slab(f, rank);
+        const int owner = c.nblk > 1 ? rank : 0;            // the block that holds the coarse cells
+        const BottomSlab<T> cs = slab(c, owner);
+        T* const smc = owner == rank ? sm : cluster.map_shared_rank(sm, owner);
+        const T* xf = sm + arr(f, AX);
+        const T* bf = sm + arr(f, AB);
+        const int ob = arr(c, AB), oy = arr(c, AY);
+        const int zc0 = fs.zb / 2, zc1 = (fs.ze + 1) / 2, ncol = c.n[1] * c.n[2];
+        const int nt = rank < f.nblk ? ncol * (zc1 - zc0) : 0;
+        for (int t = threadIdx.x; t < nt; t += BT_THREADS) {
+            const int g = bottom_div(t, c.mcol), col = t - g * ncol, z = zc0 + g;
+            const int y = bottom_div(col, c.mx), x = col - y * c.n[2];
+            const int x0 = 2 * x, y0 = 2 * y;
+            const int wxl = a.per[2] || x0 > 0, wxh = a.per[2] || x0 + 2 < f.n[2];
+            const int wyl = a.per[1] || y0 > 0, wyh = a.per[1] || y0 + 2 < f.n[1];
+            // sum(b) + sum(w x) - sum(24 outside cells), w = wet outside neighbours (k_mg_restrict), or
+            // the children's residuals one by one
+            T sb = T(0), sx = T(0), so = T(0), sr = T(0);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int zf = 2 * z + h;
+                const int p = (zf - fs.zb + 1) * f.sz + (y0 + 1) * f.sy + x0 + 1;
+                const T *q = xf + p, *qb = bf + p, *ol = q - f.sz, *oh = q + f.sz;
+                const T p0 = q[0], p1 = q[1], p2 = q[f.sy], p3 = q[f.sy + 1];
+                const T xm0 = q[-1], xm1 = q[f.sy - 1], xp0 = q[2], xp1 = q[f.sy + 2];
+                const T ym0 = q[-f.sy], ym1 = q[1 - f.sy], yp0 = q[2 * f.sy], yp1 = q[2 * f.sy + 1];
+                if (sizeof(T) == sizeof(float) && f.bychild) {
+                    const int dz = bottom_wet_z(f, a.per, zf);
+                    const T r00 = (qb[0] + T(wxl + wyl + 2 + dz) * p0) - (((((xm0 + p1) + ym0) + p2) + ol[0]) + oh[0]);
+                    const T r01 = (qb[1] + T(wxh + wyl + 2 + dz) * p1) - (((((p0 + xp0) + ym1) + p3) + ol[1]) + oh[1]);
+                    const T r10 = (qb[f.sy] + T(wxl + wyh + 2 + dz) * p2) -
+                                  (((((xm1 + p3) + p0) + yp0) + ol[f.sy]) + oh[f.sy]);
+                    const T r11 = (qb[f.sy + 1] + T(wxh + wyh + 2 + dz) * p3) -
+                                  (((((p2 + xp1) + p1) + yp1) + ol[f.sy + 1]) + oh[f.sy + 1]);
+                    sr = (h == 0) ? r00 : sr + r00;
+                    sr = sr + r01;
+                    sr = sr + r10;
+                    sr = sr + r11;
+                } else {
+                    const T* o = h == 0 ? ol : oh;
+                    const bool wz = a.per[0] || (h == 0 ? zf > 0 : zf < f.n[0] - 1);
+                    sb = sb + ((qb[0] + qb[1]) + (qb[f.sy] + qb[f.sy + 1]));
+                    sx = sx + (T(wxl + wyl) * p0 + T(wxh + wyl) * p1 + T(wxl + wyh) * p2 + T(wxh + wyh) * p3);
+                    sx = wz ? sx + ((p0 + p1) + (p2 + p3)) : sx;
+                    so = so + ((((xm0 + xm1) + (xp0 + xp1)) + ((ym0 + ym1) + (yp0 + yp1))) +
+                               ((o[0] + o[1]) + (o[f.sy] + o[f.sy + 1])));
+                }
+            }
+            const T bv = T(0.5) * (sizeof(T) == sizeof(float) && f.bychild ? sr : (sb + sx) - so);
+            const int p = (z - cs.zb + 1) * c.sz + (y + 1) * c.sy + x + 1;
+            smc[ob + p] = bv;
+            const int dg = bottom_wet_xy(c, a.per, y, x) + bottom_wet_z(c, a.per, z);
+            bottom_put<false>(cs, bottom_ring(c, a.per, y, x), smc, oy, p, z, mg_jacobi_from_zero(bv, T(0), a.idiag[dg]));
+        }
+        sync(f);
+    }
+    sweep(last, AY, AX, std::true_type());
+    for (int i = a.resmooth ? L - 1 : L - 2; i >= 0; --i) {
+        const MgBottomLevel& f = a.lev[i];
+        if (i < L - 1) {
+            const MgBottomLevel& c = a.lev[i + 1];
+            if (f.nblk > 1 && c.nblk == 1) cluster.sync();   // block 0's x is ready
+            const BottomSlab<T> fs = slab(f, rank);
+            const int owner = c.nblk > 1 ? rank : 0, czb = owner * c.pp;
+            const T* xc = (owner == rank ? sm : cluster.map_shared_rank(sm, owner)) + arr(c, AX);
+            const int nt = ntasks(f), ox_ = arr(f, AX);
+            T* xf = sm + ox_;
+            for (int t = threadIdx.x; t < nt; t += BT_THREADS) {
+                const BottomTask k = bottom_task(f, fs.zb, t);
+                const int ic = k.x >> 1, jc = k.y >> 1;
+                const int ox = (k.x & 1) ? 1 : -1, oy = (k.y & 1) ? c.sy : -c.sy;
+                const int wx = a.per[2] || ((k.x & 1) ? ic + 1 < c.n[2] : ic > 0);
+                const int wy = a.per[1] || ((k.y & 1) ? jc + 1 < c.n[1] : jc > 0);
+                const T* col = xc + (jc + 1) * c.sy + ic + 1;
+                // in-plane sums of a coarse plane as the cell's own and as the one beyond it (alike but
+                // for the roundings of the smallest FP32 levels)
+                struct Plane { T own, beyond; };
+                const bool unfused = sizeof(T) == sizeof(float) && f.bychild;
+                auto plane = [&](int kk) -> Plane {
+                    const T* q = col + (kk - czb + 1) * c.sz;
+                    const T q0 = q[0], qx = q[ox], qy = q[oy], qxy = q[ox + oy];
+                    const T b3 = mul_rn(T(3), qx), d3 = mul_rn(T(3), qy), t = fma(T(9), q0, b3);
+                    Plane r;
+                    r.own = r.beyond = fma(T(3), qy, t) + qxy;
+                    if (unfused) {
+                        r.own = add_rn(add_rn(t, d3), qxy);
+                        r.beyond = add_rn(add_rn(add_rn(mul_rn(T(9), q0), b3), d3), qxy);
+                    }
+                    return r;
+                };
+                const BottomRing ring = bottom_ring(f, a.per, k.y, k.x);
+                const T pin = a.pcoef[wx | (wy << 1) | 4], pend = a.pcoef[wx | (wy << 1) | (a.per[0] ? 4 : 0)];
+                // segments start at even z: each coarse plane is formed once
+                int p = k.p, kc = k.z0 >> 1;
+                Plane pm = plane(kc - 1), pc = plane(kc);
+                for (int z = k.z0; z < k.z1; z += 2, ++kc) {
+                    const Plane pn = plane(kc + 1);
+                    bottom_put<false>(fs, ring, sm, ox_, p, z,
+                                      fma(kc > 0 ? pin : pend, fma(T(3), pc.own, pm.beyond), xf[p]));
+                    p += f.sz;
+                    bottom_put<false>(fs, ring, sm, ox_, p, z + 1,
+                                      fma(kc < c.n[0] - 1 ? pin : pend, fma(T(3), pc.own, pn.beyond), xf[p]));
+                    p += f.sz;
+                    pm = pc;
+                    pc = pn;
+                }
+            }
+            sync(f);
+        }
+        sweep(f, AX, AY, std::false_type());
+        sweep(f, AY, AX, std::true_type());
+    }
+    const MgBottomLevel& l = a.lev[0];
+    const int nplane = l.n[1] * l.n[2], nt = ntasks(l), zb = rank * l.pp, ox = arr(l, AX);
+    for (int t = threadIdx.x; t < nt; t += BT_THREADS) {
+        const BottomTask k = bottom_task(l, zb, t);
+        for (int z = k.z0; z < k.z1; ++z)
+            xg[z * nplane + k.y * l.n[2] + k.x] = sm[ox + k.p + (z - k.z0) * l.sz];
+    }
+    cluster.sync();   // no block leaves while another may still write its ghosts
+}
+
+// The levels of the cluster kernel from level l0 on (n: extents; none of them empty): how each is cut, the
+// arrays' places; returns the elements of shared memory per block. A level of more than `solo` cells
+// is cut into an even number of planes per block, and the level under it too while half of them is even.
+// FP32 keeps each level's roundings, so that solutions do not depend, to the bit, on which kernel a level
+// runs in: a restriction child by child and partly unfused sums in the prolongation where this level and
+// those under it hold at most 200 KB of x, b and y, as the grid kernels above.
+static long long bottom_plan(const int (*n)[3], int nlev, long long solo, MgBottomLevel* lev) {
+    long long off = 0;
+    int half = 0;   // planes per block of the next level, from the one above (0: not cut)
+    for (int k = 0; k < nlev; ++k) {
+        MgBottomLevel l;
+        for (int i = 0; i < 3; ++i) l.n[i] = n[k][i];
+        const int nz = l.n[0], ncol = l.n[1] * l.n[2];
+        const bool cut = (long long)nz * ncol > solo && nz >= 4 && (k == 0 || (half && half % 2 == 0));
+        l.pp = !cut ? nz : (k == 0 ? 2 * ((nz + 2 * BT_CTAS - 1) / (2 * BT_CTAS)) : half);
+        l.nblk = (nz + l.pp - 1) / l.pp;
+        half = l.nblk > 1 ? l.pp / 2 : 0;
+        l.sy = l.n[2] + 2;
+        l.sz = l.sy * (l.n[1] + 2);
+        l.vol = l.sz * (l.pp + 2);
+        l.off = (int)off;
+        off += 3ll * l.vol;
+        // columns are cut in z (in pairs of planes, which share their coarse planes) so that the block's
+        // rounds of tasks take the fewest cells, a task's start counted as two
+        long long best = 1ll << 60;
+        for (int zg = l.pp < 2 ? 1 : 2; zg <= 8 && (zg <= l.pp || zg <= 2); zg += zg < 2 ? 1 : 2) {
+            const long long rounds = ((long long)ncol * ((l.pp + zg - 1) / zg) + BT_THREADS - 1) / BT_THREADS;
+            if (rounds * (zg + 2) < best) {
+                best = rounds * (zg + 2);
+                l.zg = zg;
+            }
+        }
+        l.ng = (l.pp + l.zg - 1) / l.zg;
+        l.mx = (unsigned int)(((1ull << 32) + l.n[2] - 1) / l.n[2]);
+        l.mcol = (unsigned int)(((1ull << 32) + ncol - 1) / ncol);
+        long long under = 0;
+        for (int j = k; j < nlev; ++j) under += (long long)n[j][0] * n[j][1] * n[j][2];
+        l.bychild = 3 * (long long)sizeof(float) * under <= 200 * 1024;
+        if (lev) lev[k] = l;
+    }
+    return off;
 }
 
 // ---------------------------------------------------------------- reductions
@@ -2285,6 +2462,21 @@ static float2* mg_pdf_old(MgImpl* mg, int h) {
 }
 static int* mg_hist_count(MgImpl* mg) { return reinterpret_cast<int*>(mg->ws + mg->off_hist) + mg->cur_sol; }
 
+// non-empty levels from l0 on, and their extents
+static int bottom_extents(const MgImpl* mg, int l0, int (*n)[3]) {
+    int k = 0;
+    for (; l0 + k < mg->nlevels && !empty(mg, l0 + k); ++k)
+        for (int i = 0; i < 3; ++i) n[k][i] = mg->lev[l0 + k].n[i];
+    return k;
+}
+// The largest level of the cluster kernel, and the largest that block 0 holds alone. Measured (us): FP32
+// up to 4096 / 14000 / 32768 cells: a 256 x 256 x 128 solve 1670 / 1665 / 1648, ten steps of eight 64^3
+// runs 19300 / 19370 / 18410; block 0 alone up to 512 / 1024 / 2048 cells of a 48^3 step 1232 / 1232 / 1289.
+// FP64 up to 1024 / 2048 / 4096 / 8192 cells: a 128^3 solve 1408 / 1409 / 1356 / 1304-1370, a 64 x 32 x 32
+// step 1438 / 1438 / 1437 / 1599; block 0 alone up to 256 / 1024 cells 1438 / 1515.
+static long long bottom_maxvol(int precision) { return precision == NYLES_MIXED ? 1 << 15 : 1 << 12; }
+static long long bottom_solo(int precision) { return precision == NYLES_MIXED ? 1024 : 256; }
+
 // mg_setup.f90:225-307 (create_hierarchy) for one rank. The reference leaves the loop
 // only when x == 2 or y == 2; here coarsening also stops before an odd extent, so
 // 3*2^n sizes terminate (the reference does not terminate on them).
@@ -2339,22 +2531,18 @@ int mg_init(MgImpl* mg, int nx, int ny, int nz, int topology, int precision, int
         mg->off_fp = take(mg->lev[0].vol * sizeof(float));
         mg->off_fq = take(mg->lev[0].vol * sizeof(float));
     }
-    // the coarsest levels whose arrays fit in one block's shared memory (two levels at
-    // least, never level 0) run as one k_mg_bottom launch per V-cycle. In FP64 the block's
-    // SM does the levels' FP64 work alone (~2 FP64 instructions per cycle): levels above
-    // MG_BOTTOM_MAXVOL_FP64 cells are faster as grid launches spread over every SM.
+    // the coarsest levels (two at least, never level 0), up to bottom_maxvol cells, whose slabs
+    // fit in a block's shared memory, run as one k_mg_bottom launch per V-cycle
     mg->bottom = L;
     mg->bottom_smem = 0;
     {
-        size_t bytes = 0;
-        for (int l = L - 1; l >= 1 && L - l <= MG_BOTTOM_MAXLEV; --l) {
-            bytes += 3 * (size_t)mg->lev[l].vol * es;
+        for (int l = L - 2; l >= 1 && L - l <= MG_BOTTOM_MAXLEV; --l) {
+            if (mg->lev[l].vol > bottom_maxvol(precision)) break;
+            int n[MG_BOTTOM_MAXLEV][3];
+            const size_t bytes = (size_t)bottom_plan(n, bottom_extents(mg, l, n), bottom_solo(precision), nullptr) * es;
             if (bytes > MG_BOTTOM_SMEM) break;
-            if (precision != NYLES_MIXED && mg->lev[l].vol > MG_BOTTOM_MAXVOL_FP64) break;
-            if (L - l >= 2) {
-                mg->bottom = l;
-                mg->bottom_smem = bytes;
-            }
+            mg->bottom = l;
+            mg->bottom_smem = bytes;
         }
         if (mg->bottom < L) {
             cudaError_t e = precision == NYLES_MIXED
@@ -2477,20 +2665,22 @@ template <typename T>
 static void bottom(MgImpl* mg, cudaStream_t st) {
     const int l0 = mg->bottom;
     if (empty(mg, l0)) return;
+    const MgGeom g0 = mgg(mg, l0);
     MgBottom<T> a;
-    a.nlev = mg->nlevels - l0;
-    int off = 0;
-    for (int k = 0; k < a.nlev; ++k) {
-        a.g[k] = mgg(mg, l0 + k);
-        a.off[k] = off;
-        off += 3 * (int)mg->lev[l0 + k].vol;
+    for (int k = 0; k < 3; ++k) a.per[k] = mg->per[k];
+    for (int k = 0; k < 8; ++k) {
+        a.idiag[k] = sizeof(T) == sizeof(float) ? T(g0.fidiag[k]) : T(g0.idiag[k]);
+        a.pcoef[k] = sizeof(T) == sizeof(float) ? T(g0.fpcoef[k]) : T(g0.pcoef[k]);
     }
+    int n[MG_BOTTOM_MAXLEV][3];
+    a.nlev = bottom_extents(mg, l0, n);
+    bottom_plan(n, a.nlev, bottom_solo(mg->precision), a.lev);
+    a.resmooth = l0 + a.nlev < mg->nlevels;
     a.xg = lvp<T>(mg, l0, 1);
     a.bg = lvp<T>(mg, l0, 2);
-    a.omega = T(mg->omega);
     ProfScope ps(mg->prof, 8, st);
     note_launch();
-    k_mg_bottom<T><<<bgrid(mg, dim3(1, 1, 1)), MgBottomThreads<T>::n, mg->bottom_smem, st>>>(a, mg->bat);
+    k_mg_bottom<T><<<bgrid(mg, dim3(BT_CTAS, 1, 1)), BT_THREADS, mg->bottom_smem, st>>>(a, mg->bat);
 }
 
 // level0_last: mode of the last level-0 half-sweep (see smooth)
