@@ -324,166 +324,162 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, RhsMinBlocks<T>::n) k_rhs_march
 }
 
 // ---------------------------------------------------------------- right-hand side, 32-bit offsets
-// k_rhs_march<T, true, 1, false> (buoyancy advection, WENO vortex force, Bernoulli,
-// viscosity) for arrays of fewer than 2^31 cells: the same operations in the same order
-// (values equal up to where the compiler fuses multiply-adds), with fewer instructions
-// per cell:
-//  - 32-bit offsets; the six values around a face are loaded at offsets shared by every
-//    field read along that direction (x: constant offsets from one pointer; y and z:
-//    c + k sy and c + k sz formed once per cell);
+// k_rhs_march<float, true, 1, false> (buoyancy advection, WENO vortex force, Bernoulli,
+// viscosity) where a block's reach fits 32-bit byte offsets: the same operations in the same order
+// outside the reconstructions, with fewer instructions per cell:
+//  - 32-bit offsets from a block's own pointers; the six values around a face are loaded at
+//    offsets shared by every field read along that direction;
 //  - the upwind side is chosen among the six loaded values, so every reconstruction is
-//    one weno5 on registers (no data-dependent addresses);
+//    one weno5 on registers (no data-dependent addresses), written in differences;
 //  - the advecting velocity averaged at the face behind the cell, (UU0 of vf_flux),
 //    comes from the neighbouring lane along x and from the previous cell of the column
 //    along z instead of two more loads;
 //  - within three cells of an array end, where flux1d_at takes a closure branch, the
 //    reconstruction falls back to flux1d_at.
+// Bound by instruction issue (64% of cycles; 484 FP32 and 270 integer instructions per cell). Measured
+// against reconstructions from the values themselves, paired where two fields share a line:
+// 301 x 203 x 97 365 -> 328 us, 512 x 256 x 256 1433 -> 1289 us; a passive tracer there 907 -> 520 us
+// against k_tracer_march. Two rows of cells per thread with every reconstruction paired took 407
+// us (1 x 1 constants cost the paired form a move each, and its 128 registers leave 16 warps).
 
 // u * weno5 of the five values upwind of the face between v[2] and v[3] (flux1d_at's
-// interior branch): v[0..4] for u > 0, v[5..1] otherwise
-template <typename T>
-__device__ __forceinline__ T weno5_upwind(T u, const T (&v)[6]) {
-    const bool pos = u > T(0);
-    const T qa = pos ? v[0] : v[5];
-    const T qb = pos ? v[1] : v[4];
-    const T qc = pos ? v[2] : v[3];
-    const T qd = pos ? v[3] : v[2];
-    const T qe = pos ? v[4] : v[1];
-    return u * weno5(qa, qb, qc, qd, qe);
+// interior branch): v[0..4] for u > 0, v[5..1] otherwise. Written in differences of the line
+// (core/weno.f90:25-54 regrouped, as in nyles_line.cu): the indicators, carried as 4 (beta +
+// eps), take 18 instructions instead of 27, and the weights 6 and 3 ride in the constants.
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float weno5_upwind(float u, const float (&v)[6]) {
+    constexpr float c13 = 1.0f / 3.0f, c76 = 7.0f / 6.0f, c116 = 11.0f / 6.0f, c16 = 1.0f / 6.0f, c56 = 5.0f / 6.0f;
+    constexpr float k4 = 4.0f * (13.0f / 12.0f), eps4 = 4.0f * 1e-16f;
+    // sums of the candidates' coefficients (REAL(4) literals: not quite 1)
+    constexpr double s1 = (double)c13 - (double)c76 + (double)c116, s2 = (double)c56 + (double)c13 - (double)c16;
+    const bool pos = u > 0.f;
+    const float qa = pos ? v[0] : v[5], qb = pos ? v[1] : v[4], qc = pos ? v[2] : v[3], qd = pos ? v[3] : v[2],
+                qe = pos ? v[4] : v[1];
+    const float d0 = qb - qa, d1 = qc - qb, d2 = qd - qc, d3 = qe - qd;
+    const float e0 = d1 - d0, e1 = d2 - d1, e2 = d3 - d2;
+    auto ind = [&](float e, float s) { return fmaf(s, s, fmaf(k4 * e, e, eps4)); };
+    const float b1 = ind(e0, fmaf(3.f, d1, -d0)), b2 = ind(e1, d1 + d2), b3 = ind(e2, fmaf(-3.f, d2, d3));
+    const float tau = fabsf(b1 - b3);
+    // every denominator is at least 4e-16 (eps) or 1 and far below 2^126
+    const float w1 = fmaf(tau, rcp_approx(b1), 1.f), w2 = fmaf(tau, rcp_approx(b2), 1.f),
+                w3 = fmaf(tau, rcp_approx(b3), 1.f);
+    const float den = fmaf(3.f, w3, fmaf(6.f, w2, w1));
+    const float g1 = fmaf(c76 - c13, d1, fmaf(-c13, d0, (float)(s1 - s2) * qc));
+    const float g2 = fmaf(6.f * c13, d2, (6.f * c16) * d1);
+    const float g3 = fmaf(3.f * (c56 - c16), d2, (-3.f * c16) * d3);
+    const float num = fmaf(w3, g3, fmaf(w2, g2, w1 * g1));
+    return u * fmaf(num, rcp_approx(den), (float)s2 * qc);
 }
 
 // flux1d_at near an array end, out of line: the closures are rare (walls), and inlined
-// at the nine reconstruction sites they would multiply the kernel's code size
-template <typename T>
-__device__ __noinline__ T tr_flux_closure(const T* __restrict__ q, T u, int base, int i, int n, int s) {
-    auto Q = [&](int kk) -> T { return __ldg(q + base + kk * s); };
+// at the nine reconstruction sites they would multiply the kernel's code size. p: the line's
+// value at index i; vortex force: q(kk) = W(kk - 1), q(0) = 0.
+static __device__ __noinline__ float tr_flux_closure(const float* __restrict__ p, float u, int i, int n, int s) {
+    auto Q = [&](int kk) -> float { return __ldg(p + (long long)(kk - i) * s); };
     return flux1d_at(i, n, u, Q);
 }
-template <typename T>
-__device__ __noinline__ T vf_flux_closure(const T* __restrict__ W, T u1, int base, int i, int n, int s) {
-    auto Q = [&](int kk) -> T { return kk == 0 ? T(0) : __ldg(W + base + (kk - 1) * s); };
+static __device__ __noinline__ float vf_flux_closure(const float* __restrict__ p, float u1, int i, int n, int s) {
+    auto Q = [&](int kk) -> float { return kk == 0 ? 0.f : __ldg(p + (long long)(kk - 1 - i) * s); };
     return flux1d_at(i, n, u1, Q);
 }
 
-// tracer flux at index i of a line through c with stride s (flux1d_at of tr_flux);
-// o[k] = c + (k - 3) s
-template <typename T>
-__device__ __forceinline__ T tr_flux32(const T* __restrict__ q, T u, int c, int i, int n, int s, bool fast,
-                                       const int (&o)[7]) {
-    if (fast) {
-        T v[6];
+// Addresses: a block's cells and their stencils are reached from one point below the block's first
+// cell (the block's own pointer of each field) by unsigned byte offsets, so that the arrays may be of
+// any size; the offsets of a line are formed once for every field read along it.
+struct LineOff {
+    unsigned int o[7];   // cells -3 .. 3
+    __device__ __forceinline__ LineOff(unsigned int c, unsigned int s) {
 #pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = __ldg(q + o[k + 1]);
+        for (int k = 0; k < 7; ++k) o[k] = c + (unsigned int)(k - 3) * s;
+    }
+};
+__device__ __forceinline__ float ldo(const char* __restrict__ f, unsigned int off) {
+    return __ldg(reinterpret_cast<const float*>(f + off));
+}
+// flux of a tracer at index i of a line (flux1d_at of tr_flux), and of the vortex force given its
+// velocity (vf_flux); `fast`: i lies where flux1d_at takes its interior branch
+__device__ __forceinline__ float tr_flux32(const char* __restrict__ f, float u, const LineOff& l, int i, int n, int s,
+                                           bool fast) {
+    if (fast) {
+        float v[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) v[k] = ldo(f, l.o[k + 1]);
         return weno5_upwind(u, v);
     }
-    return tr_flux_closure(q, u, c - i * s, i, n, s);
+    return tr_flux_closure(reinterpret_cast<const float*>(f + l.o[3]), u, i, n, s);
 }
-// the same along x (stride 1: constant offsets)
-template <typename T>
-__device__ __forceinline__ T tr_flux32x(const T* __restrict__ q, T u, int c, int i, int n, bool fast) {
+__device__ __forceinline__ float vf_flux32(const char* __restrict__ f, float u, const LineOff& l, int i, int n, int s,
+                                           bool fast) {
     if (fast) {
-        T v[6];
+        float v[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = __ldg(q + c + (k - 2));
+        for (int k = 0; k < 6; ++k) v[k] = ldo(f, l.o[k]);
         return weno5_upwind(u, v);
     }
-    return tr_flux_closure(q, u, c - i, i, n, 1);
+    return vf_flux_closure(reinterpret_cast<const float*>(f + l.o[3]), u, i, n, s);
 }
 
-// ---- two FP32 reconstructions at once. Blackwell issues two FP32 lanes' worth of
-// multiply-adds in one paired instruction (__ffma2_rn, __fadd2_rn, __fmul2_rn), and the
-// FP32 right-hand side is bound by instruction issue: the two vortex-force fluxes that
-// share a direction (and so their load offsets) are reconstructed together. The same
-// formula as weno5<float>; the weights' divisions stay per component (hardware
-// reciprocal).
-__device__ __forceinline__ float2 f2s(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 weno5_x2(float2 qmm, float2 qm, float2 q0, float2 qp, float2 qpp) {
-    typedef WenoK<float> K;
-    const float2 qi1 = __ffma2_rn(f2s(K::c116()), q0, __ffma2_rn(f2s(-K::c76()), qm, __fmul2_rn(f2s(K::c13()), qmm)));
-    const float2 qi2 = __ffma2_rn(f2s(K::c13()), qp, __ffma2_rn(f2s(K::c56()), q0, __fmul2_rn(f2s(-K::c16()), qm)));
-    const float2 qi3 = __ffma2_rn(f2s(-K::c16()), qpp, __ffma2_rn(f2s(K::c56()), qp, __fmul2_rn(f2s(K::c13()), q0)));
-    const float2 a1 = __fadd2_rn(__ffma2_rn(f2s(-2.f), qm, qmm), q0);
-    const float2 b1 = __ffma2_rn(f2s(3.f), q0, __ffma2_rn(f2s(-4.f), qm, qmm));
-    const float2 a2 = __fadd2_rn(__ffma2_rn(f2s(-2.f), q0, qm), qp);
-    const float2 b2 = __ffma2_rn(f2s(-1.f), qp, qm);
-    const float2 a3 = __fadd2_rn(__ffma2_rn(f2s(-2.f), qp, q0), qpp);
-    const float2 b3 = __fadd2_rn(__ffma2_rn(f2s(-4.f), qp, __fmul2_rn(f2s(3.f), q0)), qpp);
-    auto beta = [&](float2 a, float2 b) {
-        return __ffma2_rn(__fmul2_rn(f2s(K::k1()), a), a, __fmul2_rn(__fmul2_rn(f2s(0.25f), b), b));
-    };
-    const float2 be1 = beta(a1, b1), be2 = beta(a2, b2), be3 = beta(a3, b3);
-    const float2 t = __ffma2_rn(f2s(-1.f), be3, be1);
-    const float2 tau5 = make_float2(fabsf(t.x), fabsf(t.y));
-    const float2 d1 = __fadd2_rn(be1, f2s(K::eps5())), d2 = __fadd2_rn(be2, f2s(K::eps5())),
-                 d3 = __fadd2_rn(be3, f2s(K::eps5()));
-    const float2 r1 = make_float2(__fdividef(tau5.x, d1.x), __fdividef(tau5.y, d1.y));
-    const float2 r2 = make_float2(__fdividef(tau5.x, d2.x), __fdividef(tau5.y, d2.y));
-    const float2 r3 = make_float2(__fdividef(tau5.x, d3.x), __fdividef(tau5.y, d3.y));
-    const float2 w1 = __fadd2_rn(f2s(1.f), r1);
-    const float2 w2 = __fmul2_rn(f2s(6.f), __fadd2_rn(f2s(1.f), r2));
-    const float2 w3 = __fmul2_rn(f2s(3.f), __fadd2_rn(f2s(1.f), r3));
-    const float2 num = __ffma2_rn(w3, qi3, __ffma2_rn(w2, qi2, __fmul2_rn(w1, qi1)));
-    const float2 den = __fadd2_rn(__fadd2_rn(w1, w2), w3);
-    return make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
-}
-// u * weno5_x2 of the five values upwind of the face, each component on its own side
-__device__ __forceinline__ float2 weno5_upwind_x2(float2 u, const float2 (&v)[6]) {
-    const bool px = u.x > 0.f, py = u.y > 0.f;
-    auto sel = [&](int a, int b) { return make_float2(px ? v[a].x : v[b].x, py ? v[a].y : v[b].y); };
-    return __fmul2_rn(u, weno5_x2(sel(0, 5), sel(1, 4), sel(2, 3), sel(3, 2), sel(4, 1)));
-}
-// vf_flux32 of two vorticity fields along one direction (offsets o shared)
-__device__ __forceinline__ float2 vf_flux32_x2(const float* __restrict__ Wa, const float* __restrict__ Wb, float2 u1,
-                                               int c, int i, int n, int s, bool fast, const int (&o)[7]) {
-    if (fast) {
-        float2 v[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = make_float2(__ldg(Wa + o[k]), __ldg(Wb + o[k]));
-        return weno5_upwind_x2(u1, v);
+// One tracer in a block of RZ_BX x RZ_BY columns: -(flux divergence), summed as TracerMarch::step
+// (x, y, z), with the faces shared as there
+struct TracerMarch32 {
+    float fz_prev;
+    // u*: the velocity along each axis at the cell; every thread of the block must call it
+    __device__ __forceinline__ float step(const char* __restrict__ f, const char* __restrict__ fU0,
+                                          const char* __restrict__ fU1, float u0, float u1, float u2, const LineOff& lx,
+                                          const LineOff& ly, const LineOff& lz, int z, int ys, int xs, int sy, int sz,
+                                          int Nz, int Ny, int Nx, float (*sfy)[RZ_BX]) {
+        const int tx = threadIdx.x, ty = threadIdx.y;
+        const float fz = tr_flux32(f, u2, lz, z, Nz, sz, z >= 2 && z <= Nz - 4);
+        const float fy = tr_flux32(f, u1, ly, ys, Ny, sy, ys >= 2 && ys <= Ny - 4);
+        sfy[ty][tx] = fy;
+        __syncthreads();
+        float fym = (ty > 0) ? sfy[ty - 1][tx] : 0.f;
+        __syncthreads();
+        if (ty == 0 && ys > 0)   // the face below the block's first row
+            fym = tr_flux32(f, ldo(fU1, ly.o[2]), LineOff(ly.o[2], sy * 4u), ys - 1, Ny, sy, ys - 1 >= 2 && ys - 1 <= Ny - 4);
+        const float fx = tr_flux32(f, u0, lx, xs, Nx, 1, xs >= 2 && xs <= Nx - 4);
+        float fxm = __shfl_up_sync(0xffffffffu, fx, 1);
+        if (tx == 0 && xs > 0)
+            fxm = tr_flux32(f, ldo(fU0, lx.o[2]), LineOff(lx.o[2], 4u), xs - 1, Nx, 1, xs - 1 >= 2 && xs - 1 <= Nx - 4);
+        float db = (xs > 0) ? (0.f + fxm) - fx : 0.f - fx;
+        db = (ys > 0) ? (db + fym) - fy : db - fy;
+        db = (z > 0) ? (db + fz_prev) - fz : db - fz;
+        fz_prev = fz;
+        return db;
     }
-    return make_float2(vf_flux_closure(Wa, u1.x, c - i * s, i, n, s), vf_flux_closure(Wb, u1.y, c - i * s, i, n, s));
-}
-__device__ __forceinline__ float2 vf_flux32x_x2(const float* __restrict__ Wa, const float* __restrict__ Wb, float2 u1,
-                                                int c, int i, int n, bool fast) {
-    if (fast) {
-        float2 v[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = make_float2(__ldg(Wa + c + (k - 3)), __ldg(Wb + c + (k - 3)));
-        return weno5_upwind_x2(u1, v);
-    }
-    return make_float2(vf_flux_closure(Wa, u1.x, c - i, i, n, 1), vf_flux_closure(Wb, u1.y, c - i, i, n, 1));
-}
+};
 
-// vortex-force reconstruction of vf_flux given u1: q(kk) = W(kk - 1), q(0) = 0
-template <typename T>
-__device__ __forceinline__ T vf_flux32(const T* __restrict__ W, T u1, int c, int i, int n, int s, bool fast,
-                                       const int (&o)[7]) {
-    if (fast) {
-        T v[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = __ldg(W + o[k]);
-        return weno5_upwind(u1, v);
+// a block's columns: thread positions, the byte offset of a thread's cell at plane z0, and the
+// distance from a field's start to the point the offsets count from
+struct Block32 {
+    int x, y, xs, ys, z0, z1;
+    unsigned int c0;
+    long long org;
+    __device__ __forceinline__ Block32(const int* lo, const int* hi, int bz, int zc, int sy, int sz) {
+        const int bx = lo[2] + blockIdx.x * RZ_BX, by = lo[1] + blockIdx.y * RZ_BY;
+        x = bx + threadIdx.x;
+        y = by + threadIdx.y;
+        xs = min(x, hi[2] - 1);   // idle lanes shadow a real cell
+        ys = min(y, hi[1] - 1);
+        z0 = lo[0] + bz * zc;
+        z1 = min(z0 + zc, hi[0]);
+        // bx, by may lie beyond hi by less than a block: count from the shadowed cells' side
+        const int ox = min(bx, hi[2] - 1) - 3, oy = min(by, hi[1] - 1) - 3, oz = z0 - 3;
+        org = 4ll * ((long long)oz * sz + (long long)oy * sy + ox);
+        c0 = 4u * (3u * (unsigned int)sz + (unsigned int)(ys - oy) * (unsigned int)sy + (unsigned int)(xs - ox));
     }
-    return vf_flux_closure(W, u1, c - i * s, i, n, s);
-}
-template <typename T>
-__device__ __forceinline__ T vf_flux32x(const T* __restrict__ W, T u1, int c, int i, int n, bool fast) {
-    if (fast) {
-        T v[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = __ldg(W + c + (k - 3));
-        return weno5_upwind(u1, v);
-    }
-    return vf_flux_closure(W, u1, c - i, i, n, 1);
-}
+};
 
 // blocks per SM asked of the register allocator: 48 registers (the closure branches out
-// of line; inlined, they took it to 64). The paired reconstructions spill a few values
-// at 48 and still beat 4 blocks per SM at 64 registers (2.28 vs 2.41 ms per 256^3 step)
+// of line; inlined, they took it to 64)
 template <typename T> struct LesMinBlocks { static constexpr int n = 5; };
 
 template <typename T, bool BAT>
-__global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(const RhsArgs<T> a0,
+__global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(const RhsArgs<T> a0, const int zc,
                                                                              const Bat bat = Bat()) {
     __shared__ T sfy[RZ_BY][RZ_BX];
     int bz = blockIdx.z;
@@ -493,143 +489,86 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(c
         if (!batch_enter(bat, bz, dlt)) return;
         shift_rhs_args(a, dlt);
     }
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x = a.lo[2] + blockIdx.x * RZ_BX + tx;
-    const int y = a.lo[1] + blockIdx.y * RZ_BY + ty;
-    const int z0 = a.lo[0] + bz * RZ_ZC;
-    const int z1 = min(z0 + RZ_ZC, a.hi[0]) - 1;
     const int Nz = a.g.N[0], Ny = a.g.N[1], Nx = a.g.N[2];
     const int sy = (int)a.g.sy, sz = (int)a.g.sz;
-    const bool valid = x < a.hi[2] && y < a.hi[1];
-    const int xs = min(x, a.hi[2] - 1), ys = min(y, a.hi[1] - 1);   // idle lanes shadow a real cell
-    const T* __restrict__ b = a.b;
-    const T* __restrict__ U0 = a.U[0];
-    const T* __restrict__ U1 = a.U[1];
-    const T* __restrict__ U2 = a.U[2];
-    const T* __restrict__ W0 = a.W[0];
-    const T* __restrict__ W1 = a.W[1];
-    const T* __restrict__ W2 = a.W[2];
-    const T* __restrict__ ke = a.ke;
-    // interior reconstructions: tracer 2 <= i <= n - 4, vortex force 3 <= i <= n - 4
-    const bool xt = xs >= 2 && xs <= Nx - 4, xv = xs >= 3 && xs <= Nx - 4;
-    const bool yt = ys >= 2 && ys <= Ny - 4, yv = ys >= 3 && ys <= Ny - 4;
+    const Block32 k(a.lo, a.hi, bz, zc, sy, sz);
+    const int xs = k.xs, ys = k.ys, tx = threadIdx.x;
+    const bool valid = k.x < a.hi[2] && k.y < a.hi[1];
+    auto fld = [&](const T* p) { return reinterpret_cast<const char*>(p) + k.org; };
+    const char* __restrict__ b = fld(a.b);
+    const char* __restrict__ U0 = fld(a.U[0]);
+    const char* __restrict__ U1 = fld(a.U[1]);
+    const char* __restrict__ U2 = fld(a.U[2]);
+    const char* __restrict__ W0 = fld(a.W[0]);
+    const char* __restrict__ W1 = fld(a.W[1]);
+    const char* __restrict__ W2 = fld(a.W[2]);
+    const char* __restrict__ ke = fld(a.ke);
+    const unsigned int by = 4u * (unsigned int)sy, bzs = 4u * (unsigned int)sz;
+    // interior vortex-force reconstructions: 3 <= i <= n - 4
+    const bool xv = xs >= 3 && xs <= Nx - 4, yv = ys >= 3 && ys <= Ny - 4;
     const bool ylo = ys < Ny - 1, xlo = xs < Nx - 1;
-    const int cxy = ys * sy + xs;
     // carried up the column: the tracer flux through the face below the cell and the
     // two z-fluxes' velocities averaged at that face
-    T fz_prev = T(0), uu_zy = T(0), uu_zx = T(0);
-    if (z0 > 0) {
-        const int c = (z0 - 1) * sz + cxy;
-        int oz[7];
-#pragma unroll
-        for (int k = 0; k < 7; ++k) oz[k] = c + (k - 3) * sz;
-        const int zm = z0 - 1;
-        fz_prev = tr_flux32(b, __ldg(U2 + c), c, zm, Nz, sz, zm >= 2 && zm <= Nz - 4, oz);
-        if (ylo) uu_zy = T(0.5) * (__ldg(U2 + c) + __ldg(U2 + c + sy));
-        if (xlo) uu_zx = T(0.5) * (__ldg(U2 + c) + __ldg(U2 + c + 1));
+    TracerMarch32 tm;
+    tm.fz_prev = 0.f;
+    T uu_zy = T(0), uu_zx = T(0);
+    if (k.z0 > 0) {
+        const int zm = k.z0 - 1;
+        const LineOff lz(k.c0 - bzs, bzs);
+        const T u = ldo(U2, lz.o[3]);
+        tm.fz_prev = tr_flux32(b, u, lz, zm, Nz, sz, zm >= 2 && zm <= Nz - 4);
+        if (ylo) uu_zy = T(0.5) * (u + ldo(U2, lz.o[3] + by));
+        if (xlo) uu_zx = T(0.5) * (u + ldo(U2, lz.o[3] + 4u));
     }
-    for (int z = z0; z <= z1; ++z) {
-        const int c = z * sz + cxy;
-        const bool zt = z >= 2 && z <= Nz - 4, zv = z >= 3 && z <= Nz - 4;
-        const bool zlo = z < Nz - 1;
-        // The fluxes are formed direction by direction (z, y, x: one set of offsets
-        // live at a time) and summed afterwards in the order of TracerMarch::step and
-        // vortex_force_cell.
-        T fz, f4 = T(0), f5 = T(0);
+    unsigned int c = k.c0;
+    for (int z = k.z0; z < k.z1; ++z, c += bzs) {
+        const bool zv = z >= 3 && z <= Nz - 4, zlo = z < Nz - 1;
+        const T u0 = ldo(U0, c), u1 = ldo(U1, c), u2 = ldo(U2, c);
+        // The vortex-force fluxes are formed direction by direction (one set of offsets live at a
+        // time) and summed afterwards in the order of vortex_force_cell.
+        T f1 = T(0), f2 = T(0), f3 = T(0), f4 = T(0), f5 = T(0), f6 = T(0);
+        const LineOff lz(c, bzs), ly(c, by), lx(c, 4u);
+        // f4 (ylo): u_j += U^k w_i along k (U^k averaged along j); f5 (xlo): u_i -= U^k w_j along
+        // k (U^k averaged along i)
+        if (ylo) {
+            const T uu1 = T(0.5) * (u2 + ldo(U2, c + by)), uu0 = z > 0 ? uu_zy : T(0);
+            uu_zy = uu1;
+            f4 = vf_flux32(W0, T(0.5) * (uu0 + uu1), lz, z, Nz, sz, zv);
+        }
+        if (xlo) {
+            const T uu1 = T(0.5) * (u2 + ldo(U2, c + 4u)), uu0 = z > 0 ? uu_zx : T(0);
+            uu_zx = uu1;
+            f5 = vf_flux32(W1, T(0.5) * (uu0 + uu1), lz, z, Nz, sz, zv);
+        }
+        // f2 (xlo): u_i += U^j w_k along j (U^j averaged along i); f3 (zlo): u_k -= U^j w_i along
+        // j (U^j averaged along k)
+        if (xlo) {
+            const T uu1 = T(0.5) * (u1 + ldo(U1, c + 4u));
+            const T uu0 = ys > 0 ? T(0.5) * (ldo(U1, c - by) + ldo(U1, c - by + 4u)) : T(0);
+            f2 = vf_flux32(W2, T(0.5) * (uu0 + uu1), ly, ys, Ny, sy, yv);
+        }
+        if (zlo) {
+            const T uu1 = T(0.5) * (u1 + ldo(U1, c + bzs));
+            const T uu0 = ys > 0 ? T(0.5) * (ldo(U1, c - by) + ldo(U1, c - by + bzs)) : T(0);
+            f3 = vf_flux32(W0, T(0.5) * (uu0 + uu1), ly, ys, Ny, sy, yv);
+        }
+        // f1 (ylo): u_j -= U^i w_k along i (U^i averaged along j); f6 (zlo): u_k += U^i w_j along
+        // i (U^i averaged along k)
         {
-            int oz[7];
-#pragma unroll
-            for (int k = 0; k < 7; ++k) oz[k] = c + (k - 3) * sz;
-            fz = tr_flux32(b, __ldg(U2 + c), c, z, Nz, sz, zt, oz);
-            // f4 (ylo): u_j += U^k w_i along k (U^k averaged along j); f5 (xlo): u_i -= U^k
-            // w_j along k (U^k averaged along i); reconstructed as a pair
-            float2 u45 = make_float2(0.f, 0.f);
-            if (ylo) {
-                const T uu1 = T(0.5) * (__ldg(U2 + c) + __ldg(U2 + c + sy));
-                const T uu0 = z > 0 ? uu_zy : T(0);
-                uu_zy = uu1;
-                u45.x = T(0.5) * (uu0 + uu1);
+            const T uy = ylo ? T(0.5) * (u0 + ldo(U0, c + by)) : T(0), uz = zlo ? T(0.5) * (u0 + ldo(U0, c + bzs)) : T(0);
+            T my = __shfl_up_sync(0xffffffffu, uy, 1), mz = __shfl_up_sync(0xffffffffu, uz, 1);
+            if (tx == 0) {
+                my = mz = T(0);
+                if (xs > 0) {
+                    const T um = ldo(U0, c - 4u);
+                    if (ylo) my = T(0.5) * (um + ldo(U0, c - 4u + by));
+                    if (zlo) mz = T(0.5) * (um + ldo(U0, c - 4u + bzs));
+                }
             }
-            if (xlo) {
-                const T uu1 = T(0.5) * (__ldg(U2 + c) + __ldg(U2 + c + 1));
-                const T uu0 = z > 0 ? uu_zx : T(0);
-                uu_zx = uu1;
-                u45.y = T(0.5) * (uu0 + uu1);
-            }
-            if (ylo || xlo) {
-                const float2 f45 = vf_flux32_x2(W0, W1, u45, c, z, Nz, sz, zv, oz);
-                f4 = f45.x;
-                f5 = f45.y;
-            }
+            if (ylo) f1 = vf_flux32(W2, T(0.5) * (my + uy), lx, xs, Nx, 1, xv);
+            if (zlo) f6 = vf_flux32(W1, T(0.5) * (mz + uz), lx, xs, Nx, 1, xv);
         }
-        T fy, fym, f2 = T(0), f3 = T(0);
-        {
-            int oy[7];
-#pragma unroll
-            for (int k = 0; k < 7; ++k) oy[k] = c + (k - 3) * sy;
-            fy = tr_flux32(b, __ldg(U1 + c), c, ys, Ny, sy, yt, oy);
-            sfy[ty][tx] = fy;
-            __syncthreads();
-            fym = (ty > 0) ? sfy[ty - 1][tx] : T(0);
-            __syncthreads();
-            // f2 (xlo): u_i += U^j w_k along j (U^j averaged along i); f3 (zlo): u_k -= U^j
-            // w_i along j (U^j averaged along k)
-            float2 u23 = make_float2(0.f, 0.f);
-            if (xlo) {
-                const T uu1 = T(0.5) * (__ldg(U1 + c) + __ldg(U1 + c + 1));
-                const T uu0 = ys > 0 ? T(0.5) * (__ldg(U1 + c - sy) + __ldg(U1 + c - sy + 1)) : T(0);
-                u23.x = T(0.5) * (uu0 + uu1);
-            }
-            if (zlo) {
-                const T uu1 = T(0.5) * (__ldg(U1 + c) + __ldg(U1 + c + sz));
-                const T uu0 = ys > 0 ? T(0.5) * (__ldg(U1 + c - sy) + __ldg(U1 + c - sy + sz)) : T(0);
-                u23.y = T(0.5) * (uu0 + uu1);
-            }
-            if (xlo || zlo) {
-                const float2 f23 = vf_flux32_x2(W2, W0, u23, c, ys, Ny, sy, yv, oy);
-                f2 = f23.x;
-                f3 = f23.y;
-            }
-        }
-        if (ty == 0 && ys > 0) {   // the face below the block's first row
-            const int cm = c - sy;
-            int om[7];
-#pragma unroll
-            for (int k = 0; k < 7; ++k) om[k] = cm + (k - 3) * sy;
-            fym = tr_flux32(b, __ldg(U1 + cm), cm, ys - 1, Ny, sy, ys - 1 >= 2 && ys - 1 <= Ny - 4, om);
-        }
-        T fx, fxm, f1 = T(0), f6 = T(0);
-        {
-            fx = tr_flux32x(b, __ldg(U0 + c), c, xs, Nx, xt);
-            fxm = __shfl_up_sync(0xffffffffu, fx, 1);
-            if (tx == 0 && xs > 0) fxm = tr_flux32x(b, __ldg(U0 + c - 1), c - 1, xs - 1, Nx,
-                                                     xs - 1 >= 2 && xs - 1 <= Nx - 4);
-            // f1 (ylo): u_j -= U^i w_k along i (U^i averaged along j); f6 (zlo): u_k += U^i
-            // w_j along i (U^i averaged along k)
-            float2 u16 = make_float2(0.f, 0.f);
-            if (ylo) {
-                const T uu1 = T(0.5) * (__ldg(U0 + c) + __ldg(U0 + c + sy));
-                T uu0 = __shfl_up_sync(0xffffffffu, uu1, 1);
-                if (tx == 0) uu0 = xs > 0 ? T(0.5) * (__ldg(U0 + c - 1) + __ldg(U0 + c - 1 + sy)) : T(0);
-                u16.x = T(0.5) * (uu0 + uu1);
-            }
-            if (zlo) {
-                const T uu1 = T(0.5) * (__ldg(U0 + c) + __ldg(U0 + c + sz));
-                T uu0 = __shfl_up_sync(0xffffffffu, uu1, 1);
-                if (tx == 0) uu0 = xs > 0 ? T(0.5) * (__ldg(U0 + c - 1) + __ldg(U0 + c - 1 + sz)) : T(0);
-                u16.y = T(0.5) * (uu0 + uu1);
-            }
-            if (ylo || zlo) {
-                const float2 f16 = vf_flux32x_x2(W2, W1, u16, c, xs, Nx, xv);
-                f1 = f16.x;
-                f6 = f16.y;
-            }
-        }
-        // ---- buoyancy advection, summed as TracerMarch::step
-        T db = (xs > 0) ? (T(0) + fxm) - fx : T(0) - fx;
-        db = (ys > 0) ? (db + fym) - fy : db - fy;
-        db = (z > 0) ? (db + fz_prev) - fz : db - fz;
-        fz_prev = fz;
+        const T db = tm.step(b, U0, U1, u0, u1, u2, lx, ly, lz, z, ys, xs, sy, sz, Nz, Ny, Nx, sfy);
         // ---- vortex force, summed in the order of vortex_force_cell
         T dux = T(0), duy = T(0), duz = T(0);
         if (ylo) duy = duy - f1;
@@ -639,14 +578,15 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(c
         if (xlo) dux = dux - f5;
         if (zlo) duz = duz + f6;
         // ---- Bernoulli (core/bernoulli.py:14-23)
-        if (xlo) dux = sub_rn(dux, sub_rn(__ldg(ke + c + 1), __ldg(ke + c)));
-        if (ylo) duy = sub_rn(duy, sub_rn(__ldg(ke + c + sy), __ldg(ke + c)));
+        const T k0 = ldo(ke, c);
+        if (xlo) dux = sub_rn(dux, sub_rn(ldo(ke, c + 4u), k0));
+        if (ylo) duy = sub_rn(duy, sub_rn(ldo(ke, c + by), k0));
         if (zlo) {
-            duz = sub_rn(duz, sub_rn(__ldg(ke + c + sz), __ldg(ke + c)));
-            if (!a.euler) duz = add_rn(duz, mul_rn(a.half_dz, add_rn(__ldg(b + c + sz), __ldg(b + c))));
+            duz = sub_rn(duz, sub_rn(ldo(ke, c + bzs), k0));
+            if (!a.euler) duz = add_rn(duz, mul_rn(a.half_dz, add_rn(ldo(b, c + bzs), ldo(b, c))));
         }
+        const long long cl = ((long long)z * sz + (long long)ys * sy) + xs;
         if (a.terms & TERM_VISC) {
-            const long long cl = c;
             const int pos[3] = {z, ys, xs};
             for (int pass = 0; pass < 3; ++pass) {
                 const int d = 2 - pass;
@@ -657,11 +597,38 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(c
             }
         }
         if (valid) {
-            a.ds[0][c] = db;
-            a.ds[1][c] = dux;
-            a.ds[2][c] = duy;
-            a.ds[3][c] = duz;
+            a.ds[0][cl] = db;
+            a.ds[1][cl] = dux;
+            a.ds[2][cl] = duy;
+            a.ds[3][cl] = duz;
         }
+    }
+}
+
+// the same for one passive tracer over the whole arrays (core/tracer.py:59-72)
+__global__ void __launch_bounds__(RZ_BX * RZ_BY, 5) k_tracer_les(const Geom g, const float* __restrict__ Ux,
+                                                               const float* __restrict__ Uy, const float* __restrict__ Uz,
+                                                               const float* __restrict__ q, float* __restrict__ dq,
+                                                               const int zc) {
+    __shared__ float sfy[RZ_BY][RZ_BX];
+    const int sy = (int)g.sy, sz = (int)g.sz, lo[3] = {0, 0, 0};
+    const Block32 k(lo, g.N, blockIdx.z, zc, sy, sz);
+    const bool valid = k.x < g.N[2] && k.y < g.N[1];
+    auto fld = [&](const float* p) { return reinterpret_cast<const char*>(p) + k.org; };
+    const char *U0 = fld(Ux), *U1 = fld(Uy), *U2 = fld(Uz), *f = fld(q);
+    const unsigned int by = 4u * (unsigned int)sy, bzs = 4u * (unsigned int)sz;
+    TracerMarch32 tm;
+    tm.fz_prev = 0.f;
+    if (k.z0 > 0) {
+        const int zm = k.z0 - 1;
+        const LineOff lz(k.c0 - bzs, bzs);
+        tm.fz_prev = tr_flux32(f, ldo(U2, lz.o[3]), lz, zm, g.N[0], sz, zm >= 2 && zm <= g.N[0] - 4);
+    }
+    unsigned int c = k.c0;
+    for (int z = k.z0; z < k.z1; ++z, c += bzs) {
+        const float v = tm.step(f, U0, U1, ldo(U0, c), ldo(U1, c), ldo(U2, c), LineOff(c, 4u), LineOff(c, by),
+                                LineOff(c, bzs), z, k.ys, k.xs, sy, sz, g.N[0], g.N[1], g.N[2], sfy);
+        if (valid) dq[g.at(z, k.ys, k.xs)] = v;
     }
 }
 
@@ -755,14 +722,25 @@ __global__ void __launch_bounds__(256) k_tracer_linear(const Geom g, const T* __
     dq[c] = acc;
 }
 
-// k_rhs_les serves FP32 arrays of fewer than 2^31 cells (32-bit offsets, the largest
-// one c + 3 sz + sy + 1 below 2^31); NYLES_GB300_GENERIC_RHS=1 selects k_rhs_march
-// instead (the same operations; values equal to rounding). The FP64 right-hand side
-// keeps k_rhs_march: it is bound by the FP64 pipe, and k_rhs_les (80 registers, 3
-// blocks per SM) ran it in the same time.
+// k_rhs_les serves FP32 arrays whose 22 planes (a block's reach) lie within 4 GB; NYLES_GB300_GENERIC_RHS=1
+// selects k_rhs_march instead (values equal to rounding).
+// Planes per thread of the FP32 marches: 16 where that gives every SM its five blocks, fewer on small
+// grids (each thread starts with the flux below its first plane, a tenth of a plane's work): 16 / 2
+// planes of a 48^3 right-hand side (36 / 288 blocks) 118 / 19 us.
+static int rhs32_chunk(long long columns, int nz) {
+    int zc = 16;
+    while (zc > 2 && columns * ((nz + zc - 1) / zc) < 152 * 5) zc /= 2;
+    return zc;
+}
+
 template <typename T, bool BAT>
 static void launch_rhs_les(dim3 grd, dim3 blk, cudaStream_t st, const RhsArgs<T>& a, const Bat& bat) {
-    if constexpr (sizeof(T) == sizeof(float)) k_rhs_les<T, BAT><<<grd, blk, 0, st>>>(a, bat);
+    if constexpr (sizeof(T) == sizeof(float)) {
+        const int nz = a.hi[0] - a.lo[0], nrun = BAT ? bat.nrun : 1;
+        const int zc = rhs32_chunk((long long)grd.x * grd.y * nrun, nz);
+        grd.z = (unsigned)((nz + zc - 1) / zc * nrun);
+        k_rhs_les<T, BAT><<<grd, blk, 0, st>>>(a, zc, bat);
+    }
 }
 
 template <typename T>
@@ -772,7 +750,7 @@ static bool rhs32_ok(const Geom& g) {
         const char* e = getenv("NYLES_GB300_GENERIC_RHS");
         return e && e[0] == '1';
     }();
-    return !generic && g.vol + 4 * g.sz + g.sy + 1 < (1ll << 31);
+    return !generic && 4 * (22 * g.sz + 16 * g.sy + 64) < (1ll << 32);
 }
 
 bool make_geom(const NylesDesc* d, Geom* g) {
@@ -854,6 +832,17 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
                                                             kc[0], kc[1], kc[2]);
         note_launch();
     };
+    auto tracer32 = [&](const T* q, T* dq) {   // FP32, no diffusion
+        if constexpr (sizeof(T) == sizeof(float)) {
+            if (rhs32_ok<T>(g)) {
+                const int zc = rhs32_chunk((long long)grd.x * grd.y, g.N[0]);
+                const dim3 gt(grd.x, grd.y, (unsigned)((g.N[0] + zc - 1) / zc));
+                k_tracer_les<<<gt, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], q, dq, zc);
+            } else {
+                k_tracer_march<T, false><<<grd, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], q, dq, T(0), T(0), T(0));
+            }
+        }
+    };
     if (d->model == NYLES_MODEL_ADVECTION) {
         // Advection.rhs (core/model_advection.py:59-61): b only; the velocity registers
         // are not touched (the reference never writes them)
@@ -865,8 +854,7 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
                 k_tracer_march<T, true><<<grd, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], a.b, a.ds[0], kc[0], kc[1],
                                                              kc[2]);
             else
-                k_tracer_march<T, false><<<grd, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], a.b, a.ds[0], T(0), T(0),
-                                                              T(0));
+                tracer32(a.b, a.ds[0]);
             note_launch();
         }
         return cuda_status(cudaGetLastError(), "rhs kernel");
@@ -930,8 +918,7 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
                 k_tracer_march<T, true><<<grd, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], a.tr[t], a.ds[4 + t],
                                                              kc[0], kc[1], kc[2]);
             else
-                k_tracer_march<T, false><<<grd, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], a.tr[t], a.ds[4 + t],
-                                                              T(0), T(0), T(0));
+                tracer32(a.tr[t], a.ds[4 + t]);
             note_launch();
         } else {   // Euler3d: tracers are not advected, their tendency is zero (reset_state)
             cudaMemsetAsync(a.ds[4 + t], 0, sizeof(T) * g.vol, st);
