@@ -2353,15 +2353,43 @@ static inline dim3 grid_v4(const int n[3], int zc = V4_ZC) {
     return dim3((unsigned)((n[2] / 4 + MG_BX - 1) / MG_BX), (unsigned)((n[1] + MG_BY - 1) / MG_BY),
                 (unsigned)(n[0] / zc));
 }
-// z cells per thread of the half-sweeps of level l: level 0 reuses each z row from
-// registers over V4_ZC cells; the coarser levels are latency-bound (a few microseconds
-// per launch whatever their size), where more blocks with shorter chains of dependent
-// loads finish sooner
-static inline int lvl_zc(const MgImpl* mg, int l) { return l == 0 ? V4_ZC : mg->czc; }
+// Block partials of a level-0 sum over `count` blocks (which = 0, 1: two sums of one kernel): in
+// the workspace's own slots where these hold them, else in level 1's y, which holds nothing while
+// the kernels that sum over level 0 run.
+static inline long long blocks(dim3 g) { return (long long)g.x * g.y * g.z; }
+static inline bool partials_fit(const MgImpl* mg, long long count) {
+    const long long es = mg->precision == NYLES_MIXED ? sizeof(float) : sizeof(double);
+    return count <= mg->npartial || (mg->nlevels > 1 && mg->lev[1].vol * es >= 2 * count * (long long)sizeof(double));
+}
+static double* partials(const MgImpl* mg, int which, long long count) {
+    if (count <= mg->npartial)
+        return reinterpret_cast<double*>(mg->ws + (which ? mg->off_partial2 : mg->off_partial));
+    return reinterpret_cast<double*>(mg->ws + mg->lev[1].off_y) + which * count;
+}
+
+// Whether the kernels that sum over level 0 (residual, Krylov) take their vector form: on narrow
+// levels its blocks can be more than the workspace has slots for partials (nx <= 32 of 32 lanes x 4).
+static inline bool use_v4_sums(const MgImpl* mg) {
+    return use_v4(mg, mg->lev[0].n) && partials_fit(mg, blocks(grid_v4(mg->lev[0].n)));
+}
+// z cells per thread of the half-sweeps of level l that keep no sums (0: the scalar kernel). A large
+// level 0, and one of a batch, reuses each z row from registers over V4_ZC cells; the coarser levels
+// and a small level 0 are latency-bound (a few microseconds per launch whatever their size), where
+// more blocks with shorter chains of dependent loads finish sooner. Mixed time steps with 4 / 1
+// planes (us): 48^3 981 / 890, 64 x 64 x 32 1103 / 1008, 128 x 64 x 64 1203 / 1109, 96^3 1415 / 1379,
+// 128 x 128 x 64 1555 / 1566; ten steps of four 48^3 runs 12.91 / 12.91 ms, of eight 16.64 / 17.61, of
+// sixteen 32^3 runs 14.72 / 15.46. The residual stays at 4 planes: one per thread, it gains 3% of a 64 x 64 x 32
+// step and loses 2% of a 64^3 one and 7% of eight batched 32^3 runs.
+constexpr long long V4_SMALL = 1 << 20;
+static inline int lvl_zc(const MgImpl* mg, int l) {
+    if (l) return mg->czc;
+    if (!mg->bat.tab && mg->lev[0].vol < V4_SMALL) return 1;
+    return V4_ZC;
+}
 // coarse planes per thread of the restriction out of level l, fine planes per thread of
 // the prolongation into level l (even)
-static inline int lvl_rzc(const MgImpl* mg, int l) { return l == 0 ? MG_RZC : (mg->czc >= 4 ? MG_RZC : 1); }
-static inline int lvl_pzc(const MgImpl* mg, int l) { return l == 0 ? V4_ZC : (mg->czc >= 4 ? V4_ZC : 2); }
+static inline int lvl_rzc(const MgImpl* mg, int l) { return lvl_zc(mg, l) >= 4 ? MG_RZC : 1; }
+static inline int lvl_pzc(const MgImpl* mg, int l) { return lvl_zc(mg, l) >= 4 ? V4_ZC : 2; }
 static inline dim3 grid_v4_restrict(const MgGeom& gf, const MgGeom& gc, int rzc) {
     return dim3((unsigned)((gf.n[2] / 4 + MG_BX - 1) / MG_BX), (unsigned)((gc.n[1] + MG_BY - 1) / MG_BY),
                 (unsigned)(gc.n[0] / rzc));
@@ -2398,6 +2426,15 @@ static void launch_jacobi_v4_0(int zc, dim3 grd, cudaStream_t st, const MgGeom& 
         k_mg_jacobi_v4<0, BAT, 2><<<grd, kBlk, 0, st>>>(g, in, b, out, om, nullptr, nullptr, nullptr, nullptr, bt);
     else
         k_mg_jacobi_v4<0, BAT, 4><<<grd, kBlk, 0, st>>>(g, in, b, out, om, nullptr, nullptr, nullptr, nullptr, bt);
+}
+// the last half-sweep of the mixed V-cycle, which adds the correction to the float pairs
+template <bool BAT>
+static void launch_jacobi_v4_1(int zc, dim3 grd, cudaStream_t st, const MgGeom& g, const float* in, const float* b,
+                               float* out, float om, float2* pdf, const Bat& bt) {
+    if (zc == 1)
+        k_mg_jacobi_v4<1, BAT, 1><<<grd, kBlk, 0, st>>>(g, in, b, out, om, pdf, nullptr, nullptr, nullptr, bt);
+    else
+        k_mg_jacobi_v4<1, BAT, V4_ZC><<<grd, kBlk, 0, st>>>(g, in, b, out, om, pdf, nullptr, nullptr, nullptr, bt);
 }
 template <bool BAT>
 static void launch_restrict_v4(int rzc, dim3 grd, cudaStream_t st, const MgGeom& gf, const float* xf, const float* bf,
@@ -2554,7 +2591,7 @@ int mg_init(MgImpl* mg, int nx, int ny, int nz, int topology, int precision, int
         }
     }
     // one partial per block of the largest reduction grid (the float-pair residual's)
-    const dim3 g0 = grid_zc(mg->lev[0].n, precision == NYLES_FP64 && !use_fx(mg, 0) ? 1 : (MG_DFZC < MG_ZC ? MG_DFZC : MG_ZC));
+    const dim3 g0 = grid_zc(mg->lev[0].n, MG_DFZC < MG_ZC ? MG_DFZC : MG_ZC);
     mg->npartial = (int)(g0.x * g0.y * g0.z);
     {
         const char* e = getenv("NYLES_GB300_SCALAR_KERNELS");
@@ -2601,12 +2638,12 @@ static void smooth(MgImpl* mg, int l, cudaStream_t st, int last_mode, bool from_
         const Bat& bt = mg->bat;
         float2* pdf = last_mode == 1 ? mg_pdf(mg) : nullptr;
         if constexpr (sizeof(T) == sizeof(float)) {
-            const int zc = last_mode == 1 ? V4_ZC : lvl_zc(mg, l);
+            const int zc = lvl_zc(mg, l);
             if (use_v4(mg, g.n, zc)) {
                 const dim3 gv = bgrid(mg, grid_v4(g.n, zc));
                 if (!from_y) launch_jacobi_v4_0<true>(zc, gv, st, g, x, b, y, om, bt);
                 if (last_mode == 1)
-                    k_mg_jacobi_v4<1, true><<<gv, kBlk, 0, st>>>(g, y, b, x, om, pdf, nullptr, nullptr, nullptr, bt);
+                    launch_jacobi_v4_1<true>(zc, gv, st, g, y, b, x, om, pdf, bt);
                 else
                     launch_jacobi_v4_0<true>(zc, gv, st, g, y, b, x, om, bt);
                 return;
@@ -2621,24 +2658,22 @@ static void smooth(MgImpl* mg, int l, cudaStream_t st, int last_mode, bool from_
         return;
     }
     if constexpr (sizeof(T) == sizeof(float)) {
-        const int zc = last_mode != 0 ? V4_ZC : lvl_zc(mg, l);
-        if (use_v4(mg, g.n, zc)) {
+        const int zc = last_mode == 2 ? V4_ZC : lvl_zc(mg, l);
+        if (last_mode == 2 ? use_v4_sums(mg) : use_v4(mg, g.n, zc)) {
             const dim3 gv = grid_v4(g.n, zc);
             if (!from_y) launch_jacobi_v4_0<false>(zc, gv, st, g, x, b, y, om, Bat());
             if (last_mode == 1)
-                k_mg_jacobi_v4<1><<<gv, kBlk, 0, st>>>(g, y, b, x, om, mg_pdf(mg),
-                                                      nullptr, nullptr, nullptr);
+                launch_jacobi_v4_1<false>(zc, gv, st, g, y, b, x, om, mg_pdf(mg), Bat());
             else if (last_mode == 2) {   // also beta and the mean of z for the Krylov update
                 MgFin fin;
                 fin.ticket = fin_ticket(mg);
                 fin.sc = reinterpret_cast<double*>(mg->ws + mg->off_scalars);
                 fin.k = mg->fcg_k;
                 fin.vol = (double)mg->lev[0].vol;
-                k_mg_jacobi_v4<2><<<gv, kBlk, 0, st>>>(g, y, b, x, om, nullptr,
-                                                      reinterpret_cast<const float*>(mg->ws + mg->off_fq),
-                                                      reinterpret_cast<double*>(mg->ws + mg->off_partial),
-                                                      reinterpret_cast<double*>(mg->ws + mg->off_partial2), Bat(),
-                                                      fin);
+                const float* q = reinterpret_cast<const float*>(mg->ws + mg->off_fq);
+                double* part = partials(mg, 0, blocks(gv));
+                double* part2 = partials(mg, 1, blocks(gv));
+                k_mg_jacobi_v4<2><<<gv, kBlk, 0, st>>>(g, y, b, x, om, nullptr, q, part, part2, Bat(), fin);
             }
             else
                 launch_jacobi_v4_0<false>(zc, gv, st, g, y, b, x, om, Bat());
@@ -2808,10 +2843,10 @@ static void enqueue_normb_df(MgImpl* mg, cudaStream_t st) {
 // and its sum of squares into sc[SC_RR]
 static void enqueue_resid_df(MgImpl* mg, cudaStream_t st) {
     MgGeom g = mgg(mg, 0);
-    double* part = reinterpret_cast<double*>(mg->ws + mg->off_partial);
     double* sc = reinterpret_cast<double*>(mg->ws + mg->off_scalars);
-    const bool v4 = use_v4(mg, g.n);
+    const bool v4 = use_v4_sums(mg);
     const dim3 grd = v4 ? grid_v4(g.n) : grid_zc(g.n, MG_DFZC);
+    double* part = partials(mg, 0, blocks(grd));
     ProfScope ps(mg->prof, 11, st);
     note_launch(v4 ? 1 : 2);
     const float2* pdf = mg_pdf(mg);
@@ -2819,19 +2854,19 @@ static void enqueue_resid_df(MgImpl* mg, cudaStream_t st) {
     MgFin fin;   // the vector kernel also adds the partials into sc[SC_RR]
     fin.ticket = fin_ticket(mg);
     fin.sc = sc;
-    if (mg->bat.tab) {
-        if (v4)
-            k_mg_resid_df_v4<true><<<bgrid(mg, grd), kBlk, 0, st>>>(g, pdf, bdf, lvp<float>(mg, 0, 2), lvp<float>(mg, 0, 3),
-                                                                    (float)mg->omega, sc, part, mg->bat, fin);
+    float* b = lvp<float>(mg, 0, 2);
+    float* y = lvp<float>(mg, 0, 3);
+    const float om = (float)mg->omega;
+    const dim3 gb = bgrid(mg, grd);
+    if (v4) {
+        if (mg->bat.tab)
+            k_mg_resid_df_v4<true><<<gb, kBlk, 0, st>>>(g, pdf, bdf, b, y, om, sc, part, mg->bat, fin);
         else
-            k_mg_resid_df<true><<<bgrid(mg, grd), kBlk, 0, st>>>(g, pdf, bdf, lvp<float>(mg, 0, 2), lvp<float>(mg, 0, 3),
-                                                                 (float)mg->omega, sc, part, mg->bat);
-    } else if (v4) {
-        k_mg_resid_df_v4<<<grd, kBlk, 0, st>>>(g, pdf, bdf, lvp<float>(mg, 0, 2), lvp<float>(mg, 0, 3),
-                                               (float)mg->omega, sc, part, Bat(), fin);
+            k_mg_resid_df_v4<<<grd, kBlk, 0, st>>>(g, pdf, bdf, b, y, om, sc, part, Bat(), fin);
+    } else if (mg->bat.tab) {
+        k_mg_resid_df<true><<<gb, kBlk, 0, st>>>(g, pdf, bdf, b, y, om, sc, part, mg->bat);
     } else {
-        k_mg_resid_df<<<grd, kBlk, 0, st>>>(g, pdf, bdf, lvp<float>(mg, 0, 2), lvp<float>(mg, 0, 3), (float)mg->omega,
-                                            sc, part);
+        k_mg_resid_df<<<grd, kBlk, 0, st>>>(g, pdf, bdf, b, y, om, sc, part);
     }
     if (!v4)
         k_mg_final<<<bgrid(mg, dim3(1, 1, 1)), 1024, 0, st>>>(part, (int)(grd.x * grd.y * grd.z), sc + SC_RR, mg->bat);
@@ -2841,18 +2876,21 @@ static void enqueue_resid_df(MgImpl* mg, cudaStream_t st) {
 // first level-0 half-sweep (k_mg_resid_sweep)
 static void enqueue_resid_sweep(MgImpl* mg, cudaStream_t st) {
     MgGeom g = mgg(mg, 0);
-    double* part = reinterpret_cast<double*>(mg->ws + mg->off_partial);
     double* sc = reinterpret_cast<double*>(mg->ws + mg->off_scalars);
-    const bool fx = use_fx(mg, 0);
-    const dim3 grd = grid_zc(g.n, fx ? FX_ZC : 1);
+    const bool fx = use_fx(mg, 0), one = !fx && partials_fit(mg, blocks(grid_zc(g.n, 1)));
+    const dim3 grd = grid_zc(g.n, fx ? FX_ZC : (one ? 1 : MG_ZC));
+    double* part = partials(mg, 0, blocks(grd));
     ProfScope ps(mg->prof, 11, st);
     note_launch(2);
     if (fx)
         k_mg_fx<FX_ZC, 1><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2), lvp<double>(mg, 0, 3),
                                                 part, g, nullptr);
-    else
+    else if (one)
         k_mg_resid_sweep<double, 1><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2),
                                                           lvp<double>(mg, 0, 3), mg->omega, part);
+    else
+        k_mg_resid_sweep<double><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2),
+                                                       lvp<double>(mg, 0, 3), mg->omega, part);
     k_mg_final<<<1, 1024, 0, st>>>(part, (int)(grd.x * grd.y * grd.z), sc + SC_RR);
 }
 
@@ -2862,26 +2900,27 @@ static void enqueue_resid_sweep(MgImpl* mg, cudaStream_t st) {
 // on the device)
 static void enqueue_fcg_update(MgImpl* mg, cudaStream_t st, int k) {
     MgGeom g = mgg(mg, 0);
-    double* part = reinterpret_cast<double*>(mg->ws + mg->off_partial);
-    double* part2 = reinterpret_cast<double*>(mg->ws + mg->off_partial2);
     double* sc = scalars(mg);
     float* z = lvp<float>(mg, 0, 1);
     float* r = lvp<float>(mg, 0, 2);
     float* P = reinterpret_cast<float*>(mg->ws + mg->off_fp);
     float* Q = reinterpret_cast<float*>(mg->ws + mg->off_fq);
     const long long n = mg->lev[0].vol;
-    const dim3 grd = grid_zc(g.n, MG_ZC);
-    const int nb = (int)(grd.x * grd.y * grd.z);
+    const bool v4 = use_v4_sums(mg);
+    const dim3 grd = v4 ? grid_v4(g.n) : grid_zc(g.n, MG_ZC);
+    const int nb = (int)blocks(grd);
+    double* part = partials(mg, 0, nb);
+    double* part2 = partials(mg, 1, nb);
     const unsigned eb = (unsigned)((n + 255) / 256);
     ProfScope ps(mg->prof, 11, st);
-    if (use_v4(mg, g.n)) {
+    if (v4) {
         // beta came with the V-cycle's last level-0 half-sweep (k_mg_jacobi_v4<2>); the
         // direction kernel also sets alpha
         note_launch(1);
         MgFin fin;
         fin.ticket = fin_ticket(mg);
         fin.sc = sc;
-        k_fcg_direction_v4<<<grid_v4(g.n), kBlk, 0, st>>>(g, z, r, P, Q, sc, part, part2, fin);
+        k_fcg_direction_v4<<<grd, kBlk, 0, st>>>(g, z, r, P, Q, sc, part, part2, fin);
     } else {
         // the partial sums of z.q and z were written by the V-cycle's last level-0 half-sweep
         note_launch(3);
