@@ -314,6 +314,12 @@ __device__ __forceinline__ double2 mg_block_total2(const double* pa, const doubl
     }
     return r;
 }
+// the same for a kernel of one sum: the total in the last block's thread (0, 0) (false elsewhere)
+__device__ __forceinline__ bool mg_fin_total(const MgFin& fin, const double* partial, unsigned int nblk, double& total) {
+    if (!mg_last_block(fin.ticket, nblk)) return false;
+    total = mg_block_total2(partial, nullptr, (int)nblk).x;
+    return threadIdx.x == 0 && threadIdx.y == 0;
+}
 // beta = -(z.q)/(p.q) of the previous iteration (0 on the first: k = iteration of this
 // solve, or sc[SC_NITE] when k < 0) stored as a float, and the mean of z (float)
 __device__ __forceinline__ void fcg_set_beta(double zq, double zs, double vol, double* sc, int k) {
@@ -1411,7 +1417,8 @@ static long long bottom_plan(const int (*n)[3], int nlev, long long solo, MgBott
 // MODE 0: sum v^2 ; MODE 1: sum r^2 with r = b + diag*x - sum(x_nb)
 template <typename T, int MODE>
 __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_sumsq(const MgGeom g, const T* __restrict__ v,
-                                                           const T* __restrict__ b, double* __restrict__ partial) {
+                                                           const T* __restrict__ b, double* __restrict__ partial,
+                                                           const MgFin fin, double* __restrict__ out) {
     const int x = blockIdx.x * MG_BX + threadIdx.x;
     const int y = blockIdx.y * MG_BY + threadIdx.y;
     const int nz = g.n[0], z0 = blockIdx.z * MG_ZC;
@@ -1457,6 +1464,8 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_sumsq(const MgGeom g, cons
         }
     }
     block_partial(s, partial, blockIdx.z);
+    double t;
+    if (mg_fin_total(fin, partial, gridDim.x * gridDim.y * gridDim.z, t)) *out = t;
 }
 
 // Stop-test residual of the level-1 solution together with the first half-sweep of the
@@ -1466,7 +1475,8 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_sumsq(const MgGeom g, cons
 template <typename T, int ZC = MG_ZC>
 __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_resid_sweep(const MgGeom g, const T* __restrict__ v,
                                                                  const T* __restrict__ b, T* __restrict__ y_out,
-                                                                 T omega, double* __restrict__ partial) {
+                                                                 T omega, double* __restrict__ partial,
+                                                                 const MgFin fin) {
     const int x = blockIdx.x * MG_BX + threadIdx.x;
     const int y = blockIdx.y * MG_BY + threadIdx.y;
     const int nz = g.n[0], z0 = blockIdx.z * ZC;
@@ -1507,6 +1517,8 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_resid_sweep(const MgGeom g
         }
     }
     block_partial(s, partial, blockIdx.z);
+    double t;
+    if (mg_fin_total(fin, partial, gridDim.x * gridDim.y * gridDim.z, t)) fin.sc[SC_RR] = t;
 }
 
 // ---------------------------------------------------------------- FP64 levels on the integer pipes
@@ -1735,7 +1747,7 @@ __device__ __forceinline__ float2 mg_ldw_df(const float2* __restrict__ a, long l
 // float right-hand side r32 of the next correction V-cycle, and the first half-sweep
 // of that V-cycle from its zero initial correction, y32. The squares are summed in
 // float per thread on r * scale, scale = sc[SC_SCALE] a power of two near 1/rms(b)
-// (k_mg_scale), so that they neither underflow nor overflow; each block partial is
+// (k_mg_sumsq_df), so that they neither underflow nor overflow; each block partial is
 // unscaled in double.
 template <bool BAT = false>
 __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_resid_df(const MgGeom g, const float2* __restrict__ p,
@@ -2209,13 +2221,18 @@ __global__ void k_mg_hist_count(int* count, const double* sc, const Bat bat = Ba
 }
 
 // sum of squares of a float-pair array (high parts, squared and summed in double)
+// Also the scale of the float sums of squares: 2^-e with 2^e near rms(b) = sqrt(sum(b^2)/vol),
+// and its inverse square (both exact powers of two).
 __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_sumsq_df(const MgGeom g, const float2* __restrict__ v,
-                                                              double* __restrict__ partial, const Bat bat = Bat()) {
+                                                              double* __restrict__ partial, MgFin fin,
+                                                              const Bat bat = Bat()) {
     int bz;
     long long dlt;
     if (!batch_enter(bat, bz, dlt)) return;
     v = bshift(v, dlt);
     partial = bshift(partial, dlt);
+    fin.ticket = bshift(fin.ticket, dlt);
+    double* const sc = bshift(fin.sc, dlt);
     const int x = blockIdx.x * MG_BX + threadIdx.x;
     const int y = blockIdx.y * MG_BY + threadIdx.y;
     const int z0 = bz * MG_ZC;
@@ -2227,21 +2244,15 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_sumsq_df(const MgGeom g, c
             s += h * h;
         }
     block_partial(s, partial, bz);
-}
-
-// scale of the float sums of squares: 2^-e with 2^e near rms(b) = sqrt(sum(b^2)/vol),
-// and its inverse square (both exact powers of two)
-__global__ void k_mg_scale(double* __restrict__ sc, double vol, const Bat bat = Bat()) {
-    int bz;
-    long long dlt;
-    if (!batch_enter(bat, bz, dlt)) return;
-    sc = bshift(sc, dlt);
-    const double nb = sc[SC_NORMB];
-    int e = 0;
-    if (nb > 0.0) frexp(sqrt(nb / vol), &e);
-    e = max(-120, min(120, e));
-    sc[SC_SCALE] = ldexp(1.0, -e);
-    sc[SC_INVSCALE2] = ldexp(1.0, 2 * e);
+    double nb;
+    if (mg_fin_total(fin, partial, gridDim.x * gridDim.y * (gridDim.z / bat.nrun), nb)) {
+        int e = 0;
+        if (nb > 0.0) frexp(sqrt(nb / fin.vol), &e);
+        e = max(-120, min(120, e));
+        sc[SC_NORMB] = nb;
+        sc[SC_SCALE] = ldexp(1.0, -e);
+        sc[SC_INVSCALE2] = ldexp(1.0, 2 * e);
+    }
 }
 
 __global__ void k_mg_final(const double* __restrict__ partial, int n, double* __restrict__ out,
@@ -2398,6 +2409,13 @@ static inline dim3 grid_v4_restrict(const MgGeom& gf, const MgGeom& gc, int rzc)
 // slot zeroed when the workspace is bound
 static inline unsigned int* fin_ticket(MgImpl* mg) {
     return reinterpret_cast<unsigned int*>(mg->ws + mg->off_ticket);
+}
+static MgFin mg_fin(MgImpl* mg) {
+    MgFin fin;
+    fin.ticket = fin_ticket(mg);
+    fin.sc = reinterpret_cast<double*>(mg->ws + mg->off_scalars);
+    fin.vol = (double)mg->lev[0].vol;
+    return fin;
 }
 
 // the vector transfers between levels l and l + 1: exact halving in every direction,
@@ -2819,9 +2837,8 @@ static void enqueue_sumsq(MgImpl* mg, const MgGeom& g, const T* v, const T* b, d
     double* part = reinterpret_cast<double*>(mg->ws + mg->off_partial);
     const dim3 grd = grid_zc(g.n, MG_ZC);
     ProfScope ps(mg->prof, 11, st);
-    note_launch(2);
-    k_mg_sumsq<T, MODE><<<grd, kBlk, 0, st>>>(g, v, b, part);
-    k_mg_final<<<1, 1024, 0, st>>>(part, (int)(grd.x * grd.y * grd.z), out);
+    note_launch(1);
+    k_mg_sumsq<T, MODE><<<grd, kBlk, 0, st>>>(g, v, b, part, mg_fin(mg), out);
 }
 
 // mixed precision: enqueue sum(b^2) of the float-pair right-hand side into
@@ -2829,14 +2846,11 @@ static void enqueue_sumsq(MgImpl* mg, const MgGeom& g, const T* v, const T* b, d
 static void enqueue_normb_df(MgImpl* mg, cudaStream_t st) {
     MgGeom g = mgg(mg, 0);
     double* part = reinterpret_cast<double*>(mg->ws + mg->off_partial);
-    double* sc = reinterpret_cast<double*>(mg->ws + mg->off_scalars);
     const dim3 grd = grid_zc(g.n, MG_ZC);
     ProfScope ps(mg->prof, 11, st);
-    note_launch(3);
+    note_launch(1);
     k_mg_sumsq_df<<<bgrid(mg, grd), kBlk, 0, st>>>(g, reinterpret_cast<const float2*>(mg->ws + mg->off_bdf), part,
-                                                   mg->bat);
-    k_mg_final<<<bgrid(mg, dim3(1, 1, 1)), 1024, 0, st>>>(part, (int)(grd.x * grd.y * grd.z), sc + SC_NORMB, mg->bat);
-    k_mg_scale<<<bgrid(mg, dim3(1, 1, 1)), 1, 0, st>>>(sc, (double)mg->lev[0].vol, mg->bat);
+                                                   mg_fin(mg), mg->bat);
 }
 
 // mixed precision: enqueue the float-pair residual (also the next correction's rhs)
@@ -2876,22 +2890,22 @@ static void enqueue_resid_df(MgImpl* mg, cudaStream_t st) {
 // first level-0 half-sweep (k_mg_resid_sweep)
 static void enqueue_resid_sweep(MgImpl* mg, cudaStream_t st) {
     MgGeom g = mgg(mg, 0);
-    double* sc = reinterpret_cast<double*>(mg->ws + mg->off_scalars);
     const bool fx = use_fx(mg, 0), one = !fx && partials_fit(mg, blocks(grid_zc(g.n, 1)));
     const dim3 grd = grid_zc(g.n, fx ? FX_ZC : (one ? 1 : MG_ZC));
     double* part = partials(mg, 0, blocks(grd));
     ProfScope ps(mg->prof, 11, st);
-    note_launch(2);
-    if (fx)
+    const MgFin fin = mg_fin(mg);
+    note_launch(fx ? 2 : 1);
+    if (fx) {   // (many blocks: the ticket took 30 us of a 128^3 level against 20 + 4.5 with the sum apart)
         k_mg_fx<FX_ZC, 1><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2), lvp<double>(mg, 0, 3),
                                                 part, g, nullptr);
-    else if (one)
+        k_mg_final<<<1, 1024, 0, st>>>(part, (int)blocks(grd), fin.sc + SC_RR);
+    } else if (one)
         k_mg_resid_sweep<double, 1><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2),
-                                                          lvp<double>(mg, 0, 3), mg->omega, part);
+                                                          lvp<double>(mg, 0, 3), mg->omega, part, fin);
     else
         k_mg_resid_sweep<double><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2),
-                                                       lvp<double>(mg, 0, 3), mg->omega, part);
-    k_mg_final<<<1, 1024, 0, st>>>(part, (int)(grd.x * grd.y * grd.z), sc + SC_RR);
+                                                       lvp<double>(mg, 0, 3), mg->omega, part, fin);
 }
 
 // mixed precision with krylov: after the V-cycle left z = V(r) in level 0's x (and the

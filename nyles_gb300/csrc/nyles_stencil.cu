@@ -80,6 +80,7 @@ struct RhsArgs {
     int kmask;        // bit q: diffuse tracer q (b = 0) when TERM_TRDIFF is set
     int vf_order;     // 0: WENO vortex force; 1..5: the linear branch of that order
     int lo[3], hi[3]; // k_rhs_march: index box (z, y, x) of the cells it computes
+    int zc;           // k_rhs_march: cells per thread along z
 };
 
 // every pointer of the arguments shifted by dlt bytes (batched launches)
@@ -226,6 +227,12 @@ __global__ void __launch_bounds__(128) k_vortex_force(const RhsArgs<T> a) {
 // its column chunk. One WENO5 per direction and tracer per cell instead of two. FP32, and
 // in FP64 the terms without WENO reconstructions (those march along lines, nyles_line.cu).
 constexpr int RZ_BX = 32, RZ_BY = 8, RZ_ZC = 16;
+// Blocks of 256 threads that fill the chip: 8 on each of 152 SMs. Kernels that carry nothing from plane
+// to plane take shorter columns on grids that would give fewer: a column of 8 or 16 dependent
+// planes took 11 to 20 us whatever the grid. A 64 x 32 x 32 FP64 step 1453 -> 1378 us with the terms without
+// reconstructions and the projection so cut, a 48^3 mixed one 837 -> 814; filling a quarter to eight
+// times the chip gives the same within 0.5%.
+constexpr long long FILL_BLOCKS = 8 * 152;
 
 template <typename T>
 struct TracerMarch {
@@ -280,8 +287,8 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, RhsMinBlocks<T>::n) k_rhs_march
     const Geom& g = a.g;
     const int x = a.lo[2] + blockIdx.x * RZ_BX + threadIdx.x;
     const int y = a.lo[1] + blockIdx.y * RZ_BY + threadIdx.y;
-    const int z0 = a.lo[0] + bz * RZ_ZC;
-    const int z1 = min(z0 + RZ_ZC, a.hi[0]) - 1;
+    const int z0 = a.lo[0] + bz * a.zc;
+    const int z1 = min(z0 + a.zc, a.hi[0]) - 1;
     const int Nz = g.N[0], Ny = g.N[1], Nx = g.N[2];
     const bool valid = x < a.hi[2] && y < a.hi[1];
     const int xs = min(x, a.hi[2] - 1), ys = min(y, a.hi[1] - 1);   // idle lanes shadow a real cell
@@ -792,6 +799,7 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
         a.W[i] = s.f[NYLES_F_VOR_I + i];
         a.u[i] = s.f[NYLES_F_U_I + i];
     }
+    a.zc = RZ_ZC;
     a.ke = s.f[NYLES_F_KE];
     for (int q = 0; q < NYLES_MAX_PROG; ++q) a.ds[q] = (q < 4 + d->n_tracers) ? ds.p[q] : nullptr;
     a.ntr = d->n_tracers;
@@ -871,8 +879,12 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
             set_error("batched right-hand side: single precision only");
             return NYLES_UNSUPPORTED;
         }
-        if (lin) k_rhs_march<T, false, 2, false><<<grd_box, blk, 0, st>>>(a);
-        else k_rhs_march<T, false, 0, false><<<grd_box, blk, 0, st>>>(a);
+        // (nothing is carried from plane to plane here: shorter columns until the blocks fill the chip)
+        dim3 gi = grd_box;
+        for (; a.zc > 1 && (long long)gi.x * gi.y * gi.z < FILL_BLOCKS; a.zc >>= 1)
+            gi.z = (unsigned)((a.hi[0] - a.lo[0] + a.zc / 2 - 1) / (a.zc / 2));
+        if (lin) k_rhs_march<T, false, 2, false><<<gi, blk, 0, st>>>(a);
+        else k_rhs_march<T, false, 0, false><<<gi, blk, 0, st>>>(a);
         note_launch();
         if (linear_tr) {
             tracer_linear(a.b, a.ds[0], 0);
@@ -1104,22 +1116,29 @@ int launch_fill(const Geom& g, T* const* fields, int nf, cudaStream_t st, const 
 // (core/cov_to_contra.py:16-18), evaluated at the periodic image of each cell because
 // core/mgfordriver.py:70 fills the halo of div before the solve.
 // The divergence and the projection correction run one thread per (y, x) column of the
-// array and PJ_ZC cells in z: the column's wrapped position and interior offset are
-// computed once.
+// array and PJ_ZC cells in z (fewer on small grids, FILL_BLOCKS): the column's wrapped position and
+// interior offset are computed once.
 constexpr int PJ_BX = 32, PJ_BY = 8, PJ_ZC = 8;
-static inline dim3 grid_pj(const Geom& g) {
+// cells per thread: halved until the blocks fill the chip
+static inline int pj_chunk(const Geom& g, int nrun) {
+    const long long col = (long long)((g.N[2] + PJ_BX - 1) / PJ_BX) * ((g.N[1] + PJ_BY - 1) / PJ_BY) * nrun;
+    int zc = PJ_ZC;
+    while (zc > 1 && col * ((g.N[0] + zc - 1) / zc) < FILL_BLOCKS) zc >>= 1;
+    return zc;
+}
+static inline dim3 grid_pj(const Geom& g, int zc) {
     return dim3((unsigned)((g.N[2] + PJ_BX - 1) / PJ_BX), (unsigned)((g.N[1] + PJ_BY - 1) / PJ_BY),
-                (unsigned)((g.N[0] + PJ_ZC - 1) / PJ_ZC));
+                (unsigned)((g.N[0] + zc - 1) / zc));
 }
 
 template <typename T, typename TB>
 __global__ void __launch_bounds__(PJ_BX * PJ_BY) k_div(const Geom g, const T* __restrict__ ux, const T* __restrict__ uy,
                                                        const T* __restrict__ uz, TB idx2, TB idy2, TB idz2,
-                                                       T* __restrict__ div, TB* __restrict__ mgb) {
+                                                       T* __restrict__ div, TB* __restrict__ mgb, const int zc) {
     const int x = blockIdx.x * PJ_BX + threadIdx.x;
     const int y = blockIdx.y * PJ_BY + threadIdx.y;
     if (x >= g.N[2] || y >= g.N[1]) return;
-    const int z0 = blockIdx.z * PJ_ZC, z1 = min(z0 + PJ_ZC, g.N[0]);
+    const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, g.N[0]);
     const int yy = g.wrap(1, y), xx = g.wrap(2, x);
     const bool own_xy = yy == y && xx == x;
     const long long cxy = (long long)yy * g.sy + xx;
@@ -1165,7 +1184,7 @@ __global__ void __launch_bounds__(PJ_BX * PJ_BY) k_div_df(const Geom g, const fl
                                                           const float* __restrict__ uy, const float* __restrict__ uz,
                                                           float2 idx2, float2 idy2, float2 idz2,
                                                           float* __restrict__ div, float2* __restrict__ mgb,
-                                                          const Bat bat = Bat()) {
+                                                          const int zc, const Bat bat = Bat()) {
     int bz;
     long long dlt;
     if (!batch_enter(bat, bz, dlt)) return;
@@ -1177,7 +1196,7 @@ __global__ void __launch_bounds__(PJ_BX * PJ_BY) k_div_df(const Geom g, const fl
     const int x = blockIdx.x * PJ_BX + threadIdx.x;
     const int y = blockIdx.y * PJ_BY + threadIdx.y;
     if (x >= g.N[2] || y >= g.N[1]) return;
-    const int z0 = bz * PJ_ZC, z1 = min(z0 + PJ_ZC, g.N[0]);
+    const int z0 = bz * zc, z1 = min(z0 + zc, g.N[0]);
     const int yy = g.wrap(1, y), xx = g.wrap(2, x);
     const bool own_xy = yy == y && xx == x;
     const long long cxy = (long long)yy * g.sy + xx;
@@ -1198,19 +1217,21 @@ __global__ void __launch_bounds__(PJ_BX * PJ_BY) k_div_df(const Geom g, const fl
 
 template <typename T, typename TB>
 int launch_div(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, TB* mg_b, cudaStream_t st) {
-    k_div<T, TB><<<grid_pj(g), dim3(PJ_BX, PJ_BY), 0, st>>>(g, s.f[NYLES_F_U_I], s.f[NYLES_F_U_J], s.f[NYLES_F_U_K],
-                                                 TB(d->idx2), TB(d->idy2), TB(d->idz2), s.f[NYLES_F_DIV], mg_b);
+    const int zc = pj_chunk(g, 1);
+    k_div<T, TB><<<grid_pj(g, zc), dim3(PJ_BX, PJ_BY), 0, st>>>(g, s.f[NYLES_F_U_I], s.f[NYLES_F_U_J], s.f[NYLES_F_U_K],
+                                                 TB(d->idx2), TB(d->idy2), TB(d->idz2), s.f[NYLES_F_DIV], mg_b, zc);
     note_launch();
     return cuda_status(cudaGetLastError(), "div kernel");
 }
 
 int launch_div_df(const NylesDesc* d, const Geom& g, const StencilPtrs<float>& s, float2* mg_b, cudaStream_t st,
                   const Bat& bat) {
-    dim3 grd = grid_pj(g);
+    const int zc = pj_chunk(g, bat.nrun);
+    dim3 grd = grid_pj(g, zc);
     if (bat.tab) grd.z *= bat.nrun;
     k_div_df<<<grd, dim3(PJ_BX, PJ_BY), 0, st>>>(g, s.f[NYLES_F_U_I], s.f[NYLES_F_U_J], s.f[NYLES_F_U_K],
                                                  df_split(d->idx2), df_split(d->idy2), df_split(d->idz2),
-                                                 s.f[NYLES_F_DIV], mg_b, bat);
+                                                 s.f[NYLES_F_DIV], mg_b, zc, bat);
     note_launch();
     return cuda_status(cudaGetLastError(), "div kernel");
 }
@@ -1230,12 +1251,12 @@ struct CorrArgs {
 };
 
 template <typename T, typename TP>
-__global__ void __launch_bounds__(PJ_BX * PJ_BY) k_correct(const CorrArgs<T, TP> a) {
+__global__ void __launch_bounds__(PJ_BX * PJ_BY) k_correct(const CorrArgs<T, TP> a, const int zc) {
     const Geom& g = a.g;
     const int x = blockIdx.x * PJ_BX + threadIdx.x;
     const int y = blockIdx.y * PJ_BY + threadIdx.y;
     if (x >= g.N[2] || y >= g.N[1]) return;
-    const int z0 = blockIdx.z * PJ_ZC, z1 = min(z0 + PJ_ZC, g.N[0]);
+    const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, g.N[0]);
     const int oz = g.per[0] ? g.nh : 0, oy = g.per[1] ? g.nh : 0, ox = g.per[2] ? g.nh : 0;
     const int yy = g.wrap(1, y), xx = g.wrap(2, x);
     const bool own_xy = yy == y && xx == x;
@@ -1272,7 +1293,8 @@ int launch_correct(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, c
     a.x = mg_x;
     a.p = s.f[NYLES_F_P];
     a.dx2 = dx2;
-    k_correct<T, TP><<<grid_pj(g), dim3(PJ_BX, PJ_BY), 0, st>>>(a);
+    const int zc = pj_chunk(g, 1);
+    k_correct<T, TP><<<grid_pj(g, zc), dim3(PJ_BX, PJ_BY), 0, st>>>(a, zc);
     note_launch();
     return cuda_status(cudaGetLastError(), "correct kernel");
 }
@@ -1288,7 +1310,7 @@ struct CorrDfArgs {
 };
 
 // one thread per (y, x) column of the array, PJ_ZC cells in z (as k_div_df)
-__global__ void __launch_bounds__(PJ_BX * PJ_BY) k_correct_df(const CorrDfArgs a0, const Bat bat = Bat()) {
+__global__ void __launch_bounds__(PJ_BX * PJ_BY) k_correct_df(const CorrDfArgs a0, const int zc, const Bat bat = Bat()) {
     int bz;
     long long dlt;
     if (!batch_enter(bat, bz, dlt)) return;
@@ -1308,7 +1330,7 @@ __global__ void __launch_bounds__(PJ_BX * PJ_BY) k_correct_df(const CorrDfArgs a
     float* __restrict__ U0 = a.u[0];
     float* __restrict__ U1 = a.u[1];
     float* __restrict__ U2 = a.u[2];
-    const int z0 = bz * PJ_ZC, z1 = min(z0 + PJ_ZC, g.N[0]);
+    const int z0 = bz * zc, z1 = min(z0 + zc, g.N[0]);
     const int oz = g.per[0] ? g.nh : 0, oy = g.per[1] ? g.nh : 0, ox = g.per[2] ? g.nh : 0;
     const int yy = g.wrap(1, y), xx = g.wrap(2, x);
     const bool own_xy = yy == y && xx == x;
@@ -1343,9 +1365,10 @@ int launch_correct_df(const Geom& g, const StencilPtrs<float>& s, const float2* 
     a.x = mg_x;
     a.p = s.f[NYLES_F_P];
     a.dx2 = df_split(dx2);
-    dim3 grd = grid_pj(g);
+    const int zc = pj_chunk(g, bat.nrun);
+    dim3 grd = grid_pj(g, zc);
     if (bat.tab) grd.z *= bat.nrun;
-    k_correct_df<<<grd, dim3(PJ_BX, PJ_BY), 0, st>>>(a, bat);
+    k_correct_df<<<grd, dim3(PJ_BX, PJ_BY), 0, st>>>(a, zc, bat);
     note_launch();
     return cuda_status(cudaGetLastError(), "correct kernel");
 }
