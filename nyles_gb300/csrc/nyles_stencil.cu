@@ -337,51 +337,70 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, RhsMinBlocks<T>::n) k_rhs_march
 //  - 32-bit offsets from a block's own pointers; the six values around a face are loaded at
 //    offsets shared by every field read along that direction;
 //  - the upwind side is chosen among the six loaded values, so every reconstruction is
-//    one weno5 on registers (no data-dependent addresses), written in differences;
+//    one weno5 on registers (no data-dependent addresses), the two vortex-force fluxes that share
+//    a direction as a pair;
 //  - the advecting velocity averaged at the face behind the cell, (UU0 of vf_flux),
 //    comes from the neighbouring lane along x and from the previous cell of the column
 //    along z instead of two more loads;
 //  - within three cells of an array end, where flux1d_at takes a closure branch, the
 //    reconstruction falls back to flux1d_at.
-// Bound by instruction issue (64% of cycles; 484 FP32 and 270 integer instructions per cell). Measured
-// against reconstructions from the values themselves, paired where two fields share a line:
-// 301 x 203 x 97 365 -> 328 us, 512 x 256 x 256 1433 -> 1289 us; a passive tracer there 907 -> 520 us
-// against k_tracer_march. Two rows of cells per thread with every reconstruction paired took 407
-// us (1 x 1 constants cost the paired form a move each, and its 128 registers leave 16 warps).
+// Bound by instruction issue (64% of cycles). Measured against 64-bit index arithmetic per load:
+// 301 x 203 x 97 371 -> 335 us, 512 x 256 x 256 1433 -> 1320 us; a passive tracer there 907 -> 612 us against
+// k_tracer_march. The reconstructions written in differences (as in nyles_line.cu) took 328, 1289 and 520 us,
+// but round anew what smooth fields leave ill-conditioned: the weights of isolated cells (1e-3 of a small
+// velocity component's rms after one step) and the constant of a closed box's pressure (1e-6 of p).
 
 // u * weno5 of the five values upwind of the face between v[2] and v[3] (flux1d_at's
-// interior branch): v[0..4] for u > 0, v[5..1] otherwise. Written in differences of the line
-// (core/weno.f90:25-54 regrouped, as in nyles_line.cu): the indicators, carried as 4 (beta +
-// eps), take 18 instructions instead of 27, and the weights 6 and 3 ride in the constants.
-__device__ __forceinline__ float rcp_approx(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
+// interior branch): v[0..4] for u > 0, v[5..1] otherwise
 __device__ __forceinline__ float weno5_upwind(float u, const float (&v)[6]) {
-    constexpr float c13 = 1.0f / 3.0f, c76 = 7.0f / 6.0f, c116 = 11.0f / 6.0f, c16 = 1.0f / 6.0f, c56 = 5.0f / 6.0f;
-    constexpr float k4 = 4.0f * (13.0f / 12.0f), eps4 = 4.0f * 1e-16f;
-    // sums of the candidates' coefficients (REAL(4) literals: not quite 1)
-    constexpr double s1 = (double)c13 - (double)c76 + (double)c116, s2 = (double)c56 + (double)c13 - (double)c16;
     const bool pos = u > 0.f;
     const float qa = pos ? v[0] : v[5], qb = pos ? v[1] : v[4], qc = pos ? v[2] : v[3], qd = pos ? v[3] : v[2],
                 qe = pos ? v[4] : v[1];
-    const float d0 = qb - qa, d1 = qc - qb, d2 = qd - qc, d3 = qe - qd;
-    const float e0 = d1 - d0, e1 = d2 - d1, e2 = d3 - d2;
-    auto ind = [&](float e, float s) { return fmaf(s, s, fmaf(k4 * e, e, eps4)); };
-    const float b1 = ind(e0, fmaf(3.f, d1, -d0)), b2 = ind(e1, d1 + d2), b3 = ind(e2, fmaf(-3.f, d2, d3));
-    const float tau = fabsf(b1 - b3);
-    // every denominator is at least 4e-16 (eps) or 1 and far below 2^126
-    const float w1 = fmaf(tau, rcp_approx(b1), 1.f), w2 = fmaf(tau, rcp_approx(b2), 1.f),
-                w3 = fmaf(tau, rcp_approx(b3), 1.f);
-    const float den = fmaf(3.f, w3, fmaf(6.f, w2, w1));
-    const float g1 = fmaf(c76 - c13, d1, fmaf(-c13, d0, (float)(s1 - s2) * qc));
-    const float g2 = fmaf(6.f * c13, d2, (6.f * c16) * d1);
-    const float g3 = fmaf(3.f * (c56 - c16), d2, (-3.f * c16) * d3);
-    const float num = fmaf(w3, g3, fmaf(w2, g2, w1 * g1));
-    return u * fmaf(num, rcp_approx(den), (float)s2 * qc);
+    return u * weno5(qa, qb, qc, qd, qe);
 }
 
+// ---- two FP32 reconstructions at once. Blackwell issues two FP32 lanes' worth of
+// multiply-adds in one paired instruction (__ffma2_rn, __fadd2_rn, __fmul2_rn), and the
+// FP32 right-hand side is bound by instruction issue: the two vortex-force fluxes that
+// share a direction (and so their load offsets) are reconstructed together. The same
+// formula as weno5<float>; the weights' divisions stay per component (hardware
+// reciprocal).
+__device__ __forceinline__ float2 f2s(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 weno5_x2(float2 qmm, float2 qm, float2 q0, float2 qp, float2 qpp) {
+    typedef WenoK<float> K;
+    const float2 qi1 = __ffma2_rn(f2s(K::c116()), q0, __ffma2_rn(f2s(-K::c76()), qm, __fmul2_rn(f2s(K::c13()), qmm)));
+    const float2 qi2 = __ffma2_rn(f2s(K::c13()), qp, __ffma2_rn(f2s(K::c56()), q0, __fmul2_rn(f2s(-K::c16()), qm)));
+    const float2 qi3 = __ffma2_rn(f2s(-K::c16()), qpp, __ffma2_rn(f2s(K::c56()), qp, __fmul2_rn(f2s(K::c13()), q0)));
+    const float2 a1 = __fadd2_rn(__ffma2_rn(f2s(-2.f), qm, qmm), q0);
+    const float2 b1 = __ffma2_rn(f2s(3.f), q0, __ffma2_rn(f2s(-4.f), qm, qmm));
+    const float2 a2 = __fadd2_rn(__ffma2_rn(f2s(-2.f), q0, qm), qp);
+    const float2 b2 = __ffma2_rn(f2s(-1.f), qp, qm);
+    const float2 a3 = __fadd2_rn(__ffma2_rn(f2s(-2.f), qp, q0), qpp);
+    const float2 b3 = __fadd2_rn(__ffma2_rn(f2s(-4.f), qp, __fmul2_rn(f2s(3.f), q0)), qpp);
+    auto beta = [&](float2 a, float2 b) {
+        return __ffma2_rn(__fmul2_rn(f2s(K::k1()), a), a, __fmul2_rn(__fmul2_rn(f2s(0.25f), b), b));
+    };
+    const float2 be1 = beta(a1, b1), be2 = beta(a2, b2), be3 = beta(a3, b3);
+    const float2 t = __ffma2_rn(f2s(-1.f), be3, be1);
+    const float2 tau5 = make_float2(fabsf(t.x), fabsf(t.y));
+    const float2 d1 = __fadd2_rn(be1, f2s(K::eps5())), d2 = __fadd2_rn(be2, f2s(K::eps5())),
+                 d3 = __fadd2_rn(be3, f2s(K::eps5()));
+    const float2 r1 = make_float2(__fdividef(tau5.x, d1.x), __fdividef(tau5.y, d1.y));
+    const float2 r2 = make_float2(__fdividef(tau5.x, d2.x), __fdividef(tau5.y, d2.y));
+    const float2 r3 = make_float2(__fdividef(tau5.x, d3.x), __fdividef(tau5.y, d3.y));
+    const float2 w1 = __fadd2_rn(f2s(1.f), r1);
+    const float2 w2 = __fmul2_rn(f2s(6.f), __fadd2_rn(f2s(1.f), r2));
+    const float2 w3 = __fmul2_rn(f2s(3.f), __fadd2_rn(f2s(1.f), r3));
+    const float2 num = __ffma2_rn(w3, qi3, __ffma2_rn(w2, qi2, __fmul2_rn(w1, qi1)));
+    const float2 den = __fadd2_rn(__fadd2_rn(w1, w2), w3);
+    return make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
+}
+// u * weno5_x2 of the five values upwind of the face, each component on its own side
+__device__ __forceinline__ float2 weno5_upwind_x2(float2 u, const float2 (&v)[6]) {
+    const bool px = u.x > 0.f, py = u.y > 0.f;
+    auto sel = [&](int a, int b) { return make_float2(px ? v[a].x : v[b].x, py ? v[a].y : v[b].y); };
+    return __fmul2_rn(u, weno5_x2(sel(0, 5), sel(1, 4), sel(2, 3), sel(3, 2), sel(4, 1)));
+}
 // flux1d_at near an array end, out of line: the closures are rare (walls), and inlined
 // at the nine reconstruction sites they would multiply the kernel's code size. p: the line's
 // value at index i; vortex force: q(kk) = W(kk - 1), q(0) = 0.
@@ -419,15 +438,16 @@ __device__ __forceinline__ float tr_flux32(const char* __restrict__ f, float u, 
     }
     return tr_flux_closure(reinterpret_cast<const float*>(f + l.o[3]), u, i, n, s);
 }
-__device__ __forceinline__ float vf_flux32(const char* __restrict__ f, float u, const LineOff& l, int i, int n, int s,
-                                           bool fast) {
+__device__ __forceinline__ float2 vf_flux32_x2(const char* __restrict__ fa, const char* __restrict__ fb, float2 u,
+                                               const LineOff& l, int i, int n, int s, bool fast) {
     if (fast) {
-        float v[6];
+        float2 v[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = ldo(f, l.o[k]);
-        return weno5_upwind(u, v);
+        for (int k = 0; k < 6; ++k) v[k] = make_float2(ldo(fa, l.o[k]), ldo(fb, l.o[k]));
+        return weno5_upwind_x2(u, v);
     }
-    return vf_flux_closure(reinterpret_cast<const float*>(f + l.o[3]), u, i, n, s);
+    return make_float2(vf_flux_closure(reinterpret_cast<const float*>(fa + l.o[3]), u.x, i, n, s),
+                       vf_flux_closure(reinterpret_cast<const float*>(fb + l.o[3]), u.y, i, n, s));
 }
 
 // One tracer in a block of RZ_BX x RZ_BY columns: -(flux divergence), summed as TracerMarch::step
@@ -537,27 +557,43 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(c
         const LineOff lz(c, bzs), ly(c, by), lx(c, 4u);
         // f4 (ylo): u_j += U^k w_i along k (U^k averaged along j); f5 (xlo): u_i -= U^k w_j along
         // k (U^k averaged along i)
-        if (ylo) {
-            const T uu1 = T(0.5) * (u2 + ldo(U2, c + by)), uu0 = z > 0 ? uu_zy : T(0);
-            uu_zy = uu1;
-            f4 = vf_flux32(W0, T(0.5) * (uu0 + uu1), lz, z, Nz, sz, zv);
-        }
-        if (xlo) {
-            const T uu1 = T(0.5) * (u2 + ldo(U2, c + 4u)), uu0 = z > 0 ? uu_zx : T(0);
-            uu_zx = uu1;
-            f5 = vf_flux32(W1, T(0.5) * (uu0 + uu1), lz, z, Nz, sz, zv);
+        {
+            float2 u = make_float2(0.f, 0.f);
+            if (ylo) {
+                const T uu1 = T(0.5) * (u2 + ldo(U2, c + by)), uu0 = z > 0 ? uu_zy : T(0);
+                uu_zy = uu1;
+                u.x = T(0.5) * (uu0 + uu1);
+            }
+            if (xlo) {
+                const T uu1 = T(0.5) * (u2 + ldo(U2, c + 4u)), uu0 = z > 0 ? uu_zx : T(0);
+                uu_zx = uu1;
+                u.y = T(0.5) * (uu0 + uu1);
+            }
+            if (ylo || xlo) {
+                const float2 f = vf_flux32_x2(W0, W1, u, lz, z, Nz, sz, zv);
+                f4 = f.x;
+                f5 = f.y;
+            }
         }
         // f2 (xlo): u_i += U^j w_k along j (U^j averaged along i); f3 (zlo): u_k -= U^j w_i along
         // j (U^j averaged along k)
-        if (xlo) {
-            const T uu1 = T(0.5) * (u1 + ldo(U1, c + 4u));
-            const T uu0 = ys > 0 ? T(0.5) * (ldo(U1, c - by) + ldo(U1, c - by + 4u)) : T(0);
-            f2 = vf_flux32(W2, T(0.5) * (uu0 + uu1), ly, ys, Ny, sy, yv);
-        }
-        if (zlo) {
-            const T uu1 = T(0.5) * (u1 + ldo(U1, c + bzs));
-            const T uu0 = ys > 0 ? T(0.5) * (ldo(U1, c - by) + ldo(U1, c - by + bzs)) : T(0);
-            f3 = vf_flux32(W0, T(0.5) * (uu0 + uu1), ly, ys, Ny, sy, yv);
+        {
+            float2 u = make_float2(0.f, 0.f);
+            if (xlo) {
+                const T uu1 = T(0.5) * (u1 + ldo(U1, c + 4u));
+                const T uu0 = ys > 0 ? T(0.5) * (ldo(U1, c - by) + ldo(U1, c - by + 4u)) : T(0);
+                u.x = T(0.5) * (uu0 + uu1);
+            }
+            if (zlo) {
+                const T uu1 = T(0.5) * (u1 + ldo(U1, c + bzs));
+                const T uu0 = ys > 0 ? T(0.5) * (ldo(U1, c - by) + ldo(U1, c - by + bzs)) : T(0);
+                u.y = T(0.5) * (uu0 + uu1);
+            }
+            if (xlo || zlo) {
+                const float2 f = vf_flux32_x2(W2, W0, u, ly, ys, Ny, sy, yv);
+                f2 = f.x;
+                f3 = f.y;
+            }
         }
         // f1 (ylo): u_j -= U^i w_k along i (U^i averaged along j); f6 (zlo): u_k += U^i w_j along
         // i (U^i averaged along k)
@@ -572,8 +608,12 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(c
                     if (zlo) mz = T(0.5) * (um + ldo(U0, c - 4u + bzs));
                 }
             }
-            if (ylo) f1 = vf_flux32(W2, T(0.5) * (my + uy), lx, xs, Nx, 1, xv);
-            if (zlo) f6 = vf_flux32(W1, T(0.5) * (mz + uz), lx, xs, Nx, 1, xv);
+            if (ylo || zlo) {
+                const float2 u = make_float2(ylo ? T(0.5) * (my + uy) : T(0), zlo ? T(0.5) * (mz + uz) : T(0));
+                const float2 f = vf_flux32_x2(W2, W1, u, lx, xs, Nx, 1, xv);
+                f1 = f.x;
+                f6 = f.y;
+            }
         }
         const T db = tm.step(b, U0, U1, u0, u1, u2, lx, ly, lz, z, ys, xs, sy, sz, Nz, Ny, Nx, sfy);
         // ---- vortex force, summed in the order of vortex_force_cell
@@ -638,305 +678,6 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, 5) k_tracer_les(const Geom g, c
         if (valid) dq[g.at(z, k.ys, k.xs)] = v;
     }
 }
-
-// ---------------------------------------------------------------- right-hand side, paired reconstructions
-// k_rhs_les's cell with the reconstructions of k_rhs_march, from the values themselves, the two
-// vortex-force fluxes that share a direction as a pair: for grids below RHS32_SMALL cells. Planes per
-// thread by rhs32_chunk: 16 / 2 of a 48^3 right-hand side 118 / 20 us.
-namespace pairs {
-// u * weno5 of the five values upwind of the face between v[2] and v[3] (flux1d_at's
-// interior branch): v[0..4] for u > 0, v[5..1] otherwise
-static __device__ __forceinline__ float weno5_upwind(float u, const float (&v)[6]) {
-    const bool pos = u > float(0);
-    const float qa = pos ? v[0] : v[5];
-    const float qb = pos ? v[1] : v[4];
-    const float qc = pos ? v[2] : v[3];
-    const float qd = pos ? v[3] : v[2];
-    const float qe = pos ? v[4] : v[1];
-    return u * weno5(qa, qb, qc, qd, qe);
-}
-
-// flux1d_at near an array end, out of line: the closures are rare (walls), and inlined
-// at the nine reconstruction sites they would multiply the kernel's code size
-static __device__ __noinline__ float tr_flux_closure(const float* __restrict__ q, float u, int base, int i, int n, int s) {
-    auto Q = [&](int kk) -> float { return __ldg(q + base + kk * s); };
-    return flux1d_at(i, n, u, Q);
-}
-static __device__ __noinline__ float vf_flux_closure(const float* __restrict__ W, float u1, int base, int i, int n, int s) {
-    auto Q = [&](int kk) -> float { return kk == 0 ? float(0) : __ldg(W + base + (kk - 1) * s); };
-    return flux1d_at(i, n, u1, Q);
-}
-
-// tracer flux at index i of a line through c with stride s (flux1d_at of tr_flux);
-// o[k] = c + (k - 3) s
-static __device__ __forceinline__ float tr_flux32(const float* __restrict__ q, float u, int c, int i, int n, int s, bool fast,
-                                       const int (&o)[7]) {
-    if (fast) {
-        float v[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = __ldg(q + o[k + 1]);
-        return weno5_upwind(u, v);
-    }
-    return tr_flux_closure(q, u, c - i * s, i, n, s);
-}
-// the same along x (stride 1: constant offsets)
-static __device__ __forceinline__ float tr_flux32x(const float* __restrict__ q, float u, int c, int i, int n, bool fast) {
-    if (fast) {
-        float v[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = __ldg(q + c + (k - 2));
-        return weno5_upwind(u, v);
-    }
-    return tr_flux_closure(q, u, c - i, i, n, 1);
-}
-
-// ---- two FP32 reconstructions at once. Blackwell issues two FP32 lanes' worth of
-// multiply-adds in one paired instruction (__ffma2_rn, __fadd2_rn, __fmul2_rn), and the
-// FP32 right-hand side is bound by instruction issue: the two vortex-force fluxes that
-// share a direction (and so their load offsets) are reconstructed together. The same
-// formula as weno5<float>; the weights' divisions stay per component (hardware
-// reciprocal).
-static __device__ __forceinline__ float2 f2s(float a) { return make_float2(a, a); }
-static __device__ __forceinline__ float2 weno5_x2(float2 qmm, float2 qm, float2 q0, float2 qp, float2 qpp) {
-    typedef WenoK<float> K;
-    const float2 qi1 = __ffma2_rn(f2s(K::c116()), q0, __ffma2_rn(f2s(-K::c76()), qm, __fmul2_rn(f2s(K::c13()), qmm)));
-    const float2 qi2 = __ffma2_rn(f2s(K::c13()), qp, __ffma2_rn(f2s(K::c56()), q0, __fmul2_rn(f2s(-K::c16()), qm)));
-    const float2 qi3 = __ffma2_rn(f2s(-K::c16()), qpp, __ffma2_rn(f2s(K::c56()), qp, __fmul2_rn(f2s(K::c13()), q0)));
-    const float2 a1 = __fadd2_rn(__ffma2_rn(f2s(-2.f), qm, qmm), q0);
-    const float2 b1 = __ffma2_rn(f2s(3.f), q0, __ffma2_rn(f2s(-4.f), qm, qmm));
-    const float2 a2 = __fadd2_rn(__ffma2_rn(f2s(-2.f), q0, qm), qp);
-    const float2 b2 = __ffma2_rn(f2s(-1.f), qp, qm);
-    const float2 a3 = __fadd2_rn(__ffma2_rn(f2s(-2.f), qp, q0), qpp);
-    const float2 b3 = __fadd2_rn(__ffma2_rn(f2s(-4.f), qp, __fmul2_rn(f2s(3.f), q0)), qpp);
-    auto beta = [&](float2 a, float2 b) {
-        return __ffma2_rn(__fmul2_rn(f2s(K::k1()), a), a, __fmul2_rn(__fmul2_rn(f2s(0.25f), b), b));
-    };
-    const float2 be1 = beta(a1, b1), be2 = beta(a2, b2), be3 = beta(a3, b3);
-    const float2 t = __ffma2_rn(f2s(-1.f), be3, be1);
-    const float2 tau5 = make_float2(fabsf(t.x), fabsf(t.y));
-    const float2 d1 = __fadd2_rn(be1, f2s(K::eps5())), d2 = __fadd2_rn(be2, f2s(K::eps5())),
-                 d3 = __fadd2_rn(be3, f2s(K::eps5()));
-    const float2 r1 = make_float2(__fdividef(tau5.x, d1.x), __fdividef(tau5.y, d1.y));
-    const float2 r2 = make_float2(__fdividef(tau5.x, d2.x), __fdividef(tau5.y, d2.y));
-    const float2 r3 = make_float2(__fdividef(tau5.x, d3.x), __fdividef(tau5.y, d3.y));
-    const float2 w1 = __fadd2_rn(f2s(1.f), r1);
-    const float2 w2 = __fmul2_rn(f2s(6.f), __fadd2_rn(f2s(1.f), r2));
-    const float2 w3 = __fmul2_rn(f2s(3.f), __fadd2_rn(f2s(1.f), r3));
-    const float2 num = __ffma2_rn(w3, qi3, __ffma2_rn(w2, qi2, __fmul2_rn(w1, qi1)));
-    const float2 den = __fadd2_rn(__fadd2_rn(w1, w2), w3);
-    return make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
-}
-// u * weno5_x2 of the five values upwind of the face, each component on its own side
-static __device__ __forceinline__ float2 weno5_upwind_x2(float2 u, const float2 (&v)[6]) {
-    const bool px = u.x > 0.f, py = u.y > 0.f;
-    auto sel = [&](int a, int b) { return make_float2(px ? v[a].x : v[b].x, py ? v[a].y : v[b].y); };
-    return __fmul2_rn(u, weno5_x2(sel(0, 5), sel(1, 4), sel(2, 3), sel(3, 2), sel(4, 1)));
-}
-// vf_flux32 of two vorticity fields along one direction (offsets o shared)
-static __device__ __forceinline__ float2 vf_flux32_x2(const float* __restrict__ Wa, const float* __restrict__ Wb, float2 u1,
-                                               int c, int i, int n, int s, bool fast, const int (&o)[7]) {
-    if (fast) {
-        float2 v[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = make_float2(__ldg(Wa + o[k]), __ldg(Wb + o[k]));
-        return weno5_upwind_x2(u1, v);
-    }
-    return make_float2(vf_flux_closure(Wa, u1.x, c - i * s, i, n, s), vf_flux_closure(Wb, u1.y, c - i * s, i, n, s));
-}
-static __device__ __forceinline__ float2 vf_flux32x_x2(const float* __restrict__ Wa, const float* __restrict__ Wb, float2 u1,
-                                                int c, int i, int n, bool fast) {
-    if (fast) {
-        float2 v[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = make_float2(__ldg(Wa + c + (k - 3)), __ldg(Wb + c + (k - 3)));
-        return weno5_upwind_x2(u1, v);
-    }
-    return make_float2(vf_flux_closure(Wa, u1.x, c - i, i, n, 1), vf_flux_closure(Wb, u1.y, c - i, i, n, 1));
-}
-
-template <bool BAT>
-__global__ void __launch_bounds__(RZ_BX * RZ_BY, 5) k_rhs_les_pairs(const RhsArgs<float> a0, const int zc,
-                                                                   const Bat bat = Bat()) {
-    __shared__ float sfy[RZ_BY][RZ_BX];
-    int bz = blockIdx.z;
-    RhsArgs<float> a = a0;
-    if constexpr (BAT) {
-        long long dlt;
-        if (!batch_enter(bat, bz, dlt)) return;
-        shift_rhs_args(a, dlt);
-    }
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int x = a.lo[2] + blockIdx.x * RZ_BX + tx;
-    const int y = a.lo[1] + blockIdx.y * RZ_BY + ty;
-    const int z0 = a.lo[0] + bz * zc;
-    const int z1 = min(z0 + zc, a.hi[0]) - 1;
-    const int Nz = a.g.N[0], Ny = a.g.N[1], Nx = a.g.N[2];
-    const int sy = (int)a.g.sy, sz = (int)a.g.sz;
-    const bool valid = x < a.hi[2] && y < a.hi[1];
-    const int xs = min(x, a.hi[2] - 1), ys = min(y, a.hi[1] - 1);   // idle lanes shadow a real cell
-    const float* __restrict__ b = a.b;
-    const float* __restrict__ U0 = a.U[0];
-    const float* __restrict__ U1 = a.U[1];
-    const float* __restrict__ U2 = a.U[2];
-    const float* __restrict__ W0 = a.W[0];
-    const float* __restrict__ W1 = a.W[1];
-    const float* __restrict__ W2 = a.W[2];
-    const float* __restrict__ ke = a.ke;
-    // interior reconstructions: tracer 2 <= i <= n - 4, vortex force 3 <= i <= n - 4
-    const bool xt = xs >= 2 && xs <= Nx - 4, xv = xs >= 3 && xs <= Nx - 4;
-    const bool yt = ys >= 2 && ys <= Ny - 4, yv = ys >= 3 && ys <= Ny - 4;
-    const bool ylo = ys < Ny - 1, xlo = xs < Nx - 1;
-    const int cxy = ys * sy + xs;
-    // carried up the column: the tracer flux through the face below the cell and the
-    // two z-fluxes' velocities averaged at that face
-    float fz_prev = float(0), uu_zy = float(0), uu_zx = float(0);
-    if (z0 > 0) {
-        const int c = (z0 - 1) * sz + cxy;
-        int oz[7];
-#pragma unroll
-        for (int k = 0; k < 7; ++k) oz[k] = c + (k - 3) * sz;
-        const int zm = z0 - 1;
-        fz_prev = tr_flux32(b, __ldg(U2 + c), c, zm, Nz, sz, zm >= 2 && zm <= Nz - 4, oz);
-        if (ylo) uu_zy = float(0.5) * (__ldg(U2 + c) + __ldg(U2 + c + sy));
-        if (xlo) uu_zx = float(0.5) * (__ldg(U2 + c) + __ldg(U2 + c + 1));
-    }
-    for (int z = z0; z <= z1; ++z) {
-        const int c = z * sz + cxy;
-        const bool zt = z >= 2 && z <= Nz - 4, zv = z >= 3 && z <= Nz - 4;
-        const bool zlo = z < Nz - 1;
-        // The fluxes are formed direction by direction (z, y, x: one set of offsets
-        // live at a time) and summed afterwards in the order of TracerMarch::step and
-        // vortex_force_cell.
-        float fz, f4 = float(0), f5 = float(0);
-        {
-            int oz[7];
-#pragma unroll
-            for (int k = 0; k < 7; ++k) oz[k] = c + (k - 3) * sz;
-            fz = tr_flux32(b, __ldg(U2 + c), c, z, Nz, sz, zt, oz);
-            // f4 (ylo): u_j += U^k w_i along k (U^k averaged along j); f5 (xlo): u_i -= U^k
-            // w_j along k (U^k averaged along i); reconstructed as a pair
-            float2 u45 = make_float2(0.f, 0.f);
-            if (ylo) {
-                const float uu1 = float(0.5) * (__ldg(U2 + c) + __ldg(U2 + c + sy));
-                const float uu0 = z > 0 ? uu_zy : float(0);
-                uu_zy = uu1;
-                u45.x = float(0.5) * (uu0 + uu1);
-            }
-            if (xlo) {
-                const float uu1 = float(0.5) * (__ldg(U2 + c) + __ldg(U2 + c + 1));
-                const float uu0 = z > 0 ? uu_zx : float(0);
-                uu_zx = uu1;
-                u45.y = float(0.5) * (uu0 + uu1);
-            }
-            if (ylo || xlo) {
-                const float2 f45 = vf_flux32_x2(W0, W1, u45, c, z, Nz, sz, zv, oz);
-                f4 = f45.x;
-                f5 = f45.y;
-            }
-        }
-        float fy, fym, f2 = float(0), f3 = float(0);
-        {
-            int oy[7];
-#pragma unroll
-            for (int k = 0; k < 7; ++k) oy[k] = c + (k - 3) * sy;
-            fy = tr_flux32(b, __ldg(U1 + c), c, ys, Ny, sy, yt, oy);
-            sfy[ty][tx] = fy;
-            __syncthreads();
-            fym = (ty > 0) ? sfy[ty - 1][tx] : float(0);
-            __syncthreads();
-            // f2 (xlo): u_i += U^j w_k along j (U^j averaged along i); f3 (zlo): u_k -= U^j
-            // w_i along j (U^j averaged along k)
-            float2 u23 = make_float2(0.f, 0.f);
-            if (xlo) {
-                const float uu1 = float(0.5) * (__ldg(U1 + c) + __ldg(U1 + c + 1));
-                const float uu0 = ys > 0 ? float(0.5) * (__ldg(U1 + c - sy) + __ldg(U1 + c - sy + 1)) : float(0);
-                u23.x = float(0.5) * (uu0 + uu1);
-            }
-            if (zlo) {
-                const float uu1 = float(0.5) * (__ldg(U1 + c) + __ldg(U1 + c + sz));
-                const float uu0 = ys > 0 ? float(0.5) * (__ldg(U1 + c - sy) + __ldg(U1 + c - sy + sz)) : float(0);
-                u23.y = float(0.5) * (uu0 + uu1);
-            }
-            if (xlo || zlo) {
-                const float2 f23 = vf_flux32_x2(W2, W0, u23, c, ys, Ny, sy, yv, oy);
-                f2 = f23.x;
-                f3 = f23.y;
-            }
-        }
-        if (ty == 0 && ys > 0) {   // the face below the block's first row
-            const int cm = c - sy;
-            int om[7];
-#pragma unroll
-            for (int k = 0; k < 7; ++k) om[k] = cm + (k - 3) * sy;
-            fym = tr_flux32(b, __ldg(U1 + cm), cm, ys - 1, Ny, sy, ys - 1 >= 2 && ys - 1 <= Ny - 4, om);
-        }
-        float fx, fxm, f1 = float(0), f6 = float(0);
-        {
-            fx = tr_flux32x(b, __ldg(U0 + c), c, xs, Nx, xt);
-            fxm = __shfl_up_sync(0xffffffffu, fx, 1);
-            if (tx == 0 && xs > 0) fxm = tr_flux32x(b, __ldg(U0 + c - 1), c - 1, xs - 1, Nx,
-                                                     xs - 1 >= 2 && xs - 1 <= Nx - 4);
-            // f1 (ylo): u_j -= U^i w_k along i (U^i averaged along j); f6 (zlo): u_k += U^i
-            // w_j along i (U^i averaged along k)
-            float2 u16 = make_float2(0.f, 0.f);
-            if (ylo) {
-                const float uu1 = float(0.5) * (__ldg(U0 + c) + __ldg(U0 + c + sy));
-                float uu0 = __shfl_up_sync(0xffffffffu, uu1, 1);
-                if (tx == 0) uu0 = xs > 0 ? float(0.5) * (__ldg(U0 + c - 1) + __ldg(U0 + c - 1 + sy)) : float(0);
-                u16.x = float(0.5) * (uu0 + uu1);
-            }
-            if (zlo) {
-                const float uu1 = float(0.5) * (__ldg(U0 + c) + __ldg(U0 + c + sz));
-                float uu0 = __shfl_up_sync(0xffffffffu, uu1, 1);
-                if (tx == 0) uu0 = xs > 0 ? float(0.5) * (__ldg(U0 + c - 1) + __ldg(U0 + c - 1 + sz)) : float(0);
-                u16.y = float(0.5) * (uu0 + uu1);
-            }
-            if (ylo || zlo) {
-                const float2 f16 = vf_flux32x_x2(W2, W1, u16, c, xs, Nx, xv);
-                f1 = f16.x;
-                f6 = f16.y;
-            }
-        }
-        // ---- buoyancy advection, summed as TracerMarch::step
-        float db = (xs > 0) ? (float(0) + fxm) - fx : float(0) - fx;
-        db = (ys > 0) ? (db + fym) - fy : db - fy;
-        db = (z > 0) ? (db + fz_prev) - fz : db - fz;
-        fz_prev = fz;
-        // ---- vortex force, summed in the order of vortex_force_cell
-        float dux = float(0), duy = float(0), duz = float(0);
-        if (ylo) duy = duy - f1;
-        if (xlo) dux = dux + f2;
-        if (zlo) duz = duz - f3;
-        if (ylo) duy = duy + f4;
-        if (xlo) dux = dux - f5;
-        if (zlo) duz = duz + f6;
-        // ---- Bernoulli (core/bernoulli.py:14-23)
-        if (xlo) dux = sub_rn(dux, sub_rn(__ldg(ke + c + 1), __ldg(ke + c)));
-        if (ylo) duy = sub_rn(duy, sub_rn(__ldg(ke + c + sy), __ldg(ke + c)));
-        if (zlo) {
-            duz = sub_rn(duz, sub_rn(__ldg(ke + c + sz), __ldg(ke + c)));
-            if (!a.euler) duz = add_rn(duz, mul_rn(a.half_dz, add_rn(__ldg(b + c + sz), __ldg(b + c))));
-        }
-        if (a.terms & TERM_VISC) {
-            const long long cl = c;
-            const int pos[3] = {z, ys, xs};
-            for (int pass = 0; pass < 3; ++pass) {
-                const int d = 2 - pass;
-                const float cf = a.vcoef[pass];
-                dux = dux + cf * lap1d(a.u[0], a.g, cl, pos[d], d);
-                duy = duy + cf * lap1d(a.u[1], a.g, cl, pos[d], d);
-                duz = duz + cf * lap1d(a.u[2], a.g, cl, pos[d], d);
-            }
-        }
-        if (valid) {
-            a.ds[0][c] = db;
-            a.ds[1][c] = dux;
-            a.ds[2][c] = duy;
-            a.ds[3][c] = duz;
-        }
-    }
-}
-}  // namespace pairs
 
 // advection of one passive tracer (core/tracer.py:59-72) with the same flux sharing
 template <typename T, bool DIFF>
@@ -1039,24 +780,13 @@ static int rhs32_chunk(long long columns, int nz) {
     return zc;
 }
 
-// Array cells below which the right-hand side keeps the reconstructions from the values, in pairs. Large grids
-// are bound by instruction issue, where the differences gain 10% (k_rhs_les); small ones mostly wait for loads and
-// launches: differences / pairs, a 48^3 mixed step 831 / 835 us, 64 x 64 x 32 960 / 963, 96^3 1382 / 1403, ten steps of
-// eight batched 64^3 runs 17.1 / 17.6 ms. There the constant of a closed or triply periodic box's pressure,
-// which the singular equation leaves to the rounding of the velocity, moves by 1e-7 to 1e-6 of p with the form of a
-// reconstruction (1e-8 on 256^3 cells); this form keeps it to the bit.
-constexpr long long RHS32_SMALL = 1 << 20;
-
 template <typename T, bool BAT>
 static void launch_rhs_les(dim3 grd, dim3 blk, cudaStream_t st, const RhsArgs<T>& a, const Bat& bat) {
     if constexpr (sizeof(T) == sizeof(float)) {
         const int nz = a.hi[0] - a.lo[0], nrun = BAT ? bat.nrun : 1;
         const int zc = rhs32_chunk((long long)grd.x * grd.y * nrun, nz);
         grd.z = (unsigned)((nz + zc - 1) / zc * nrun);
-        if (a.g.vol < RHS32_SMALL)
-            pairs::k_rhs_les_pairs<BAT><<<grd, blk, 0, st>>>(a, zc, bat);
-        else
-            k_rhs_les<T, BAT><<<grd, blk, 0, st>>>(a, zc, bat);
+        k_rhs_les<T, BAT><<<grd, blk, 0, st>>>(a, zc, bat);
     }
 }
 

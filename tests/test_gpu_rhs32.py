@@ -23,7 +23,6 @@ FIELDS = ["b", "p", "ke", "div", "u_i", "u_j", "u_k", "U_i", "U_j", "U_k", "vor_
 @pytest.mark.parametrize("geometry,n", [("closed", (5, 6, 7)), ("closed", (33, 5, 9)), ("closed", (32, 17, 5)),
                                         ("closed", (65, 8, 35)), ("perio_xy", (26, 35, 6)),
                                         ("perio_xyz", (7, 6, 9)), ("perio_x", (59, 16, 18)),
-                                        # from 2^20 cells on: k_rhs_les
                                         ("closed", (1201, 35, 26)), ("perio_xy", (27, 200, 190)),
                                         ("perio_xyz", (130, 101, 79))])
 def test_rhs_f32_any_extents(geometry, n, last):
