@@ -1507,19 +1507,8 @@ int launch_diag(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, int 
 // ---------------------------------------------------------------- CFL reduction
 // max over all stored points of U^2+V^2+W^2, core/nyles.py:241-251 (max is exact
 // whatever the reduction order)
-template <typename T>
-__global__ void __launch_bounds__(256) k_max_U2(const long long vol, const T* __restrict__ U,
-                                                const T* __restrict__ V, const T* __restrict__ W,
-                                                double* __restrict__ partial) {
-    double m = 0.0;
-    bool any_nan = false;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vol; i += stride) {
-        const double a = U[i], b = V[i], c = W[i];
-        const double s = __dadd_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)), __dmul_rn(c, c));
-        if (s != s) any_nan = true;
-        m = fmax(m, s);
-    }
+// block maximum of the threads' maxima and NaN flags
+__device__ __forceinline__ void max_U2_block(double m, bool any_nan, double* __restrict__ partial) {
     __shared__ double sm[8];
     __shared__ int snan;
     if (threadIdx.x == 0) snan = 0;
@@ -1533,6 +1522,70 @@ __global__ void __launch_bounds__(256) k_max_U2(const long long vol, const T* __
         v = warp_max(v);
         if (threadIdx.x == 0) partial[blockIdx.x] = snan ? __longlong_as_double(0x7ff8000000000000ULL) : v;
     }
+}
+__device__ __forceinline__ double sum_U2(double a, double b, double c) {
+    return __dadd_rn(__dadd_rn(__dmul_rn(a, a), __dmul_rn(b, b)), __dmul_rn(c, c));
+}
+
+__global__ void __launch_bounds__(256) k_max_U2(const long long vol, const double* __restrict__ U,
+                                                const double* __restrict__ V, const double* __restrict__ W,
+                                                double* __restrict__ partial) {
+    double m = 0.0;
+    bool any_nan = false;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vol; i += stride) {
+        const double s = sum_U2(U[i], V[i], W[i]);
+        if (s != s) any_nan = true;
+        m = fmax(m, s);
+    }
+    max_U2_block(m, any_nan, partial);
+}
+
+// FP32 velocities, the same doubles: a cell's sum is formed in double only where its FP32 sum
+// (three operations, within 3 x 2^-24 of it) comes within 1e-6 of the warp's largest so far. FP32 sums
+// that are NaN or infinite, or while the largest lies where FP32 loses relative precision, always are.
+// Bound by memory: 512 x 256 x 256 cells 660 -> 83 us (the double sums of every cell are three conversions
+// and five operations on the FP64 pipe).
+__global__ void __launch_bounds__(256) k_max_U2f(const long long vol, const float* __restrict__ U,
+                                                 const float* __restrict__ V, const float* __restrict__ W,
+                                                 double* __restrict__ partial) {
+    double m = 0.0;
+    bool any_nan = false;
+    float top = 0.f, skip = -1.f;   // the warp's largest FP32 sum; cells up to `skip` cannot be the maximum
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    constexpr int UN = 4;           // cells in flight
+    for (long long base = (long long)blockIdx.x * blockDim.x; base < vol; base += UN * stride) {   // one count per warp
+        float a[UN], b[UN], c[UN];
+#pragma unroll
+        for (int k = 0; k < UN; ++k) {
+            const long long i = base + k * stride + threadIdx.x;
+            const bool in = i < vol;
+            a[k] = in ? U[i] : 0.f;
+            b[k] = in ? V[i] : 0.f;
+            c[k] = in ? W[i] : 0.f;
+        }
+        bool any = false;
+        float f[UN];
+#pragma unroll
+        for (int k = 0; k < UN; ++k) {
+            f[k] = __fmaf_rn(a[k], a[k], __fmaf_rn(b[k], b[k], __fmul_rn(c[k], c[k])));
+            any |= !(f[k] <= skip);
+        }
+        if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+            for (int k = 0; k < UN; ++k) {
+                if (!(f[k] <= skip)) {
+                    const double s = sum_U2(a[k], b[k], c[k]);
+                    if (s != s) any_nan = true;
+                    m = fmax(m, s);
+                    top = fmaxf(top, fminf(f[k], 3.4e38f));   // (a NaN leaves top, an infinity stays above skip)
+                }
+            }
+            top = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(top)));   // (not negative)
+            skip = top >= 1e-30f ? top * (1.f - 1e-6f) : -1.f;
+        }
+    }
+    max_U2_block(m, any_nan, partial);
 }
 
 __global__ void k_max_final(const double* __restrict__ partial, int n, double* out) {
@@ -1561,7 +1614,9 @@ __global__ void k_max_final(const double* __restrict__ partial, int n, double* o
 template <typename T>
 int launch_max_U2(const Geom& g, const StencilPtrs<T>& s, double* partial, int npartial, double* out,
                   cudaStream_t st) {
-    k_max_U2<T><<<npartial, 256, 0, st>>>(g.vol, s.f[NYLES_F_UC_I], s.f[NYLES_F_UC_J], s.f[NYLES_F_UC_K], partial);
+    const T *U = s.f[NYLES_F_UC_I], *V = s.f[NYLES_F_UC_J], *W = s.f[NYLES_F_UC_K];
+    if constexpr (sizeof(T) == sizeof(float)) k_max_U2f<<<npartial, 256, 0, st>>>(g.vol, U, V, W, partial);
+    else k_max_U2<<<npartial, 256, 0, st>>>(g.vol, U, V, W, partial);
     k_max_final<<<1, 1024, 0, st>>>(partial, npartial, out);
     note_launch(2);
     return cuda_status(cudaGetLastError(), "max_U2 kernel");
@@ -1741,7 +1796,7 @@ extern "C" int nyles_max_U2_static_f64(const double* U, const double* V, const d
     // one block per 2^18 cells (at least one), at most NYLES_STATIC_PARTIALS blocks
     long long blocks = (n + (1LL << 18) - 1) >> 18;
     if (blocks > NYLES_STATIC_PARTIALS) blocks = NYLES_STATIC_PARTIALS;
-    k_max_U2<double><<<(unsigned)blocks, 256, 0, st>>>(n, U, V, W, partial);
+    k_max_U2<<<(unsigned)blocks, 256, 0, st>>>(n, U, V, W, partial);
     k_max_final<<<1, 1024, 0, st>>>(partial, (int)blocks, out);
     note_launch(2);
     return cuda_status(cudaGetLastError(), "max_U2_static kernel");
