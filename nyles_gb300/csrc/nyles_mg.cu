@@ -1029,7 +1029,11 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_prolong_v4(const MgGeom gf
 // 1224 us, ten steps of eight 64^3 runs 19.0 -> 18.4 ms, a 64 x 32 x 32 FP64 step 1521 -> 1431 us.
 constexpr int MG_BOTTOM_MAXLEV = 12;
 constexpr size_t MG_BOTTOM_SMEM = 200 * 1024;
-constexpr int BT_CTAS = 8, BT_THREADS = 512;
+// Threads of a block: 768 where that saves the first level a round of tasks (24 x 24 columns: 576 tasks in one
+// round instead of two, a 48^3 mixed step 828 -> 807 us, eight batched ones 16.47 -> 16.27 ms), else 512 with
+// registers for two blocks per SM: sixteen clusters of a batch do not fit side by side otherwise (sixteen 32^3
+// runs 14.4 -> 16.4 ms). 1024 threads: 843 us, and 1 to 4% slower elsewhere.
+constexpr int BT_CTAS = 8, BT_THREADS = 512, BT_MAXTHREADS = 768;
 
 struct MgBottomLevel {
     int n[3];                // z, y, x
@@ -1144,8 +1148,8 @@ __device__ __forceinline__ BottomDiag<T> bottom_diag(const MgBottomLevel& l, con
     return d;
 }
 
-template <typename T>
-__global__ void __cluster_dims__(BT_CTAS, 1, 1) __launch_bounds__(BT_THREADS, 2)
+template <typename T, int THREADS>
+__global__ void __cluster_dims__(BT_CTAS, 1, 1) __launch_bounds__(THREADS, 1024 / THREADS)
     k_mg_bottom(const __grid_constant__ MgBottom<T> a, const Bat bat = Bat()) {
     extern __shared__ __align__(16) unsigned char mg_smem[];
     int bz;
@@ -1196,13 +1200,13 @@ __global__ void __cluster_dims__(BT_CTAS, 1, 1) __launch_bounds__(BT_THREADS, 2)
 
     // ghosts across walls stay 0
     const MgBottomLevel& last = a.lev[L - 1];
-    for (int q = threadIdx.x; q < last.off + 3 * last.vol; q += BT_THREADS) sm[q] = T(0);
+    for (int q = threadIdx.x; q < last.off + 3 * last.vol; q += THREADS) sm[q] = T(0);
     cluster.sync();
     {   // level l0 starts from x = 0: its first half-sweep is y = from_zero(b)
         const MgBottomLevel& l = a.lev[0];
         const BottomSlab<T> sl = slab(l, rank);
         const int nplane = l.n[1] * l.n[2], nt = ntasks(l), ob = arr(l, AB), oy = arr(l, AY);
-        for (int t = threadIdx.x; t < nt; t += BT_THREADS) {
+        for (int t = threadIdx.x; t < nt; t += THREADS) {
             const BottomTask k = bottom_task(l, sl.zb, t);
             const BottomRing ring = bottom_ring(l, a.per, k.y, k.x);
             const BottomDiag<T> dg = bottom_diag(l, a.per, a.idiag, k.y, k.x);
@@ -1223,7 +1227,7 @@ __global__ void __cluster_dims__(BT_CTAS, 1, 1) __launch_bounds__(BT_THREADS, 2)
         const int nt = ntasks(l), oo = arr(l, wo);
         const T* in = sm + arr(l, wi);
         const T* b = sm + arr(l, AB);
-        for (int t = threadIdx.x; t < nt; t += BT_THREADS) {
+        for (int t = threadIdx.x; t < nt; t += THREADS) {
             const BottomTask k = bottom_task(l, sl.zb, t);
             const BottomRing ring = bottom_ring(l, a.per, k.y, k.x);
             const BottomDiag<T> dg = bottom_diag(l, a.per, a.idiag, k.y, k.x);
@@ -1254,7 +1258,7 @@ __global__ void __cluster_dims__(BT_CTAS, 1, 1) __launch_bounds__(BT_THREADS, 2)
         const int ob = arr(c, AB), oy = arr(c, AY);
         const int zc0 = fs.zb / 2, zc1 = (fs.ze + 1) / 2, ncol = c.n[1] * c.n[2];
         const int nt = rank < f.nblk ? ncol * (zc1 - zc0) : 0;
-        for (int t = threadIdx.x; t < nt; t += BT_THREADS) {
+        for (int t = threadIdx.x; t < nt; t += THREADS) {
             const int g = bottom_div(t, c.mcol), col = t - g * ncol, z = zc0 + g;
             const int y = bottom_div(col, c.mx), x = col - y * c.n[2];
             const int x0 = 2 * x, y0 = 2 * y;
@@ -1312,7 +1316,7 @@ __global__ void __cluster_dims__(BT_CTAS, 1, 1) __launch_bounds__(BT_THREADS, 2)
             const T* xc = (owner == rank ? sm : cluster.map_shared_rank(sm, owner)) + arr(c, AX);
             const int nt = ntasks(f), ox_ = arr(f, AX);
             T* xf = sm + ox_;
-            for (int t = threadIdx.x; t < nt; t += BT_THREADS) {
+            for (int t = threadIdx.x; t < nt; t += THREADS) {
                 const BottomTask k = bottom_task(f, fs.zb, t);
                 const int ic = k.x >> 1, jc = k.y >> 1;
                 const int ox = (k.x & 1) ? 1 : -1, oy = (k.y & 1) ? c.sy : -c.sy;
@@ -1359,7 +1363,7 @@ __global__ void __cluster_dims__(BT_CTAS, 1, 1) __launch_bounds__(BT_THREADS, 2)
     }
     const MgBottomLevel& l = a.lev[0];
     const int nplane = l.n[1] * l.n[2], nt = ntasks(l), zb = rank * l.pp, ox = arr(l, AX);
-    for (int t = threadIdx.x; t < nt; t += BT_THREADS) {
+    for (int t = threadIdx.x; t < nt; t += THREADS) {
         const BottomTask k = bottom_task(l, zb, t);
         for (int z = k.z0; z < k.z1; ++z)
             xg[z * nplane + k.y * l.n[2] + k.x] = sm[ox + k.p + (z - k.z0) * l.sz];
@@ -1373,7 +1377,9 @@ __global__ void __cluster_dims__(BT_CTAS, 1, 1) __launch_bounds__(BT_THREADS, 2)
 // FP32 keeps each level's roundings, so that solutions do not depend, to the bit, on which kernel a level
 // runs in: a restriction child by child and partly unfused sums in the prolongation where this level and
 // those under it hold at most 200 KB of x, b and y, as the grid kernels above.
-static long long bottom_plan(const int (*n)[3], int nlev, long long solo, MgBottomLevel* lev) {
+// Returns the elements; *cost: what the first level's rounds of tasks take.
+static long long bottom_plan(const int (*n)[3], int nlev, long long solo, int threads, MgBottomLevel* lev,
+                             long long* cost) {
     long long off = 0;
     int half = 0;   // planes per block of the next level, from the one above (0: not cut)
     for (int k = 0; k < nlev; ++k) {
@@ -1393,12 +1399,13 @@ static long long bottom_plan(const int (*n)[3], int nlev, long long solo, MgBott
         // rounds of tasks take the fewest cells, a task's start counted as two
         long long best = 1ll << 60;
         for (int zg = l.pp < 2 ? 1 : 2; zg <= 8 && (zg <= l.pp || zg <= 2); zg += zg < 2 ? 1 : 2) {
-            const long long rounds = ((long long)ncol * ((l.pp + zg - 1) / zg) + BT_THREADS - 1) / BT_THREADS;
+            const long long rounds = ((long long)ncol * ((l.pp + zg - 1) / zg) + threads - 1) / threads;
             if (rounds * (zg + 2) < best) {
                 best = rounds * (zg + 2);
                 l.zg = zg;
             }
         }
+        if (k == 0 && cost) *cost = best;
         l.ng = (l.pp + l.zg - 1) / l.zg;
         l.mx = (unsigned int)(((1ull << 32) + l.n[2] - 1) / l.n[2]);
         l.mcol = (unsigned int)(((1ull << 32) + ncol - 1) / ncol);
@@ -2613,17 +2620,19 @@ int mg_init(MgImpl* mg, int nx, int ny, int nz, int topology, int precision, int
         for (int l = L - 2; l >= 1 && L - l <= MG_BOTTOM_MAXLEV; --l) {
             if (mg->lev[l].vol > bottom_maxvol(precision)) break;
             int n[MG_BOTTOM_MAXLEV][3];
-            const size_t bytes = (size_t)bottom_plan(n, bottom_extents(mg, l, n), bottom_solo(precision), nullptr) * es;
+            const size_t bytes = (size_t)bottom_plan(n, bottom_extents(mg, l, n), bottom_solo(precision), BT_THREADS, nullptr,
+                                                     nullptr) * es;
             if (bytes > MG_BOTTOM_SMEM) break;
             mg->bottom = l;
             mg->bottom_smem = bytes;
         }
         if (mg->bottom < L) {
-            cudaError_t e = precision == NYLES_MIXED
-                                ? cudaFuncSetAttribute(k_mg_bottom<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)MG_BOTTOM_SMEM)
-                                : cudaFuncSetAttribute(k_mg_bottom<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)MG_BOTTOM_SMEM);
+            auto smem = [](auto kernel) {
+                return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MG_BOTTOM_SMEM);
+            };
+            const bool f32 = precision == NYLES_MIXED;
+            cudaError_t e = f32 ? smem(k_mg_bottom<float, BT_THREADS>) : smem(k_mg_bottom<double, BT_THREADS>);
+            if (e == cudaSuccess) e = f32 ? smem(k_mg_bottom<float, BT_MAXTHREADS>) : smem(k_mg_bottom<double, BT_MAXTHREADS>);
             if (e != cudaSuccess) return cuda_status(e, "multigrid coarse-level kernel attribute");
         }
     }
@@ -2746,13 +2755,20 @@ static void bottom(MgImpl* mg, cudaStream_t st) {
     }
     int n[MG_BOTTOM_MAXLEV][3];
     a.nlev = bottom_extents(mg, l0, n);
-    bottom_plan(n, a.nlev, bottom_solo(mg->precision), a.lev);
+    long long few = 0, many = 0;
+    const long long solo = bottom_solo(mg->precision);
+    bottom_plan(n, a.nlev, solo, BT_THREADS, nullptr, &few);
+    bottom_plan(n, a.nlev, solo, BT_MAXTHREADS, nullptr, &many);
+    const bool wide = many < few && mg->bat.nrun <= 8;
+    bottom_plan(n, a.nlev, solo, wide ? BT_MAXTHREADS : BT_THREADS, a.lev, nullptr);
     a.resmooth = l0 + a.nlev < mg->nlevels;
     a.xg = lvp<T>(mg, l0, 1);
     a.bg = lvp<T>(mg, l0, 2);
     ProfScope ps(mg->prof, 8, st);
     note_launch();
-    k_mg_bottom<T><<<bgrid(mg, dim3(BT_CTAS, 1, 1)), BT_THREADS, mg->bottom_smem, st>>>(a, mg->bat);
+    const dim3 grd = bgrid(mg, dim3(BT_CTAS, 1, 1));
+    if (wide) k_mg_bottom<T, BT_MAXTHREADS><<<grd, BT_MAXTHREADS, mg->bottom_smem, st>>>(a, mg->bat);
+    else k_mg_bottom<T, BT_THREADS><<<grd, BT_THREADS, mg->bottom_smem, st>>>(a, mg->bat);
 }
 
 // level0_last: mode of the last level-0 half-sweep (see smooth)
