@@ -129,7 +129,7 @@ struct MgImpl {
     double tol = 1e-6, omega = 0.9;
     int maxite = 20;
     MgLevelDesc lev[32];
-    int bottom = 0;                   // first level of the one-block coarse solve (nlevels: none)
+    int bottom = 0;                   // first level of the coarse solve in one cluster (nlevels: none)
     size_t bottom_smem = 0;           // its shared memory bytes
     // mixed precision: level-1 solution and right-hand side as float pairs (hi, lo);
     // `nsol` solution arrays one after the other (sol_bytes apart), `cur_sol` the one the

@@ -1149,7 +1149,7 @@ __device__ __forceinline__ BottomDiag<T> bottom_diag(const MgBottomLevel& l, con
 }
 
 template <typename T, int THREADS>
-__global__ void __cluster_dims__(BT_CTAS, 1, 1) __launch_bounds__(THREADS, 1024 / THREADS)
+__global__ void __cluster_dims__(BT_CTAS, 1, 1) __launch_bounds__(THREADS <= 512 ? THREADS : 1024, THREADS <= 512 ? 2 : 1)
     k_mg_bottom(const __grid_constant__ MgBottom<T> a, const Bat bat = Bat()) {
     extern __shared__ __align__(16) unsigned char mg_smem[];
     int bz;
@@ -2381,8 +2381,7 @@ static inline bool use_fx(const MgImpl* mg, int l) {
 }
 
 // the 4-cell vector kernels apply to a level whose x and z extents allow them; zc = the
-// z cells per thread (V4_ZC on level 0 and for the float-pair and Krylov kernels,
-// lvl_zc below)
+// z cells per thread (V4_ZC for the float-pair and Krylov kernels, lvl_zc below for the others)
 static inline bool use_v4(const MgImpl* mg, const int n[3], int zc = V4_ZC) {
     return mg->vec4 && n[2] % 4 == 0 && n[0] % zc == 0;
 }
@@ -2741,7 +2740,7 @@ static void smooth(MgImpl* mg, int l, cudaStream_t st, int last_mode, bool from_
 }
 
 // solvers.f90:35-55
-// levels mg->bottom..L-1 of the V-cycle in one block (k_mg_bottom)
+// levels mg->bottom..L-1 of the V-cycle in one cluster of blocks (k_mg_bottom)
 template <typename T>
 static void bottom(MgImpl* mg, cudaStream_t st) {
     const int l0 = mg->bottom;
@@ -2775,7 +2774,7 @@ static void bottom(MgImpl* mg, cudaStream_t st) {
 template <typename T>
 static void vcycle(MgImpl* mg, cudaStream_t st, int level0_last) {
     const int L = mg->nlevels;
-    const int B = mg->bottom;   // < L: levels B..L-1 in one block
+    const int B = mg->bottom;   // < L: levels B..L-1 in one cluster
     // The first half-sweep of level 0 was written by the stop-test residual kernel that
     // precedes every V-cycle (k_mg_resid_sweep; mixed: k_mg_resid_df, from a zero
     // correction); every restricted level gets it from the restriction.

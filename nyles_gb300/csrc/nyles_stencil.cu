@@ -773,7 +773,7 @@ __global__ void __launch_bounds__(256) k_tracer_linear(const Geom g, const T* __
 // selects k_rhs_march instead (values equal to rounding).
 // Planes per thread of the FP32 marches: 16 where that gives every SM its five blocks, fewer on small
 // grids (each thread starts with the flux below its first plane, a tenth of a plane's work): 16 / 2
-// planes of a 48^3 right-hand side (36 / 288 blocks) 118 / 19 us.
+// planes of a 48^3 right-hand side (36 / 288 blocks) 118 / 21 us.
 static int rhs32_chunk(long long columns, int nz) {
     int zc = 16;
     while (zc > 2 && columns * ((nz + zc - 1) / zc) < 152 * 5) zc /= 2;
