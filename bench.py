@@ -227,40 +227,46 @@ def mg_levels(n):
     return levels
 
 
-# FP64 flops (DADD + DMUL + 2 x DFMA thread instructions) per interior cell of one
-# k_rhs_march<double, 1, 1, 0> launch, counted by ncu on the 128^3 case of this workload
-# (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on: 223.5 + 237.8 + 2 x 237.5
-# per cell), and the FP64 instructions (issue slots) behind them
-RHS_FP64_OPS_PER_CELL = 936
-RHS_FP64_INSTR_PER_CELL = 699
+# FP64 flops (DADD + DMUL + 2 x DFMA thread instructions) per interior cell of one FP64 right-hand
+# side (three k_line launches and the terms without reconstructions), counted by ncu on the 128^3
+# case of this workload (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on), and the FP64
+# instructions (issue slots) behind them
+RHS_FP64_OPS_PER_CELL = 599
+RHS_FP64_INSTR_PER_CELL = 396
 # DRAM bytes (read + write) per interior cell of one launch: ncu, FP64 at 128^3
-# (159.0 + 43.7 MB), mixed (k_rhs_les) at 256^3 (614.8 + 257.5 MB)
-RHS_DRAM_BYTES_PER_CELL = {8: 202.72e6 / 128 ** 3, 4: 872.35e6 / 256 ** 3}
+# (48.0 + 133.6 + 146.0 + 143.1 MB), mixed (k_rhs_les) at 256^3 (614.8 + 257.5 MB)
+RHS_DRAM_BYTES_PER_CELL = {8: 470.7e6 / 128 ** 3, 4: 872.35e6 / 256 ** 3}
 # DRAM bytes of one level-0 Jacobi half-sweep launch at 256^3, mixed (ncu, vector form:
 # 134.3 + 40.9 MB; algorithmic 201.3 MB, the rest of the output still in L2 at the end)
 JACOBI_F32_L0_DRAM_BYTES_256 = 175.2e6
 
 
-def mg_bottom_level(levels, elem, smem=200 * 1024, maxvol_fp64=1024):
-    """First level of the one-block coarse solve (the library's rule: the coarsest
-    levels whose x, b, y fit in `smem` bytes, two levels at least, never level 0; in
-    FP64 no level above `maxvol_fp64` cells)."""
+def mg_bottom_level(levels, elem, smem=200 * 1024, maxvol_fp64=1024, cluster=False):
+    """First level of the coarse solve: the coarsest levels whose x, b, y fit in `smem` bytes,
+    two levels at least, never level 0; in FP64 no level above `maxvol_fp64` cells. With `cluster`
+    the library's rule (a cluster of blocks that holds slabs of them): levels of at most 2^15
+    cells in FP32, 2^12 in FP64; the slabs fit whenever the cells do."""
     L = len(levels)
     bottom, total = L, 0
     for l in range(L - 1, 0, -1):
         z, y, x = levels[l]
-        total += 3 * z * y * x * elem
-        if total > smem:
-            break
-        if elem == 8 and z * y * x > maxvol_fp64:
-            break
+        if cluster:
+            if z * y * x > (1 << 15 if elem == 4 else 1 << 12):
+                break
+        else:
+            total += 3 * z * y * x * elem
+            if total > smem:
+                break
+            if elem == 8 and z * y * x > maxvol_fp64:
+                break
         if L - l >= 2:
             bottom = l
     return bottom
 
 
-def roofline(kernel, ph, n, elem, peak, peak_kind, fp64_peak, nv=None, solves=None, krylov=False):
-    """Roofline of one kernel family from the CUDA-event phase times.
+def roofline(kernel, ph, n, elem, peak, peak_kind, fp64_peak, nv=None, solves=None, krylov=False,
+             cluster=False):
+    """Roofline of one kernel family from the CUDA-event phase times (cluster: see mg_bottom_level).
 
     rhs       : one launch reads b, U(3), vor(3), ke and writes 4 registers: 12 words
                 per interior cell (the periodic halo's tendencies are not computed). In FP64 the kernel is bound by the FP64
@@ -270,11 +276,11 @@ def roofline(kernel, ph, n, elem, peak, peak_kind, fp64_peak, nv=None, solves=No
                 two) and the HBM figures beside it.
     mg_smooth : each Jacobi half-sweep reads its input and b and writes its output, 3
                 words per level cell; per V-cycle, on each grid level above the
-                one-block coarse levels: 3 half-sweeps (the first of the pre-smoothing
+                coarse levels of the cluster kernel: 3 half-sweeps (the first of the pre-smoothing
                 is written by the kernel that sets b; FP64 level 0, warm-started: 4),
                 plus, in mixed precision, the float-pair solution read and written by
                 the last level-0 half-sweep (16 B per cell; the Krylov solve instead
-                reads q, 4 B); the one-block coarse solve reads b and writes x of its
+                reads q, 4 B); the coarse solve reads b and writes x of its
                 first level.
     mg_norm   : mixed precision, the float-pair outer iteration per solve and level-0
                 cell: sum(b^2) 8 B, nv + 1 residuals of 24 B, and per Krylov iteration
@@ -296,17 +302,17 @@ def roofline(kernel, ph, n, elem, peak, peak_kind, fp64_peak, nv=None, solves=No
         if elem == 8 and fp64_peak:
             flops = RHS_FP64_OPS_PER_CELL * vol / (avg * 1e-3) / 1e12
             issue = RHS_FP64_INSTR_PER_CELL * vol / (avg * 1e-3) / 1e12
-            return {"kernel": "k_rhs_march", "bound": "fp64", "achieved": flops, "peak": fp64_peak,
+            return {"kernel": "k_line", "bound": "fp64", "achieved": flops, "peak": fp64_peak,
                     "unit": "TFLOP/s", "peak_kind": "measured (cuBLAS DGEMM, torch.mm float64 8192^3)",
                     "frac": flops / fp64_peak, "fp64_flops_per_cell": RHS_FP64_OPS_PER_CELL,
                     "fp64_instructions_per_cell": RHS_FP64_INSTR_PER_CELL,
                     "fp64_issue_frac": issue / (fp64_peak / 2), "avg_launch_ms": avg,
                     "traffic": hbm["traffic"], "hbm": hbm}
-        out.update({"kernel": "k_rhs_march", "avg_launch_ms": avg})
+        out.update({"kernel": "k_rhs_les" if elem == 4 else "k_line", "avg_launch_ms": avg})
         out.update({k: v for k, v in hbm.items() if k not in ("peak", "unit", "peak_kind", "frac")})
     elif kernel == "mg_smooth":
         lev = mg_levels(n)
-        B = mg_bottom_level(lev, elem)
+        B = mg_bottom_level(lev, elem, cluster=cluster)
         vol = [z * y * x for (z, y, x) in lev]
         per_vcycle = sum((4 if (l == 0 and elem == 8) else 3) * 3 * elem * vol[l] for l in range(B))
         if elem == 4:
@@ -853,8 +859,8 @@ def main():
         elem = 8 if main_prec == "fp64" else 4
         out["phases"] = {k: round(v["ms"] / max(1, a.profile_steps), 3) for k, v in ph.items()}
         kw = dict(nv=r["mean_vcycles_per_solve"], solves=3 * a.profile_steps, krylov=r.get("krylov", False))
-        out["roofline"] = roofline(dom, ph, n, elem, peak, peak_kind, fp64_peak, **kw)
-        out["roofline_kernels"] = {k: roofline(k, ph, n, elem, peak, peak_kind, fp64_peak, **kw)
+        out["roofline"] = roofline(dom, ph, n, elem, peak, peak_kind, fp64_peak, cluster=True, **kw)
+        out["roofline_kernels"] = {k: roofline(k, ph, n, elem, peak, peak_kind, fp64_peak, cluster=True, **kw)
                                    for k in ("rhs", "mg_smooth", "mg_norm") if k != dom}
     if "mixed" in results and main_prec != "mixed":
         mr = results["mixed"]
@@ -870,8 +876,8 @@ def main():
             out["mixed"]["phases"] = {k: round(v["ms"] / max(1, a.profile_steps), 3) for k, v in mph.items()}
             mdom = max((k for k in mph if k != "mg_solve"), key=lambda k: mph[k]["ms"])
             kw = dict(nv=mr["mean_vcycles_per_solve"], solves=3 * a.profile_steps, krylov=mr.get("krylov", False))
-            out["mixed"]["roofline"] = roofline(mdom, mph, n, 4, peak, peak_kind, None, **kw)
-            out["mixed"]["roofline_kernels"] = {k: roofline(k, mph, n, 4, peak, peak_kind, None, **kw)
+            out["mixed"]["roofline"] = roofline(mdom, mph, n, 4, peak, peak_kind, None, cluster=True, **kw)
+            out["mixed"]["roofline_kernels"] = {k: roofline(k, mph, n, 4, peak, peak_kind, None, cluster=True, **kw)
                                                 for k in ("rhs", "mg_smooth", "mg_norm") if k != mdom}
     if a.serving_requests > 0:
         out["serving"] = time_serving(a)
