@@ -723,8 +723,9 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_prolong(const MgGeom gf, T
 // The FP64 prolongation, one coarse column per thread: the 8 fine cells of a coarse cell share
 // the x interpolations of its three coarse rows and the y interpolations of each plane, 26
 // FP64 instructions for 8 cells where the per-fine-column form (k_mg_prolong) takes 40: 215 ->
-// 127 us into 256^3, 28 -> 21 us into 128^3, FP64-bound. CZ coarse planes per thread; fine extents are
-// twice the coarse ones (every FP64 level: only the coarsest may have odd extents).
+// 127 us into 256^3, 28 -> 21 us into 128^3, FP64-bound. CZ coarse planes per thread, and two that it shares
+// with its neighbours: 8 where the blocks still fill the chip (a 256^3 step 86.8 ms with 4, 86.3 with 8, 86.9 with 16,
+// 87.6 with 2). Fine extents are twice the coarse ones (every FP64 level: only the coarsest may have odd extents).
 template <int CZ>
 __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_prolong_f64(const MgGeom gf, double* __restrict__ xf,
                                                                  const MgGeom gc, const double* __restrict__ xc) {
@@ -2842,8 +2843,14 @@ static void vcycle(MgImpl* mg, cudaStream_t st, int level0_last) {
                 }
             }
             if constexpr (sizeof(T) == sizeof(double)) {
-                if (use_fx(mg, l))   // enough columns for 4 coarse planes per thread
-                    k_mg_prolong_f64<4><<<grid_zc(gc.n, 4), kBlk, 0, st>>>(gf, lvp<T>(mg, l, 1), gc, lvp<T>(mg, l + 1, 1));
+                if (use_fx(mg, l))   // enough columns for 4 coarse planes per thread, or 8
+                {
+                    const dim3 g8 = grid_zc(gc.n, 8);
+                    if (blocks(g8) >= 4 * 152)
+                        k_mg_prolong_f64<8><<<g8, kBlk, 0, st>>>(gf, lvp<T>(mg, l, 1), gc, lvp<T>(mg, l + 1, 1));
+                    else
+                        k_mg_prolong_f64<4><<<grid_zc(gc.n, 4), kBlk, 0, st>>>(gf, lvp<T>(mg, l, 1), gc, lvp<T>(mg, l + 1, 1));
+                }
                 else
                     k_mg_prolong_f64<1><<<grid_zc(gc.n, 1), kBlk, 0, st>>>(gf, lvp<T>(mg, l, 1), gc, lvp<T>(mg, l + 1, 1));
             } else if (!done && mg->bat.tab)

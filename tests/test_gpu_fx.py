@@ -31,7 +31,9 @@ def _rhs(kind, shape, rng):
 @pytest.mark.parametrize("topology,n,kind", [
     ("closed", (64, 64, 64), "smooth"), ("perio_xyz", (64, 64, 64), "spread"), ("perio_xy", (64, 64, 64), "point"),
     ("perio_x", (128, 40, 56), "smooth"), ("closed", (48, 104, 56), "spread"), ("perio_xyz", (80, 60, 60), "smooth"),
-    ("perio_y", (32, 128, 128), "point")])
+    ("perio_y", (32, 128, 128), "point"),
+    # 8 coarse planes per thread in the prolongation into level 0, the last thread 4
+    ("perio_xyz", (264, 264, 152), "smooth"), ("closed", (264, 264, 152), "smooth")])
 def test_fx_vcycle_against_oracle(topology, n, kind):
     from nyles_gb300.multigrid import MG
     nx, ny, nz = n
