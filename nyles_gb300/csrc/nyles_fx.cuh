@@ -7,7 +7,8 @@
 // 64 of the tile's largest convert without loss (53 + 6 bits), smaller ones to 2^-59 of it,
 // where the double sum rounds every partial sum to 2^-53 of itself. A tile in which some
 // thread's own values are all more than 64 times smaller than the largest, or not finite,
-// is summed in doubles instead.
+// is summed in doubles instead,
+// as one whose sums could leave the range of the doubles.
 #pragma once
 #include "nyles_common.cuh"
 
@@ -15,6 +16,7 @@ namespace nyles {
 
 constexpr int FX_RANGE = 6;          // exponents below the tile's largest that stay exact
 constexpr int FX_EMIN = 128;         // biased exponents below this: sum in doubles
+constexpr int FX_EMAX = 0x7f6;       // and above this: a sum of eight residuals reaches 2^7 times the largest value
 
 // |x|'s upper word: ordered as |x|, its exponent in bits 20..30
 __device__ __forceinline__ unsigned int fx_mag(double x) { return (unsigned int)__double2hiint(x) & 0x7fffffffu; }

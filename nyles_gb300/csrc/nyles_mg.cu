@@ -1646,7 +1646,7 @@ __global__ void __launch_bounds__(MG_BX * MG_BY, 3) k_mg_fx(const MgGeom g, cons
         __syncthreads();
         const int E = (int)(__reduce_max_sync(0xffffffffu, swarp[0][tx % BY]) >> 20);
         const int Emin = (int)(__reduce_min_sync(0xffffffffu, swarp[1][tx % BY]) >> 20);
-        fx = E >= FX_EMIN && E < 0x7ff && E - Emin <= FX_RANGE;
+        fx = E >= FX_EMIN && E <= FX_EMAX && E - Emin <= FX_RANGE;
         // MODE 2: eight residuals stay below 2^63 in units eight times as large
         Eu = MODE == 2 ? E + 3 : E;
         if (fx) {
