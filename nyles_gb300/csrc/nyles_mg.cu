@@ -1541,36 +1541,80 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_resid_sweep(const MgGeom g
 // A block owns 32 x 8 columns of ZC cells, one column per thread: every value of the tile
 // and of the ring around it is loaded first, the block agrees on the exponent, and the
 // converted columns meet in shared memory. Ghosts: 0 across a wall, else the periodic image.
-// Tiles that the level cuts off are summed in doubles, as those of too wide a range.
+// Tiles that the level cuts off, and those beyond the integers' exponents, are summed in doubles. So is, by
+// itself, a sum whose operands all lie more than 64 times below the tile's largest value (a thread
+// looks closer only where the cells above and below a cell, its b and itself do); in MODE 2 a
+// coarse cell's, where that holds for its eight children.
 // MODE 0: out = x - (omega/diag) r. MODE 1: also the block's sum of r^2. MODE 2: the coarse
 // right-hand side 0.5 * (sum of r over the 8 children) and its first half-sweep (k_mg_restrict);
 // fine extents are twice the coarse ones.
 
-// r of the thread's column in doubles (any tile); MODE 2: the sums over the pairs in z and x
-// go to `sums` [ZC/2][BY][BX/2] as bit patterns of doubles
+// one cell in doubles: r, and what the kernel stores
+template <int MODE>
+__device__ __forceinline__ double fx_cell_double(const MgGeom& g, const double* __restrict__ v,
+                                                 const double* __restrict__ b, double* __restrict__ out, int z, int y, int x) {
+    const long long c = mg_at(g, z, y, x);
+    const double xc = v[c], sum = mg_nsum(v, g, z, y, x);
+    const int dg = mg_diag(g, z, y, x);
+    const double r = fma((double)dg, xc, b[c]) - sum;
+    if (MODE == 0) out[c] = fma(g.idiag[dg], sum - b[c], (1.0 - g.idiag[1]) * xc);
+    else if (MODE == 1) out[c] = fma(-g.idiag[dg], r, xc);
+    return r;
+}
+// the cells of a warp's row that `redo` names, bit k for plane zb + k of a lane's column, shared out among
+// the lanes (one round trip to memory for up to 32 of them); the sum of r^2
+template <int ZC, int MODE>
+__device__ __noinline__ double fx_redo_double(const MgGeom& g, const double* __restrict__ v, const double* __restrict__ b,
+                                              double* __restrict__ out, int xb, int y, int zb, unsigned int redo) {
+    unsigned int lanes[ZC];
+    int total = 0;
+#pragma unroll
+    for (int k = 0; k < ZC; ++k) {
+        lanes[k] = __ballot_sync(0xffffffffu, redo >> k & 1u);
+        total += __popc(lanes[k]);
+    }
+    double s = 0.0;
+    for (int j = threadIdx.x; j < total; j += 32) {
+        int first = 0, pos = 0, z = 0;
+        unsigned int w = 0;
+#pragma unroll
+        for (int k = 0; k < ZC; ++k) {
+            const int n = __popc(lanes[k]);
+            if (j >= first && j < first + n) {
+                w = lanes[k];
+                pos = j - first;
+                z = zb + k;
+            }
+            first += n;
+        }
+        for (; pos; --pos) w &= w - 1;
+        const double r = fx_cell_double<MODE>(g, v, b, out, z, y, xb + __ffs((int)w) - 1);
+        if (MODE == 1) s = fma(r, r, s);
+    }
+    return s;
+}
+__device__ __noinline__ double fx_restrict_double(const MgGeom& g, const double* __restrict__ v,
+                                                  const double* __restrict__ b, int z, int y, int x) {
+    return mg_restrict_cell(g, v, b, z, y, x);
+}
+
+// the thread's column in doubles (any tile); MODE 2: the sums over the pairs in z and x
+// go to `sums` [ZC/2][BY][BX/2]
 template <int ZC, int MODE>
 __device__ __noinline__ double fx_tile_double(const MgGeom& g, const double* __restrict__ v, const double* __restrict__ b,
-                                              double* __restrict__ out, int x, int y, int zb, long long* sums) {
+                                              double* __restrict__ out, int x, int y, int zb, double* sums) {
     const bool act = x < g.n[2] && y < g.n[1];
     double s = 0.0, pair = 0.0;
     for (int k = 0; k < ZC; ++k) {
         const int z = zb + k;
         double r = 0.0;
-        if (act && z < g.n[0]) {
-            const long long c = mg_at(g, z, y, x);
-            const double xc = v[c];
-            const int dg = mg_diag(g, z, y, x);
-            r = fma((double)dg, xc, b[c]) - mg_nsum(v, g, z, y, x);
-            if (MODE == 0) out[c] = fma(g.idiag[dg], mg_nsum(v, g, z, y, x) - b[c], (1.0 - g.idiag[1]) * xc);
-            else if (MODE == 1) out[c] = fma(-g.idiag[dg], r, xc);
-            if (MODE == 1) s = fma(r, r, s);
-        }
+        if (act && z < g.n[0]) r = fx_cell_double<MODE>(g, v, b, out, z, y, x);
+        if (MODE == 1) s = fma(r, r, s);
         if (MODE == 2) {
             pair = (k & 1) ? pair + r : r;
             if (k & 1) {
                 const double w = pair + __shfl_down_sync(0xffffffffu, pair, 1);
-                if ((threadIdx.x & 1) == 0)
-                    sums[((k >> 1) * MG_BY + threadIdx.y) * (MG_BX / 2) + (threadIdx.x >> 1)] = __double_as_longlong(w);
+                if ((threadIdx.x & 1) == 0) sums[((k >> 1) * MG_BY + threadIdx.y) * (MG_BX / 2) + (threadIdx.x >> 1)] = w;
             }
         }
     }
@@ -1584,16 +1628,21 @@ __global__ void __launch_bounds__(MG_BX * MG_BY, 3) k_mg_fx(const MgGeom g, cons
                                                            double* __restrict__ bc) {
     constexpr int BX = MG_BX, BY = MG_BY, NT = BX * BY;
     __shared__ long long tile[ZC][BY + 2][BX + 2];
-    __shared__ unsigned int swarp[2][BY];
+    __shared__ unsigned int swarp[BY];
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * BX + tx;
     const int nx = g.n[2], ny = g.n[1], nz = g.n[0];
     const int xb = blockIdx.x * BX, yb = blockIdx.y * BY, zb = blockIdx.z * ZC;
     const int x = xb + tx, y = yb + ty;
     const long long sy = nx, sz = (long long)ny * nx;
-    long long* const sums = &tile[0][0][0];   // MODE 2: [ZC/2][BY][BX/2], after the tile has been read
+    // MODE 2, after the tile has been read: [ZC/2][BY][BX/2] sums over the pairs in z and x
+    constexpr int NS = ZC / 2 * BY * (BX / 2);
+    unsigned long long* const sums_lo = reinterpret_cast<unsigned long long*>(&tile[0][0][0]);
+    int* const sums_hi = reinterpret_cast<int*>(sums_lo + NS);
+    unsigned char* const sums_small = reinterpret_cast<unsigned char*>(sums_hi + NS);
+    double* const sums = reinterpret_cast<double*>(&tile[0][0][0]);
     double s = 0.0;
     bool fx = xb + BX <= nx && yb + BY <= ny && zb + ZC <= nz;
-    int Eu = 0;
+    int E = 0;
     if (fx) {
         const MgNb nlo = mg_nb(zb, nz, g.per[0], sz), nhi = mg_nb(zb + ZC - 1, nz, g.per[0], sz);
         const MgNb ylo = mg_nb(yb, ny, g.per[1], sy), yhi = mg_nb(yb + BY - 1, ny, g.per[1], sy);
@@ -1626,77 +1675,95 @@ __global__ void __launch_bounds__(MG_BX * MG_BY, 3) k_mg_fx(const MgGeom g, cons
             hx[h] = 0.0;
             if (q < 2 * ZC * BY && ((q & 1) ? xhi.wp : xlo.wm)) hx[h] = row[(q & 1) ? BX - 1 + xhi.op : xlo.om];
         }
-        // the tile's exponent, and the smallest one among the threads' own values (with the
-        // neighbouring columns': a stencil next to a zero of x is as large as its neighbours)
-        unsigned int own = max(fx_mag(col[0]), fx_mag(col[ZC + 1]));
+        // the tile's exponent, and the smallest one that the thread can vouch for among its sums: the largest
+        // of the cells above and below a cell, its b and, where the sum has it, itself
+        unsigned int all = 0, low = 0x7fffffffu;
 #pragma unroll
-        for (int k = 0; k < ZC; ++k) own = max(own, max(fx_mag(col[k + 1]), fx_mag(bcol[k])));
-        unsigned int all = own;
+        for (int k = 0; k < ZC; ++k) {
+            unsigned int m = max(max(fx_mag(col[k]), fx_mag(col[k + 2])), fx_mag(bcol[k]));
+            if (MODE != 0) m = max(m, fx_mag(col[k + 1]));
+            all = max(all, m);
+            low = min(low, m);
+        }
 #pragma unroll
         for (int h = 0; h < NHY; ++h) all = max(all, fx_mag(hy[h]));
 #pragma unroll
         for (int h = 0; h < NHX; ++h) all = max(all, fx_mag(hx[h]));
-        own = max(own, max(__shfl_up_sync(0xffffffffu, own, 1), __shfl_down_sync(0xffffffffu, own, 1)));
         all = __reduce_max_sync(0xffffffffu, all);
-        own = __reduce_min_sync(0xffffffffu, own ? own : 0x7fffffffu);
-        if (tx == 0) {
-            swarp[0][ty] = all;
-            swarp[1][ty] = own;
-        }
+        if (tx == 0) swarp[ty] = all;
         __syncthreads();
-        const int E = (int)(__reduce_max_sync(0xffffffffu, swarp[0][tx % BY]) >> 20);
-        const int Emin = (int)(__reduce_min_sync(0xffffffffu, swarp[1][tx % BY]) >> 20);
-        fx = E >= FX_EMIN && E <= FX_EMAX && E - Emin <= FX_RANGE;
-        // MODE 2: eight residuals stay below 2^63 in units eight times as large
-        Eu = MODE == 2 ? E + 3 : E;
+        E = (int)(__reduce_max_sync(0xffffffffu, swarp[tx % BY]) >> 20);
+        fx = E >= FX_EMIN && E <= FX_EMAX;
+        const bool look = (int)(low >> 20) + FX_RANGE < E;
         if (fx) {
             long long f[ZC + 2];
 #pragma unroll
-            for (int k = 0; k < ZC + 2; ++k) f[k] = fx_from(col[k], Eu);
+            for (int k = 0; k < ZC + 2; ++k) f[k] = fx_from(col[k], E);
 #pragma unroll
             for (int k = 0; k < ZC; ++k) tile[k][ty + 1][tx + 1] = f[k + 1];
 #pragma unroll
             for (int h = 0; h < NHY; ++h) {
                 const int q = ty + h * BY;
-                if (q < 2 * ZC) tile[q >> 1][(q & 1) ? BY + 1 : 0][tx + 1] = fx_from(hy[h], Eu);
+                if (q < 2 * ZC) tile[q >> 1][(q & 1) ? BY + 1 : 0][tx + 1] = fx_from(hy[h], E);
             }
 #pragma unroll
             for (int h = 0; h < NHX; ++h) {
                 const int q = tid + h * NT;
-                if (q < 2 * ZC * BY) tile[q / (2 * BY)][((q >> 1) % BY) + 1][(q & 1) ? BX + 1 : 0] = fx_from(hx[h], Eu);
+                if (q < 2 * ZC * BY) tile[q / (2 * BY)][((q >> 1) % BY) + 1][(q & 1) ? BX + 1 : 0] = fx_from(hx[h], E);
             }
             __syncthreads();
             const int dxy = (int)(x > 0 || g.per[2]) + (int)(x < nx - 1 || g.per[2]) + (int)(y > 0 || g.per[1]) +
                             (int)(y < ny - 1 || g.per[1]);
             const double idg = MODE == 2 ? 0.0 : g.idiag[dxy + 2], cff1 = 1.0 - g.idiag[1];   // idiag[1] = omega
             double* __restrict__ po = MODE == 2 ? nullptr : out + c0;
-            long long acc[MODE == 2 ? ZC / 2 : 1];
+            FxWide acc[MODE == 2 ? ZC / 2 : 1];
+            unsigned int redo = 0;   // the sums that doubles form
+            if (look) {
+#pragma unroll
+                for (int k = 0; k < ZC; ++k) {
+                    unsigned int o = fx_fold(tile[k][ty + 1][tx]) | fx_fold(tile[k][ty + 1][tx + 2]) |
+                                     fx_fold(tile[k][ty][tx + 1]) | fx_fold(tile[k][ty + 2][tx + 1]) |
+                                     fx_fold(f[k]) | fx_fold(f[k + 2]) | fx_fold(fx_round(bcol[k], E));
+                    if (MODE != 0) o |= fx_fold(f[k + 1]);
+                    redo |= (unsigned int)(o < FX_FOLD_MIN) << k;
+                }
+            }
 #pragma unroll
             for (int k = 0; k < ZC; ++k) {
                 const unsigned int dg = dxy + (k == 0 ? (int)nlo.wm : 1) + (k == ZC - 1 ? (int)nhi.wp : 1);
                 const long long sum = tile[k][ty + 1][tx] + tile[k][ty + 1][tx + 2] + tile[k][ty][tx + 1] +
                                       tile[k][ty + 2][tx + 1] + f[k] + f[k + 2];
-                const long long bk = fx_round(bcol[k], Eu);
+                const long long bk = fx_round(bcol[k], E);
                 if (MODE == 0) {
                     const double w = (k == 0 || k == ZC - 1) ? g.idiag[dg] : idg;
-                    po[k * sz] = fma(w, fx_to_double(sum - bk, Eu), cff1 * col[k + 1]);
+                    po[k * sz] = fma(w, fx_to_double(sum - bk, E), cff1 * col[k + 1]);
                 } else {
                     const long long r = bk + fx_mul(f[k + 1], dg) - sum;
                     if (MODE == 2) {
-                        acc[k >> 1] = (k & 1) ? acc[k >> 1] + r : r;
+                        if (k & 1) acc[k >> 1].add(r);
+                        else acc[k >> 1].set(r);
                     } else {
-                        const double rd = fx_to_double(r, Eu), w = (k == 0 || k == ZC - 1) ? g.idiag[dg] : idg;
+                        const double rd = fx_to_double(r, E), w = (k == 0 || k == ZC - 1) ? g.idiag[dg] : idg;
                         po[k * sz] = fma(-w, rd, col[k + 1]);
-                        s = fma(rd, rd, s);
+                        if (!(redo >> k & 1u)) s = fma(rd, rd, s);
                     }
                 }
             }
+            if (MODE != 2 && __any_sync(0xffffffffu, redo)) s += fx_redo_double<ZC, MODE>(g, v, b, out, xb, y, zb, redo);
             if (MODE == 2) {
                 __syncthreads();   // the tile has been read
+                redo &= redo >> 1;
+                redo &= __shfl_down_sync(0xffffffffu, redo, 1);
 #pragma unroll
                 for (int k = 0; k < ZC / 2; ++k) {
-                    const long long w = acc[k] + __shfl_down_sync(0xffffffffu, acc[k], 1);
-                    if ((tx & 1) == 0) sums[(k * BY + ty) * (BX / 2) + (tx >> 1)] = w;
+                    const unsigned long long w = acc[k].lo + __shfl_down_sync(0xffffffffu, acc[k].lo, 1);
+                    const int h = acc[k].hi + __shfl_down_sync(0xffffffffu, acc[k].hi, 1);
+                    if ((tx & 1) == 0) {
+                        const int q = (k * BY + ty) * (BX / 2) + (tx >> 1);
+                        sums_lo[q] = w;
+                        sums_hi[q] = h;
+                        sums_small[q] = redo >> (2 * k) & 1u;
+                    }
                 }
             }
         }
@@ -1709,8 +1776,11 @@ __global__ void __launch_bounds__(MG_BX * MG_BY, 3) k_mg_fx(const MgGeom g, cons
             const int cx = q % (BX / 2), cy = (q / (BX / 2)) % (BY / 2), cz = q / (BX / 2 * (BY / 2));
             const int X = xb / 2 + cx, Y = yb / 2 + cy, Z = zb / 2 + cz;
             if (X >= gc.n[2] || Y >= gc.n[1] || Z >= gc.n[0]) continue;
-            const long long s0 = sums[(cz * BY + 2 * cy) * (BX / 2) + cx], s1 = sums[(cz * BY + 2 * cy + 1) * (BX / 2) + cx];
-            const double t = fx ? fx_to_double(s0 + s1, Eu) : __longlong_as_double(s0) + __longlong_as_double(s1);
+            const int q0 = (cz * BY + 2 * cy) * (BX / 2) + cx, q1 = q0 + BX / 2;
+            double t;
+            if (fx && sums_small[q0] & sums_small[q1]) t = fx_restrict_double(g, v, b, Z, Y, X);
+            else if (fx) t = FxWide{sums_lo[q0] + sums_lo[q1], sums_hi[q0] + sums_hi[q1]}.value(E);
+            else t = sums[q0] + sums[q1];
             const double bv = 0.5 * t;
             const long long c = mg_at(gc, Z, Y, X);
             bc[c] = bv;
