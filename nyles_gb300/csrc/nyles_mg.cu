@@ -2445,10 +2445,17 @@ static inline dim3 bgrid(const MgImpl* mg, dim3 g) {
 // chain of FP64 instructions: 8 cells 9 us, 1 cell 4 us on 32^3 and 16^3). Measured with the line at
 // 2^15 / 2^18 / 2^19 cells / everything in doubles: a 128^3 solve 1.364 / 1.361 / 1.387 / 2.086 ms, a
 // 128 x 64 x 64 LFAM3 step 2.64 / 2.65 / 2.65 / 2.96 ms.
+// A level that the 32 x 8 x 8 tiles do not divide has cut tiles, summed in doubles cell after cell; on
+// small ones their latency shows, and the line lies higher. V-cycles in us, integers / doubles of one cell per
+// thread / of eight: 48 x 104 x 56 173 / 147 / 198, 80 x 64 x 64 184 / 161 / 207, 48 x 96 x 96 187 / 180 / 211,
+// 112 x 64 x 64 186 / 171 / 212; 80^3 191 / 194 / 224, 40 x 128 x 128 208 / 221 / 253, 48 x 192 x 96 223 / 252 / 298,
+// 144^3 389 / 547 / 536; tiles none of which is whole, 24 x 128 x 128 181 / 181 / 206.
 constexpr int FX_ZC = 8;
-constexpr long long FX_MINVOL = 1ll << 18;
+constexpr long long FX_MINVOL = 1ll << 18, FX_MINVOL_CUT = 500000;
 static inline bool use_fx(const MgImpl* mg, int l) {
-    return mg->precision == NYLES_FP64 && mg->lev[l].vol >= FX_MINVOL;
+    const MgLevelDesc& d = mg->lev[l];
+    const bool whole = d.n[2] % MG_BX == 0 && d.n[1] % MG_BY == 0 && d.n[0] % FX_ZC == 0;
+    return mg->precision == NYLES_FP64 && d.vol >= (whole ? FX_MINVOL : FX_MINVOL_CUT);
 }
 
 // the 4-cell vector kernels apply to a level whose x and z extents allow them; zc = the
