@@ -1526,7 +1526,7 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_resid_sweep(const MgGeom g
     }
     block_partial(s, partial, blockIdx.z);
     double t;
-    if (mg_fin_total(fin, partial, gridDim.x * gridDim.y * gridDim.z, t)) fin.sc[SC_RR] = t;
+    if (fin.ticket && mg_fin_total(fin, partial, gridDim.x * gridDim.y * gridDim.z, t)) fin.sc[SC_RR] = t;
 }
 
 // ---------------------------------------------------------------- FP64 levels on the integer pipes
@@ -2433,6 +2433,7 @@ __global__ void k_mg_ctl_step(double* __restrict__ sc0, cudaGraphConditionalHand
 static inline dim3 grid_zc(const int n[3], int zc) {
     return dim3((n[2] + MG_BX - 1) / MG_BX, (n[1] + MG_BY - 1) / MG_BY, (n[0] + zc - 1) / zc);
 }
+static inline long long blocks(dim3 g) { return (long long)g.x * g.y * g.z; }
 static const dim3 kBlk(MG_BX, MG_BY, 1);
 // the grid of a batched launch repeats the one-run grid along z once per run
 static inline dim3 bgrid(const MgImpl* mg, dim3 g) {
@@ -2449,13 +2450,18 @@ static inline dim3 bgrid(const MgImpl* mg, dim3 g) {
 // small ones their latency shows, and the line lies higher. V-cycles in us, integers / doubles of one cell per
 // thread / of eight: 48 x 104 x 56 173 / 147 / 198, 80 x 64 x 64 184 / 161 / 207, 48 x 96 x 96 187 / 180 / 211,
 // 112 x 64 x 64 186 / 171 / 212; 80^3 191 / 194 / 224, 40 x 128 x 128 208 / 221 / 253, 48 x 192 x 96 223 / 252 / 298,
-// 144^3 389 / 547 / 536; tiles none of which is whole, 24 x 128 x 128 181 / 181 / 206.
+// 144^3 389 / 547 / 536.
+// A level without a whole tile takes doubles: one cell per thread while that leaves few blocks (16 x 128 x 128, 2048 of
+// them: 166 / 167 / 204; 24 x 128 x 128 181 / 181 / 206), else eight (8192 or more: 16 x 256 x 256 417 / 432 / 386,
+// 4 x 512 x 512 961 / 1181 / 936, 512 x 4 x 512 193 / 186 / 178, 512 x 2 x 512 78 / 59 / 62).
 constexpr int FX_ZC = 8;
-constexpr long long FX_MINVOL = 1ll << 18, FX_MINVOL_CUT = 500000;
-static inline bool use_fx(const MgImpl* mg, int l) {
+constexpr long long FX_MINVOL = 1ll << 18, FX_MINVOL_CUT = 500000, ONE_CELL_BLOCKS = 4096;
+// cells per thread of an FP64 level's double kernels, 0: the integer sums
+static inline int fp64_zc(const MgImpl* mg, int l) {
     const MgLevelDesc& d = mg->lev[l];
-    const bool whole = d.n[2] % MG_BX == 0 && d.n[1] % MG_BY == 0 && d.n[0] % FX_ZC == 0;
-    return mg->precision == NYLES_FP64 && d.vol >= (whole ? FX_MINVOL : FX_MINVOL_CUT);
+    if (d.n[2] < MG_BX || d.n[1] < MG_BY || d.n[0] < FX_ZC) return blocks(grid_zc(d.n, 1)) <= ONE_CELL_BLOCKS ? 1 : MG_ZC;
+    const bool cut = d.n[2] % MG_BX || d.n[1] % MG_BY || d.n[0] % FX_ZC;
+    return d.vol >= (cut ? FX_MINVOL_CUT : FX_MINVOL) ? 0 : 1;
 }
 
 // the 4-cell vector kernels apply to a level whose x and z extents allow them; zc = the
@@ -2470,7 +2476,6 @@ static inline dim3 grid_v4(const int n[3], int zc = V4_ZC) {
 // Block partials of a level-0 sum over `count` blocks (which = 0, 1: two sums of one kernel): in
 // the workspace's own slots where these hold them, else in level 1's y, which holds nothing while
 // the kernels that sum over level 0 run.
-static inline long long blocks(dim3 g) { return (long long)g.x * g.y * g.z; }
 static inline bool partials_fit(const MgImpl* mg, long long count) {
     const long long es = mg->precision == NYLES_MIXED ? sizeof(float) : sizeof(double);
     return count <= mg->npartial || (mg->nlevels > 1 && mg->lev[1].vol * es >= 2 * count * (long long)sizeof(double));
@@ -2747,10 +2752,14 @@ static void smooth(MgImpl* mg, int l, cudaStream_t st, int last_mode, bool from_
     ProfScope ps(mg->prof, 8, st);
     note_launch(from_y ? 1 : 2);
     if constexpr (sizeof(T) == sizeof(double)) {   // FP64: always stored (last_mode 0)
-        if (use_fx(mg, l)) {
+        const int zc = fp64_zc(mg, l);
+        if (zc == 0) {
             const dim3 gx = grid_zc(g.n, FX_ZC);
             if (!from_y) k_mg_fx<FX_ZC, 0><<<gx, kBlk, 0, st>>>(g, x, b, y, nullptr, g, nullptr);
             k_mg_fx<FX_ZC, 0><<<gx, kBlk, 0, st>>>(g, y, b, x, nullptr, g, nullptr);
+        } else if (zc == MG_ZC) {
+            if (!from_y) k_mg_jacobi<T, 0><<<grd, kBlk, 0, st>>>(g, x, b, y, om, nullptr, nullptr, nullptr, nullptr);
+            k_mg_jacobi<T, 0><<<grd, kBlk, 0, st>>>(g, y, b, x, om, nullptr, nullptr, nullptr, nullptr);
         } else {
             const dim3 gs = grid_zc(g.n, 1);
             if (!from_y) k_mg_jacobi<T, 0, false, 1><<<gs, kBlk, 0, st>>>(g, x, b, y, om, nullptr, nullptr, nullptr, nullptr);
@@ -2879,10 +2888,15 @@ static void vcycle(MgImpl* mg, cudaStream_t st, int level0_last) {
                 }
             }
             if constexpr (sizeof(T) == sizeof(double)) {
-                if (use_fx(mg, l))
+                const int zc = fp64_zc(mg, l);
+                if (zc == 0)
                     k_mg_fx<FX_ZC, 2><<<grid_zc(gf.n, FX_ZC), kBlk, 0, st>>>(gf, lvp<T>(mg, l, 1), lvp<T>(mg, l, 2),
                                                                             lvp<T>(mg, l + 1, 3), nullptr, gc,
                                                                             lvp<T>(mg, l + 1, 2));
+                else if (zc == MG_ZC)
+                    k_mg_restrict<T><<<grid_zc(gc.n, MG_RZC), kBlk, 0, st>>>(
+                        gf, lvp<T>(mg, l, 1), lvp<T>(mg, l, 2), gc, lvp<T>(mg, l + 1, 2), lvp<T>(mg, l + 1, 3),
+                        T(mg->omega));
                 else
                     k_mg_restrict<T, false, 1><<<grid_zc(gc.n, 1), kBlk, 0, st>>>(
                         gf, lvp<T>(mg, l, 1), lvp<T>(mg, l, 2), gc, lvp<T>(mg, l + 1, 2), lvp<T>(mg, l + 1, 3),
@@ -2920,16 +2934,18 @@ static void vcycle(MgImpl* mg, cudaStream_t st, int level0_last) {
                 }
             }
             if constexpr (sizeof(T) == sizeof(double)) {
-                if (use_fx(mg, l))   // enough columns for 4 coarse planes per thread, or 8
-                {
-                    const dim3 g8 = grid_zc(gc.n, 8);
-                    if (blocks(g8) >= 4 * 152)
-                        k_mg_prolong_f64<8><<<g8, kBlk, 0, st>>>(gf, lvp<T>(mg, l, 1), gc, lvp<T>(mg, l + 1, 1));
-                    else
-                        k_mg_prolong_f64<4><<<grid_zc(gc.n, 4), kBlk, 0, st>>>(gf, lvp<T>(mg, l, 1), gc, lvp<T>(mg, l + 1, 1));
-                }
+                const int zc = fp64_zc(mg, l);
+                const double* xc = lvp<T>(mg, l + 1, 1);
+                double* xf = lvp<T>(mg, l, 1);
+                const dim3 g8 = grid_zc(gc.n, 8);
+                if (zc == 1)
+                    k_mg_prolong_f64<1><<<grid_zc(gc.n, 1), kBlk, 0, st>>>(gf, xf, gc, xc);
+                else if (zc == MG_ZC)   // (narrow levels: one fine column per thread)
+                    k_mg_prolong<T><<<grid_zc(gf.n, MG_ZC), kBlk, 0, st>>>(gf, xf, gc, xc);
+                else if (blocks(g8) >= 4 * 152)   // enough columns for 8 coarse planes per thread, or 4
+                    k_mg_prolong_f64<8><<<g8, kBlk, 0, st>>>(gf, xf, gc, xc);
                 else
-                    k_mg_prolong_f64<1><<<grid_zc(gc.n, 1), kBlk, 0, st>>>(gf, lvp<T>(mg, l, 1), gc, lvp<T>(mg, l + 1, 1));
+                    k_mg_prolong_f64<4><<<grid_zc(gc.n, 4), kBlk, 0, st>>>(gf, xf, gc, xc);
             } else if (!done && mg->bat.tab)
                 k_mg_prolong<T, true><<<bgrid(mg, grid_zc(gf.n, MG_ZC)), kBlk, 0, st>>>(
                     gf, lvp<T>(mg, l, 1), gc, lvp<T>(mg, l + 1, 1), mg->bat);
@@ -3014,22 +3030,24 @@ static void enqueue_resid_df(MgImpl* mg, cudaStream_t st) {
 // first level-0 half-sweep (k_mg_resid_sweep)
 static void enqueue_resid_sweep(MgImpl* mg, cudaStream_t st) {
     MgGeom g = mgg(mg, 0);
-    const bool fx = use_fx(mg, 0), one = !fx && partials_fit(mg, blocks(grid_zc(g.n, 1)));
+    const int zc = fp64_zc(mg, 0);
+    const bool fx = zc == 0, one = zc == 1 && partials_fit(mg, blocks(grid_zc(g.n, 1)));
     const dim3 grd = grid_zc(g.n, fx ? FX_ZC : (one ? 1 : MG_ZC));
     double* part = partials(mg, 0, blocks(grd));
     ProfScope ps(mg->prof, 11, st);
-    const MgFin fin = mg_fin(mg);
-    note_launch(fx ? 2 : 1);
-    if (fx) {   // (many blocks: the ticket took 30 us of a 128^3 level against 20 + 4.5 with the sum apart)
-        k_mg_fx<FX_ZC, 1><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2), lvp<double>(mg, 0, 3),
-                                                part, g, nullptr);
-        k_mg_final<<<1, 1024, 0, st>>>(part, (int)blocks(grd), fin.sc + SC_RR);
-    } else if (one)
-        k_mg_resid_sweep<double, 1><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2),
-                                                          lvp<double>(mg, 0, 3), mg->omega, part, fin);
+    const bool apart = fx || (!one && blocks(grd) > 1024);   // the sum (as enqueue_sumsq)
+    const MgFin fin = apart ? MgFin() : mg_fin(mg);
+    note_launch(apart ? 2 : 1);
+    const double *x = lvp<double>(mg, 0, 1), *b = lvp<double>(mg, 0, 2);
+    double* y = lvp<double>(mg, 0, 3);
+    if (fx)   // (many blocks: the ticket took 30 us of a 128^3 level against 20 + 4.5 with the sum apart)
+        k_mg_fx<FX_ZC, 1><<<grd, kBlk, 0, st>>>(g, x, b, y, part, g, nullptr);
+    else if (one)
+        k_mg_resid_sweep<double, 1><<<grd, kBlk, 0, st>>>(g, x, b, y, mg->omega, part, fin);
     else
-        k_mg_resid_sweep<double><<<grd, kBlk, 0, st>>>(g, lvp<double>(mg, 0, 1), lvp<double>(mg, 0, 2),
-                                                       lvp<double>(mg, 0, 3), mg->omega, part, fin);
+        k_mg_resid_sweep<double><<<grd, kBlk, 0, st>>>(g, x, b, y, mg->omega, part, fin);
+    if (apart)
+        k_mg_final<<<1, 1024, 0, st>>>(part, (int)blocks(grd), reinterpret_cast<double*>(mg->ws + mg->off_scalars) + SC_RR);
 }
 
 // mixed precision with krylov: after the V-cycle left z = V(r) in level 0's x (and the
