@@ -406,11 +406,14 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_jacobi(const MgGeom g, con
 #pragma unroll
             for (int k = 1; k <= ZC; ++k) col[k] = in[c0 + (k - 1) * sz];
             col[ZC + 1] = mg_ldw(in, c0 + (ZC - 1) * sz + hi.op, hi.wp);
+            const T idg = mg_idiag<T>(g, dxy + (ZC == 1 ? (int)lo.wm + (int)hi.wp : 2));
+            const T idg_lo = ZC == 1 ? idg : mg_idiag<T>(g, dxy + 1 + (int)lo.wm);
+            const T idg_hi = ZC == 1 ? idg : mg_idiag<T>(g, dxy + 1 + (int)hi.wp);
 #pragma unroll
             for (int k = 0; k < ZC; ++k) {
                 const long long c = c0 + k * sz;
-                const int dg = dxy + (k == 0 ? (int)lo.wm : 1) + (k == ZC - 1 ? (int)hi.wp : 1);
-                put(c, cell(c, col[k], col[k + 1], col[k + 2], mg_idiag<T>(g, dg)), (MODE == 2) ? dot[c] : T(0));
+                put(c, cell(c, col[k], col[k + 1], col[k + 2], k == 0 ? idg_lo : (k == ZC - 1 ? idg_hi : idg)),
+                    (MODE == 2) ? dot[c] : T(0));
             }
         } else {
             for (int z = z0; z < nz; ++z) {   // last, partial chunk
@@ -2499,10 +2502,14 @@ static inline bool use_v4_sums(const MgImpl* mg) {
 // 128 x 128 x 64 1555 / 1566; ten steps of four 48^3 runs 12.91 / 12.91 ms, of eight 16.64 / 17.61, of
 // sixteen 32^3 runs 14.72 / 15.46. The residual stays at 4 planes: one per thread, it gains 3% of a 64 x 64 x 32
 // step and loses 2% of a 64^3 one and 7% of eight batched 32^3 runs.
-constexpr long long V4_SMALL = 1 << 20;
+// Narrow levels leave lanes idle, and one plane per thread makes many blocks: 4 planes above V4_SMALL_BLOCKS of them,
+// which fill the chip (V-cycles with 4 / 1 planes, us: 96^3, 1152 blocks, 1415 / 1379 a step; 16 x 128 x 128 and
+// 16 x 1024 x 16, 2048 blocks, 100 / 99 and 110 / 113; 32 x 4 x 4096, 4096, 105 / 110; 4 x 256 x 256 and 8 x 256 x 256,
+// 8192, 135 / 153 and 169 / 183; 4 x 4 x 16384, 208 / 243). It also keeps the planes within a grid's largest z extent.
+constexpr long long V4_SMALL = 1 << 20, V4_SMALL_BLOCKS = 8 * 152;
 static inline int lvl_zc(const MgImpl* mg, int l) {
     if (l) return mg->czc;
-    if (!mg->bat.tab && mg->lev[0].vol < V4_SMALL) return 1;
+    if (!mg->bat.tab && mg->lev[0].vol < V4_SMALL && blocks(grid_v4(mg->lev[0].n, 1)) <= V4_SMALL_BLOCKS) return 1;
     return V4_ZC;
 }
 // coarse planes per thread of the restriction out of level l, fine planes per thread of
