@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, RhsMinBlocks<T>::n) k_rhs_march
 
 // ---------------------------------------------------------------- right-hand side, 32-bit offsets
 // k_rhs_march<float, true, 1, false> (buoyancy advection, WENO vortex force, Bernoulli,
-// viscosity) where a block's reach fits 32-bit byte offsets: the same operations in the same order
+// viscosity) where a block's reach fits 32-bit byte offsets (rhs32_chunk): the same operations in the same order
 // outside the reconstructions, with fewer instructions per cell:
 //  - 32-bit offsets from a block's own pointers; the six values around a face are loaded at
 //    offsets shared by every field read along that direction;
@@ -769,14 +769,18 @@ __global__ void __launch_bounds__(256) k_tracer_linear(const Geom g, const T* __
     dq[c] = acc;
 }
 
-// k_rhs_les serves FP32 arrays whose 22 planes (a block's reach) lie within 4 GB; NYLES_GB300_GENERIC_RHS=1
-// selects k_rhs_march instead (values equal to rounding).
+// k_rhs_les and k_tracer_les serve FP32 arrays whose 7 planes (the reach of a block of one plane) lie within 4 GB;
+// NYLES_GB300_GENERIC_RHS=1 selects k_rhs_march instead (values equal to rounding).
+static bool rhs32_reach(const Geom& g, int zc) { return 4 * ((zc + 6) * g.sz + 16 * g.sy + 64) < (1ll << 32); }
 // Planes per thread of the FP32 marches: 16 where that gives every SM its five blocks, fewer on small
 // grids (each thread starts with the flux below its first plane, a tenth of a plane's work): 16 / 2
-// planes of a 48^3 right-hand side (36 / 288 blocks) 118 / 21 us.
-static int rhs32_chunk(long long columns, int nz) {
+// planes of a 48^3 right-hand side (36 / 288 blocks) 118 / 21 us; fewer too where a block's planes would lie
+// beyond 4 GB, from 48.8 M cells per plane on (8200 x 6144 x 11 with a tracer 53.9 ms on the general march, 34.0 with 8
+// planes; 16400 x 8640 x 5 69.0, 59.2 with one).
+static int rhs32_chunk(const Geom& g, long long columns, int nz) {
     int zc = 16;
     while (zc > 2 && columns * ((nz + zc - 1) / zc) < 152 * 5) zc /= 2;
+    while (zc > 1 && !rhs32_reach(g, zc)) zc /= 2;
     return zc;
 }
 
@@ -784,7 +788,7 @@ template <typename T, bool BAT>
 static void launch_rhs_les(dim3 grd, dim3 blk, cudaStream_t st, const RhsArgs<T>& a, const Bat& bat) {
     if constexpr (sizeof(T) == sizeof(float)) {
         const int nz = a.hi[0] - a.lo[0], nrun = BAT ? bat.nrun : 1;
-        const int zc = rhs32_chunk((long long)grd.x * grd.y * nrun, nz);
+        const int zc = rhs32_chunk(a.g, (long long)grd.x * grd.y * nrun, nz);
         grd.z = (unsigned)((nz + zc - 1) / zc * nrun);
         k_rhs_les<T, BAT><<<grd, blk, 0, st>>>(a, zc, bat);
     }
@@ -797,7 +801,7 @@ static bool rhs32_ok(const Geom& g) {
         const char* e = getenv("NYLES_GB300_GENERIC_RHS");
         return e && e[0] == '1';
     }();
-    return !generic && 4 * (22 * g.sz + 16 * g.sy + 64) < (1ll << 32);
+    return !generic && rhs32_reach(g, 1);
 }
 
 bool make_geom(const NylesDesc* d, Geom* g) {
@@ -883,7 +887,7 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
     auto tracer32 = [&](const T* q, T* dq) {   // FP32, no diffusion
         if constexpr (sizeof(T) == sizeof(float)) {
             if (rhs32_ok<T>(g)) {
-                const int zc = rhs32_chunk((long long)grd.x * grd.y, g.N[0]);
+                const int zc = rhs32_chunk(g, (long long)grd.x * grd.y, g.N[0]);
                 const dim3 gt(grd.x, grd.y, (unsigned)((g.N[0] + zc - 1) / zc));
                 k_tracer_les<<<gt, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], q, dq, zc);
             } else {
