@@ -14,7 +14,8 @@
 //    left-ended forms of a node serve the faces beside it for either sign of the velocity,
 //    so they are formed once per node (10 FP64 instructions) and selected.
 // Written in differences, the value at the face is s*q0 + (weighted sum of differences),
-// which also lets one hardware reciprocal with a cubic correction step replace the division.
+// with a quotient by series (nyles_div.cuh): its divisor is positive, at least 6e-46 and, with differences
+// up to 1e50, within its range.
 // 40 FP64 instructions per vortex-force flux and 39 per tracer flux, where one face at a time
 // (weno5<double>) takes 77. The registers are read and written once per direction for it
 // (33 instead of 12 words per cell), which at 256^3 is 0.7 ms of memory time under 12.6 ms
@@ -23,6 +24,7 @@
 // 109 x 75 x 53 with a tracer and viscosity 2.22 -> 0.71 ms; 256^3 23.4 -> 12.6 ms;
 // 64 x 32 x 32 (16 blocks then) 1.35 -> 0.19 ms.
 #include "nyles_internal.h"
+#include "nyles_div.cuh"
 #include <algorithm>
 
 namespace nyles {
@@ -53,15 +55,6 @@ __device__ __forceinline__ double line_tau(double v) {
     b &= ~0x1fffffffull;
     if ((unsigned int)(b >> 32) >= 0x48100000u) b = 0x7ff0000000000000ull;   // 4 * 2^128
     return __longlong_as_double((long long)b);
-}
-
-// 1/x: the hardware's approximation (relative error e below 2^-20) times 1 + e + e^2
-__device__ __forceinline__ double line_rcp(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double e = fma(-x, y, 1.0);
-    e = fma(e, e, e);
-    return fma(y, e, y);
 }
 
 // the node's indicators from the differences on its left and right: left-ended, centred and
@@ -99,7 +92,7 @@ __device__ __forceinline__ double line_flux(const LineFace& f, double u, double 
     const double g2 = fma(K::g22, f.d2, K::g21 * e1);
     const double g3 = fma(K::g32, f.d2, K::g33 * e3);
     const double num = fma(wc, g3, fma(wb, g2, wa * g1));
-    return fabs(u) * fma(K::s2, qs, num * line_rcp(den));
+    return fabs(u) * fma(K::s2, qs, div_series(num, den));
 }
 
 struct LineTask {
