@@ -105,24 +105,7 @@ __device__ __forceinline__ T mg_resid(const T* __restrict__ x, const T* __restri
     const T dg = T(mg_diag(g, z, y, xx));
     return (b[c] + dg * x[c]) - mg_nsum(x, g, z, y, xx);
 }
-// same with every neighbour inside the level (diag = 6), direct loads
-template <typename T>
-__device__ __forceinline__ T mg_resid_in(const T* __restrict__ x, const T* __restrict__ b, long long c, long long sy,
-                                         long long sz) {
-    return (b[c] + T(6) * x[c]) - (((((x[c - 1] + x[c + 1]) + x[c - sy]) + x[c + sy]) + x[c - sz]) + x[c + sz]);
-}
-
-// ---- per-cell operators with the ghost logic (used at level faces and on the levels
-// held in shared memory by k_mg_bottom)
-// damped Jacobi value at (z, y, x): (1-omega)*in + omega*(sum(in_nb) - b)*idiag
-template <typename T>
-__device__ __forceinline__ T mg_jacobi_cell(const MgGeom& g, const T* __restrict__ in, const T* __restrict__ b, int z,
-                                            int y, int x, T cff1, T omega) {
-    const long long c = mg_at(g, z, y, x);
-    const T idg = mg_idiag<T>(g, mg_diag(g, z, y, x));
-    (void)omega;
-    return cff1 * in[c] + (mg_nsum(in, g, z, y, x) - b[c]) * idg;
-}
+// ---- per-cell operators with the ghost logic (used where a kernel's chunks end)
 // sum of the residuals of the 8 children of coarse cell (z, y, x)
 template <typename T>
 __device__ __forceinline__ T mg_restrict_cell(const MgGeom& gf, const T* __restrict__ xf, const T* __restrict__ bf,
@@ -1425,53 +1408,20 @@ static long long bottom_plan(const int (*n)[3], int nlev, long long solo, int th
 // Deterministic sums: one partial per block of the (x, y, z-chunk) grid, then one
 // block adds the partials in a fixed order.
 
-// MODE 0: sum v^2 ; MODE 1: sum r^2 with r = b + diag*x - sum(x_nb)
-template <typename T, int MODE>
-__global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_sumsq(const MgGeom g, const T* __restrict__ v,
-                                                           const T* __restrict__ b, double* __restrict__ partial,
-                                                           const MgFin fin, double* __restrict__ out) {
+// sum v^2
+__global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_sumsq(const MgGeom g, const double* __restrict__ v,
+                                                           double* __restrict__ partial, const MgFin fin,
+                                                           double* __restrict__ out) {
     const int x = blockIdx.x * MG_BX + threadIdx.x;
     const int y = blockIdx.y * MG_BY + threadIdx.y;
     const int nz = g.n[0], z0 = blockIdx.z * MG_ZC;
     double s = 0.0;
     if (x < g.n[2] && y < g.n[1]) {
-        const long long sy = g.n[2], sz = (long long)g.n[1] * g.n[2];
+        const long long sz = (long long)g.n[1] * g.n[2];
         const long long c0 = mg_at(g, z0, y, x);
-        if (MODE == 0) {
-            for (int z = z0; z < min(z0 + MG_ZC, nz); ++z) {
-                const double r = (double)v[c0 + (z - z0) * sz];
-                s += r * r;
-            }
-        } else {
-            const MgNb nx = mg_nb(x, g.n[2], g.per[2], 1), ny = mg_nb(y, g.n[1], g.per[1], sy);
-            const int dxy = (int)nx.wm + (int)nx.wp + (int)ny.wm + (int)ny.wp;
-            auto res = [&](long long c, T zm, T x0, T zp, T dg) -> T {
-                return (b[c] + dg * x0) - (((((mg_ldw(v, c + nx.om, nx.wm) + mg_ldw(v, c + nx.op, nx.wp)) +
-                                              mg_ldw(v, c + ny.om, ny.wm)) + mg_ldw(v, c + ny.op, ny.wp)) + zm) + zp);
-            };
-            if (z0 + MG_ZC <= nz) {
-                const MgNb lo = mg_nb(z0, nz, g.per[0], sz), hi = mg_nb(z0 + MG_ZC - 1, nz, g.per[0], sz);
-                T col[MG_ZC + 2];
-                col[0] = mg_ldw(v, c0 + lo.om, lo.wm);
-#pragma unroll
-                for (int k = 1; k <= MG_ZC; ++k) col[k] = v[c0 + (k - 1) * sz];
-                col[MG_ZC + 1] = mg_ldw(v, c0 + (MG_ZC - 1) * sz + hi.op, hi.wp);
-                const T d_mid = T(dxy + 2), d_lo = T(dxy + 1 + (int)lo.wm), d_hi = T(dxy + 1 + (int)hi.wp);
-#pragma unroll
-                for (int k = 0; k < MG_ZC; ++k) {
-                    const double r = (double)res(c0 + k * sz, col[k], col[k + 1], col[k + 2],
-                                                 k == 0 ? d_lo : (k == MG_ZC - 1 ? d_hi : d_mid));
-                    s += r * r;
-                }
-            } else {
-                for (int z = z0; z < nz; ++z) {
-                    const long long c = c0 + (z - z0) * sz;
-                    const MgNb nzb = mg_nb(z, nz, g.per[0], sz);
-                    const double r = (double)res(c, mg_ldw(v, c + nzb.om, nzb.wm), v[c], mg_ldw(v, c + nzb.op, nzb.wp),
-                                                 T(dxy + (int)nzb.wm + (int)nzb.wp));
-                    s += r * r;
-                }
-            }
+        for (int z = z0; z < min(z0 + MG_ZC, nz); ++z) {
+            const double r = v[c0 + (z - z0) * sz];
+            s += r * r;
         }
     }
     block_partial(s, partial, blockIdx.z);
@@ -1480,8 +1430,8 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_sumsq(const MgGeom g, cons
 }
 
 // Stop-test residual of the level-1 solution together with the first half-sweep of the
-// next V-cycle: both need the same neighbour sum, so one pass gives sum(r^2) (same
-// partials, same order as k_mg_sumsq MODE 1) and y = (1-omega)*x + omega*(sum - b)*idiag.
+// next V-cycle: both need the same neighbour sum, so one pass gives sum(r^2) (block
+// partials as k_mg_sumsq's) and y = (1-omega)*x + omega*(sum - b)*idiag.
 // If the solve then stops, y is simply not used.
 template <typename T, int ZC = MG_ZC>
 __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_resid_sweep(const MgGeom g, const T* __restrict__ v,
@@ -2773,63 +2723,63 @@ static void smooth(MgImpl* mg, int l, cudaStream_t st, int last_mode, bool from_
             k_mg_jacobi<T, 0, false, 1><<<gs, kBlk, 0, st>>>(g, y, b, x, om, nullptr, nullptr, nullptr, nullptr);
         }
     } else {
-    if (mg->bat.tab) {   // batched (stationary mixed refinement): modes 0 and 1
-        const Bat& bt = mg->bat;
-        float2* pdf = last_mode == 1 ? mg_pdf(mg) : nullptr;
+        if (mg->bat.tab) {   // batched (stationary mixed refinement): modes 0 and 1
+            const Bat& bt = mg->bat;
+            float2* pdf = last_mode == 1 ? mg_pdf(mg) : nullptr;
+            if constexpr (sizeof(T) == sizeof(float)) {
+                const int zc = lvl_zc(mg, l);
+                if (use_v4(mg, g.n, zc)) {
+                    const dim3 gv = bgrid(mg, grid_v4(g.n, zc));
+                    if (!from_y) launch_jacobi_v4_0<true>(zc, gv, st, g, x, b, y, om, bt);
+                    if (last_mode == 1)
+                        launch_jacobi_v4_1<true>(zc, gv, st, g, y, b, x, om, pdf, bt);
+                    else
+                        launch_jacobi_v4_0<true>(zc, gv, st, g, y, b, x, om, bt);
+                    return;
+                }
+            }
+            const dim3 gb = bgrid(mg, grd);
+            if (!from_y) k_mg_jacobi<T, 0, true><<<gb, kBlk, 0, st>>>(g, x, b, y, om, nullptr, nullptr, nullptr, nullptr, bt);
+            if (last_mode == 1)
+                k_mg_jacobi<T, 1, true><<<gb, kBlk, 0, st>>>(g, y, b, x, om, pdf, nullptr, nullptr, nullptr, bt);
+            else
+                k_mg_jacobi<T, 0, true><<<gb, kBlk, 0, st>>>(g, y, b, x, om, nullptr, nullptr, nullptr, nullptr, bt);
+            return;
+        }
         if constexpr (sizeof(T) == sizeof(float)) {
-            const int zc = lvl_zc(mg, l);
-            if (use_v4(mg, g.n, zc)) {
-                const dim3 gv = bgrid(mg, grid_v4(g.n, zc));
-                if (!from_y) launch_jacobi_v4_0<true>(zc, gv, st, g, x, b, y, om, bt);
+            const int zc = last_mode == 2 ? V4_ZC : lvl_zc(mg, l);
+            if (last_mode == 2 ? use_v4_sums(mg) : use_v4(mg, g.n, zc)) {
+                const dim3 gv = grid_v4(g.n, zc);
+                if (!from_y) launch_jacobi_v4_0<false>(zc, gv, st, g, x, b, y, om, Bat());
                 if (last_mode == 1)
-                    launch_jacobi_v4_1<true>(zc, gv, st, g, y, b, x, om, pdf, bt);
+                    launch_jacobi_v4_1<false>(zc, gv, st, g, y, b, x, om, mg_pdf(mg), Bat());
+                else if (last_mode == 2) {   // also beta and the mean of z for the Krylov update
+                    MgFin fin;
+                    fin.ticket = fin_ticket(mg);
+                    fin.sc = reinterpret_cast<double*>(mg->ws + mg->off_scalars);
+                    fin.k = mg->fcg_k;
+                    fin.vol = (double)mg->lev[0].vol;
+                    const float* q = reinterpret_cast<const float*>(mg->ws + mg->off_fq);
+                    double* part = partials(mg, 0, blocks(gv));
+                    double* part2 = partials(mg, 1, blocks(gv));
+                    k_mg_jacobi_v4<2><<<gv, kBlk, 0, st>>>(g, y, b, x, om, nullptr, q, part, part2, Bat(), fin);
+                }
                 else
-                    launch_jacobi_v4_0<true>(zc, gv, st, g, y, b, x, om, bt);
+                    launch_jacobi_v4_0<false>(zc, gv, st, g, y, b, x, om, Bat());
                 return;
             }
         }
-        const dim3 gb = bgrid(mg, grd);
-        if (!from_y) k_mg_jacobi<T, 0, true><<<gb, kBlk, 0, st>>>(g, x, b, y, om, nullptr, nullptr, nullptr, nullptr, bt);
+        if (!from_y) k_mg_jacobi<T, 0><<<grd, kBlk, 0, st>>>(g, x, b, y, om, nullptr, nullptr, nullptr, nullptr);
         if (last_mode == 1)
-            k_mg_jacobi<T, 1, true><<<gb, kBlk, 0, st>>>(g, y, b, x, om, pdf, nullptr, nullptr, nullptr, bt);
+            k_mg_jacobi<T, 1><<<grd, kBlk, 0, st>>>(g, y, b, x, om, mg_pdf(mg),
+                                                    nullptr, nullptr, nullptr);
+        else if (last_mode == 2)
+            k_mg_jacobi<T, 2><<<grd, kBlk, 0, st>>>(g, y, b, x, om, nullptr,
+                                                    reinterpret_cast<const T*>(mg->ws + mg->off_fq),
+                                                    reinterpret_cast<double*>(mg->ws + mg->off_partial),
+                                                    reinterpret_cast<double*>(mg->ws + mg->off_partial2));
         else
-            k_mg_jacobi<T, 0, true><<<gb, kBlk, 0, st>>>(g, y, b, x, om, nullptr, nullptr, nullptr, nullptr, bt);
-        return;
-    }
-    if constexpr (sizeof(T) == sizeof(float)) {
-        const int zc = last_mode == 2 ? V4_ZC : lvl_zc(mg, l);
-        if (last_mode == 2 ? use_v4_sums(mg) : use_v4(mg, g.n, zc)) {
-            const dim3 gv = grid_v4(g.n, zc);
-            if (!from_y) launch_jacobi_v4_0<false>(zc, gv, st, g, x, b, y, om, Bat());
-            if (last_mode == 1)
-                launch_jacobi_v4_1<false>(zc, gv, st, g, y, b, x, om, mg_pdf(mg), Bat());
-            else if (last_mode == 2) {   // also beta and the mean of z for the Krylov update
-                MgFin fin;
-                fin.ticket = fin_ticket(mg);
-                fin.sc = reinterpret_cast<double*>(mg->ws + mg->off_scalars);
-                fin.k = mg->fcg_k;
-                fin.vol = (double)mg->lev[0].vol;
-                const float* q = reinterpret_cast<const float*>(mg->ws + mg->off_fq);
-                double* part = partials(mg, 0, blocks(gv));
-                double* part2 = partials(mg, 1, blocks(gv));
-                k_mg_jacobi_v4<2><<<gv, kBlk, 0, st>>>(g, y, b, x, om, nullptr, q, part, part2, Bat(), fin);
-            }
-            else
-                launch_jacobi_v4_0<false>(zc, gv, st, g, y, b, x, om, Bat());
-            return;
-        }
-    }
-    if (!from_y) k_mg_jacobi<T, 0><<<grd, kBlk, 0, st>>>(g, x, b, y, om, nullptr, nullptr, nullptr, nullptr);
-    if (last_mode == 1)
-        k_mg_jacobi<T, 1><<<grd, kBlk, 0, st>>>(g, y, b, x, om, mg_pdf(mg),
-                                                nullptr, nullptr, nullptr);
-    else if (last_mode == 2)
-        k_mg_jacobi<T, 2><<<grd, kBlk, 0, st>>>(g, y, b, x, om, nullptr,
-                                                reinterpret_cast<const T*>(mg->ws + mg->off_fq),
-                                                reinterpret_cast<double*>(mg->ws + mg->off_partial),
-                                                reinterpret_cast<double*>(mg->ws + mg->off_partial2));
-    else
-        k_mg_jacobi<T, 0><<<grd, kBlk, 0, st>>>(g, y, b, x, om, nullptr, nullptr, nullptr, nullptr);
+            k_mg_jacobi<T, 0><<<grd, kBlk, 0, st>>>(g, y, b, x, om, nullptr, nullptr, nullptr, nullptr);
     }
 }
 
@@ -2972,15 +2922,14 @@ static int read_scalar(MgImpl* mg, double* host_out, cudaStream_t st) {
 
 static double* scalars(MgImpl* mg) { return reinterpret_cast<double*>(mg->ws + mg->off_scalars); }
 
-// enqueue sum(v^2) (MODE 0) or sum(r^2) (MODE 1) of level 1 into *out
-template <typename T, int MODE>
-static void enqueue_sumsq(MgImpl* mg, const MgGeom& g, const T* v, const T* b, double* out, cudaStream_t st) {
+// enqueue sum(v^2) of level 0 into *out
+static void enqueue_sumsq(MgImpl* mg, const MgGeom& g, const double* v, double* out, cudaStream_t st) {
     double* part = reinterpret_cast<double*>(mg->ws + mg->off_partial);
     const dim3 grd = grid_zc(g.n, MG_ZC);
     ProfScope ps(mg->prof, 11, st);
     const bool few = blocks(grd) <= 1024;   // (256^3, 8192 blocks: 74 us with the ticket, 59 + 7 with the sum apart)
     note_launch(few ? 1 : 2);
-    k_mg_sumsq<T, MODE><<<grd, kBlk, 0, st>>>(g, v, b, part, few ? mg_fin(mg) : MgFin(), out);
+    k_mg_sumsq<<<grd, kBlk, 0, st>>>(g, v, part, few ? mg_fin(mg) : MgFin(), out);
     if (!few) k_mg_final<<<1, 1024, 0, st>>>(part, (int)blocks(grd), out);
 }
 
@@ -3095,9 +3044,8 @@ static void enqueue_fcg_update(MgImpl* mg, cudaStream_t st, int k) {
     k_fcg_xupdate<<<eb, 256, 0, st>>>(mg_pdf(mg), P, n, sc);
 }
 
-template <typename T, int MODE>
-static int sumsq(MgImpl* mg, const MgGeom& g, const T* v, const T* b, double* host_out, cudaStream_t st) {
-    enqueue_sumsq<T, MODE>(mg, g, v, b, scalars(mg), st);
+static int sumsq(MgImpl* mg, const MgGeom& g, const double* v, double* host_out, cudaStream_t st) {
+    enqueue_sumsq(mg, g, v, scalars(mg), st);
     return read_scalar(mg, host_out, st);
 }
 
@@ -3145,7 +3093,7 @@ int mg_solve(MgImpl* mg, cudaStream_t st) {
     int rc;
     if (mg->precision == NYLES_FP64) {
         double* b = lvp<double>(mg, 0, 2);
-        if ((rc = sumsq<double, 0>(mg, g0, b, nullptr, &normb, st))) return rc;
+        if ((rc = sumsq(mg, g0, b, &normb, st))) return rc;
         if (!finite_norm(normb)) return blowup(mg, 0, normb, "right-hand side");
         if (normb > 0.0) {
             enqueue_resid_sweep(mg, st);
@@ -3243,7 +3191,7 @@ int mg_solve_graph(MgImpl* mg, GraphBuilder& gb) {
     cudaError_t e = cudaGraphConditionalHandleCreate(&h, gb.graph, 0, 0);
     if (e != cudaSuccess) return gb.error = cuda_status(e, "cudaGraphConditionalHandleCreate");
     if (!mixed) {
-        enqueue_sumsq<double, 0>(mg, g0, lvp<double>(mg, 0, 2), (const double*)nullptr, sc + SC_NORMB, st);
+        enqueue_sumsq(mg, g0, lvp<double>(mg, 0, 2), sc + SC_NORMB, st);
         enqueue_resid_sweep(mg, st);
     } else {
         enqueue_normb_df(mg, st);
