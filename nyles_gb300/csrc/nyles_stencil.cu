@@ -939,48 +939,48 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
         const int line_terms = (tr ? terms & (TERM_TRACER | TERM_TRDIFF) : 0) | (vf && !lin ? TERM_VF : 0);
         return launch_rhs_lines(d, g, s, ds, line_terms, st, interior);
     } else {
-    if (bat.tab) {   // batched: buoyancy advection, WENO vortex force, no buoyancy diffusion
-        if (!(tr && vf && !bdiff && !lin && !linear_tr && d->n_tracers == 0 && d->model != NYLES_MODEL_ADVECTION)) {
-            set_error("batched right-hand side: only buoyancy advection with the WENO vortex force and no tracers");
-            return NYLES_UNSUPPORTED;
-        }
-        const dim3 gb(grd_box.x, grd_box.y, grd_box.z * bat.nrun);
-        if (rhs32_ok<T>(g)) launch_rhs_les<T, true>(gb, blk, st, a, bat);
-        else k_rhs_march<T, true, 1, false, true><<<gb, blk, 0, st>>>(a, bat);
-        note_launch();
-        return cuda_status(cudaGetLastError(), "rhs kernel");
-    }
-    if (lin) {   // the linear vortex force (opt-in)
-        if (tr && bdiff) k_rhs_march<T, true, 2, true><<<grd_box, blk, 0, st>>>(a);
-        else if (tr) k_rhs_march<T, true, 2, false><<<grd_box, blk, 0, st>>>(a);
-        else k_rhs_march<T, false, 2, false><<<grd_box, blk, 0, st>>>(a);
-    } else if (tr && vf && bdiff) k_rhs_march<T, true, 1, true><<<grd_box, blk, 0, st>>>(a);
-    else if (tr && vf && rhs32_ok<T>(g)) launch_rhs_les<T, false>(grd_box, blk, st, a, Bat());
-    else if (tr && vf) k_rhs_march<T, true, 1, false><<<grd_box, blk, 0, st>>>(a);
-    else if (tr && bdiff) k_rhs_march<T, true, 0, true><<<grd_box, blk, 0, st>>>(a);
-    else if (tr) k_rhs_march<T, true, 0, false><<<grd_box, blk, 0, st>>>(a);
-    else if (vf) k_rhs_march<T, false, 1, false><<<grd_box, blk, 0, st>>>(a);
-    else k_rhs_march<T, false, 0, false><<<grd_box, blk, 0, st>>>(a);
-    note_launch();
-    if (linear_tr) {
-        tracer_linear(a.b, a.ds[0], 0);
-        for (int t = 0; t < d->n_tracers; ++t) tracer_linear(a.tr[t], a.ds[4 + t], t + 1);
-        return cuda_status(cudaGetLastError(), "rhs kernel");
-    }
-    for (int t = 0; t < d->n_tracers; ++t) {
-        if (tr) {
-            const T* kc = a.kcoef[t + 1];
-            if ((terms & TERM_TRDIFF) && ((d->tracer_diffusion >> (t + 1)) & 1))
-                k_tracer_march<T, true><<<grd, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], a.tr[t], a.ds[4 + t],
-                                                             kc[0], kc[1], kc[2]);
-            else
-                tracer32(a.tr[t], a.ds[4 + t]);
+        if (bat.tab) {   // batched: buoyancy advection, WENO vortex force, no buoyancy diffusion
+            if (!(tr && vf && !bdiff && !lin && !linear_tr && d->n_tracers == 0 && d->model != NYLES_MODEL_ADVECTION)) {
+                set_error("batched right-hand side: only buoyancy advection with the WENO vortex force and no tracers");
+                return NYLES_UNSUPPORTED;
+            }
+            const dim3 gb(grd_box.x, grd_box.y, grd_box.z * bat.nrun);
+            if (rhs32_ok<T>(g)) launch_rhs_les<T, true>(gb, blk, st, a, bat);
+            else k_rhs_march<T, true, 1, false, true><<<gb, blk, 0, st>>>(a, bat);
             note_launch();
-        } else {   // Euler3d: tracers are not advected, their tendency is zero (reset_state)
-            cudaMemsetAsync(a.ds[4 + t], 0, sizeof(T) * g.vol, st);
+            return cuda_status(cudaGetLastError(), "rhs kernel");
         }
-    }
-    return cuda_status(cudaGetLastError(), "rhs kernel");
+        if (lin) {   // the linear vortex force (opt-in)
+            if (tr && bdiff) k_rhs_march<T, true, 2, true><<<grd_box, blk, 0, st>>>(a);
+            else if (tr) k_rhs_march<T, true, 2, false><<<grd_box, blk, 0, st>>>(a);
+            else k_rhs_march<T, false, 2, false><<<grd_box, blk, 0, st>>>(a);
+        } else if (tr && vf && bdiff) k_rhs_march<T, true, 1, true><<<grd_box, blk, 0, st>>>(a);
+        else if (tr && vf && rhs32_ok<T>(g)) launch_rhs_les<T, false>(grd_box, blk, st, a, Bat());
+        else if (tr && vf) k_rhs_march<T, true, 1, false><<<grd_box, blk, 0, st>>>(a);
+        else if (tr && bdiff) k_rhs_march<T, true, 0, true><<<grd_box, blk, 0, st>>>(a);
+        else if (tr) k_rhs_march<T, true, 0, false><<<grd_box, blk, 0, st>>>(a);
+        else if (vf) k_rhs_march<T, false, 1, false><<<grd_box, blk, 0, st>>>(a);
+        else k_rhs_march<T, false, 0, false><<<grd_box, blk, 0, st>>>(a);
+        note_launch();
+        if (linear_tr) {
+            tracer_linear(a.b, a.ds[0], 0);
+            for (int t = 0; t < d->n_tracers; ++t) tracer_linear(a.tr[t], a.ds[4 + t], t + 1);
+            return cuda_status(cudaGetLastError(), "rhs kernel");
+        }
+        for (int t = 0; t < d->n_tracers; ++t) {
+            if (tr) {
+                const T* kc = a.kcoef[t + 1];
+                if ((terms & TERM_TRDIFF) && ((d->tracer_diffusion >> (t + 1)) & 1))
+                    k_tracer_march<T, true><<<grd, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], a.tr[t], a.ds[4 + t],
+                                                                 kc[0], kc[1], kc[2]);
+                else
+                    tracer32(a.tr[t], a.ds[4 + t]);
+                note_launch();
+            } else {   // Euler3d: tracers are not advected, their tendency is zero (reset_state)
+                cudaMemsetAsync(a.ds[4 + t], 0, sizeof(T) * g.vol, st);
+            }
+        }
+        return cuda_status(cudaGetLastError(), "rhs kernel");
     }
 }
 
