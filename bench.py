@@ -234,39 +234,58 @@ def mg_levels(n):
 RHS_FP64_OPS_PER_CELL = 599
 RHS_FP64_INSTR_PER_CELL = 396
 # DRAM bytes (read + write) per interior cell of one launch: ncu, FP64 at 128^3
-# (48.0 + 133.6 + 146.0 + 143.1 MB), mixed (k_rhs_les) at 256^3 (614.8 + 257.5 MB)
-RHS_DRAM_BYTES_PER_CELL = {8: 470.7e6 / 128 ** 3, 4: 872.35e6 / 256 ** 3}
+# (48.0 + 133.6 + 146.0 + 143.1 MB), mixed (k_rhs_les) at 256^3 (606.0 + 249.8 MB)
+RHS_DRAM_BYTES_PER_CELL = {8: 470.7e6 / 128 ** 3, 4: 855.8e6 / 256 ** 3}
 # DRAM bytes of one level-0 Jacobi half-sweep launch at 256^3, mixed (ncu, vector form:
 # 134.3 + 40.9 MB; algorithmic 201.3 MB, the rest of the output still in L2 at the end)
 JACOBI_F32_L0_DRAM_BYTES_256 = 175.2e6
 
 
-def mg_bottom_level(levels, elem, smem=200 * 1024, maxvol_fp64=1024, cluster=False):
-    """First level of the coarse solve: the coarsest levels whose x, b, y fit in `smem` bytes,
-    two levels at least, never level 0; in FP64 no level above `maxvol_fp64` cells. With `cluster`
-    the library's rule (a cluster of blocks that holds slabs of them): levels of at most 2^15
-    cells in FP32, 2^12 in FP64; the slabs fit whenever the cells do."""
+def mg_bottom_level(levels, elem, smem=200 * 1024, maxvol_fp64=1024):
+    """First level of a coarse solve in one block (as the multigrid had before mg_cluster_level's): the
+    coarsest levels whose x, b, y fit in `smem` bytes, two levels at least, never level 0; in FP64 no level above
+    `maxvol_fp64` cells."""
     L = len(levels)
     bottom, total = L, 0
     for l in range(L - 1, 0, -1):
         z, y, x = levels[l]
-        if cluster:
-            if z * y * x > (1 << 15 if elem == 4 else 1 << 12):
-                break
-        else:
-            total += 3 * z * y * x * elem
-            if total > smem:
-                break
-            if elem == 8 and z * y * x > maxvol_fp64:
-                break
+        total += 3 * z * y * x * elem
+        if total > smem:
+            break
+        if elem == 8 and z * y * x > maxvol_fp64:
+            break
         if L - l >= 2:
             bottom = l
     return bottom
 
 
+def mg_cluster_level(levels, elem, smem=200 * 1024, ctas=8):
+    """First level of the library's coarse solve in a cluster of `ctas` blocks (mg_init and bottom_plan in nyles_mg.cu):
+    levels of at most 2^15 cells in FP32 and 2^12 in FP64, two at least, never level 0, while a block's slabs fit in
+    `smem` bytes. A level of more than `solo` cells and at least 4 planes is cut into an even number of planes per block,
+    and the level under it while half of them is even; x, y and b carry a ring of ghost cells."""
+    solo, most = (1024, 1 << 15) if elem == 4 else (256, 1 << 12)
+    L = len(levels)
+    bottom = L
+    for first in range(L - 2, 0, -1):
+        if levels[first][0] * levels[first][1] * levels[first][2] > most:
+            break
+        cells, half = 0, 0
+        for k, (z, y, x) in enumerate(levels[first:]):
+            cut = z * y * x > solo and z >= 4 and (k == 0 or (half and half % 2 == 0))
+            planes = z if not cut else (2 * -(-z // (2 * ctas)) if k == 0 else half)
+            half = planes // 2 if planes < z else 0
+            cells += 3 * (planes + 2) * (y + 2) * (x + 2)
+        if cells * elem > smem:
+            break
+        bottom = first
+    return bottom
+
+
 def roofline(kernel, ph, n, elem, peak, peak_kind, fp64_peak, nv=None, solves=None, krylov=False,
              cluster=False):
-    """Roofline of one kernel family from the CUDA-event phase times (cluster: see mg_bottom_level).
+    """Roofline of one kernel family from the CUDA-event phase times (cluster: the coarse
+    levels of mg_cluster_level, else of mg_bottom_level).
 
     rhs       : one launch reads b, U(3), vor(3), ke and writes 4 registers: 12 words
                 per interior cell (the periodic halo's tendencies are not computed). In FP64 the kernel is bound by the FP64
@@ -312,7 +331,7 @@ def roofline(kernel, ph, n, elem, peak, peak_kind, fp64_peak, nv=None, solves=No
         out.update({k: v for k, v in hbm.items() if k not in ("peak", "unit", "peak_kind", "frac")})
     elif kernel == "mg_smooth":
         lev = mg_levels(n)
-        B = mg_bottom_level(lev, elem, cluster=cluster)
+        B = (mg_cluster_level if cluster else mg_bottom_level)(lev, elem)
         vol = [z * y * x for (z, y, x) in lev]
         per_vcycle = sum((4 if (l == 0 and elem == 8) else 3) * 3 * elem * vol[l] for l in range(B))
         if elem == 4:
