@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, RhsMinBlocks<T>::n) k_rhs_march
 //    along z instead of two more loads;
 //  - within three cells of an array end, where flux1d_at takes a closure branch, the
 //    reconstruction falls back to flux1d_at.
-// Bound by instruction issue (64% of cycles). Measured against 64-bit index arithmetic per load:
+// Bound by instruction issue (70% of cycles). Measured against 64-bit index arithmetic per load:
 // 301 x 203 x 97 371 -> 335 us, 512 x 256 x 256 1433 -> 1320 us; a passive tracer there 907 -> 612 us against
 // k_tracer_march. The reconstructions written in differences (as in nyles_line.cu) took 328, 1289 and 520 us,
 // but round anew what smooth fields leave ill-conditioned: the weights of isolated cells (1e-3 of a small
@@ -1589,7 +1589,7 @@ __global__ void __launch_bounds__(256) k_max_U2f(const long long vol, const floa
                     const double s = sum_U2(a[k], b[k], c[k]);
                     if (s != s) any_nan = true;
                     m = fmax(m, s);
-                    top = fmaxf(top, fminf(f[k], 3.4e38f));   // (a NaN leaves top, an infinity stays above skip)
+                    top = fmaxf(top, fminf(f[k], 3.4e38f));   // (NaN, infinity: 3.4e38, and any_nan or m says the rest)
                 }
             }
             top = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(top)));   // (not negative)
