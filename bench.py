@@ -341,7 +341,8 @@ def roofline(kernel, ph, n, elem, peak, peak_kind, fp64_peak, nv=None, solves=No
         calls_per_vcycle = 2 * B + 1   # one bracketed call per smoothing and the coarse solve
         vcycles = ph[kernel]["count"] / calls_per_vcycle
         total = per_vcycle * vcycles
-        out.update({"kernel": "k_mg_jacobi (+ k_mg_bottom)", "bytes_per_vcycle": per_vcycle, "vcycles": vcycles,
+        out.update({"kernel": "k_mg_jacobi (+ k_mg_bottom)" if elem == 4 else "k_mg_fx, k_mg_jacobi (+ k_mg_bottom)",
+                    "bytes_per_vcycle": per_vcycle, "vcycles": vcycles,
                     "ms_per_vcycle": ms / vcycles, "achieved": total / (ms * 1e-3) / 1e9})
         if elem == 4 and n == 256:
             out["traffic"] = JACOBI_F32_L0_DRAM_BYTES_256

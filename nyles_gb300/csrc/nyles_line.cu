@@ -21,7 +21,7 @@
 // (33 instead of 12 words per cell), which at 256^3 is 0.7 ms of memory time under 12.6 ms
 // of FP64 time.
 // Measured against the march that formed every face on its own in 16-cell columns:
-// 109 x 75 x 53 with a tracer and viscosity 2.22 -> 0.71 ms; 256^3 23.4 -> 12.6 ms;
+// 109 x 75 x 53 with a tracer and viscosity 2.22 -> 0.60 ms; 256^3 23.4 -> 12.6 ms;
 // 64 x 32 x 32 (16 blocks then) 1.35 -> 0.19 ms.
 #include "nyles_internal.h"
 #include "nyles_div.cuh"

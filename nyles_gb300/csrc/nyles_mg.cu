@@ -1486,11 +1486,12 @@ __global__ void __launch_bounds__(MG_BX * MG_BY) k_mg_resid_sweep(const MgGeom g
 // What the V-cycle does to a level is a sum over a cell and its neighbours: a half-sweep is
 // (1-omega) x + (omega/diag) (sum(x_nb) - b), the stop test and the restriction need the residual
 // r = b + diag*x - sum(x_nb). In doubles the sum is 6 FP64 instructions of a half-sweep's 8, at
-// 2 lanes per cycle and SM; here it is a sum of 64-bit integers (nyles_fx.cuh), about 110 integer
-// instructions per cell with the conversions, and 2 FP64 instructions are left. Bound by the integer
-// pipe (64% busy; FP64 26%, memory 25%). Measured against the double kernels (k_mg_jacobi,
+// 2 lanes per cycle and SM; here it is a sum of 64-bit integers (nyles_fx.cuh), about 130 instructions per cell
+// with the conversions and the range tests, and 2 FP64 instructions are left. Bound by the integer
+// pipe (62% busy; memory 25%). Measured against the double kernels (k_mg_jacobi,
 // k_mg_resid_sweep, k_mg_restrict in 8-cell columns) per launch: 128^3 38 -> 17, 44 -> 20 and
-// 37 -> 17 us; 256^3 step with the transfer below 142 -> 85.4 ms.
+// 37 -> 17 us (20 and 23 in a Taylor-Green step, some of whose sums are redone in doubles); 256^3 half-sweep 245 -> 95 us,
+// step with the transfer below 142 -> 86.1 ms.
 // A block owns 32 x 8 columns of ZC cells, one column per thread: every value of the tile
 // and of the ring around it is loaded first, the block agrees on the exponent, and the
 // converted columns meet in shared memory. Ghosts: 0 across a wall, else the periodic image.
