@@ -25,7 +25,8 @@ __device__ __forceinline__ unsigned int fx_mag(double x) { return (unsigned int)
 
 // x in units of 2^(E-1081) (truncated below), |x| < 2^(E-1022): at most 59 bits. What the
 // truncation takes from the x of a residual it takes from the centre's and the neighbours'
-// terms alike.
+// terms alike: rounded instead (fx_round), three cases in three seeds each were as far from 64 bits
+// (256^3 Rayleigh-Taylor 1.3e-13, 1.6e-13 and 1.8e-13 both ways) and 1.2 to 1.6% slower.
 __device__ __forceinline__ long long fx_from(double x, int E) {
     const unsigned int hi = (unsigned int)__double2hiint(x), lo = (unsigned int)__double2loint(x);
     const unsigned int e = (hi >> 20) & 0x7ffu;
