@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, RhsMinBlocks<T>::n) k_rhs_march
 
 // ---------------------------------------------------------------- right-hand side, 32-bit offsets
 // k_rhs_march<float, true, 1, false> (buoyancy advection, WENO vortex force, Bernoulli,
-// viscosity) where a block's reach fits 32-bit byte offsets (rhs32_chunk): the same operations in the same order
+// viscosity) where a block's reach fits 32-bit offsets (rhs32_form): the same operations in the same order
 // outside the reconstructions, with fewer instructions per cell:
 //  - 32-bit offsets from a block's own pointers; the six values around a face are loaded at
 //    offsets shared by every field read along that direction;
@@ -423,35 +423,44 @@ struct LineOff {
         for (int k = 0; k < 7; ++k) o[k] = c + (unsigned int)(k - 3) * s;
     }
 };
+// UNIT 4: offsets in bytes. UNIT 1: in cells, widened at each load, for planes whose reach in bytes leaves 32 bits.
+template <int UNIT>
+__device__ __forceinline__ const float* pto(const char* __restrict__ f, unsigned int off) {
+    return UNIT == 4 ? reinterpret_cast<const float*>(f + off) : reinterpret_cast<const float*>(f) + off;
+}
+template <int UNIT>
 __device__ __forceinline__ float ldo(const char* __restrict__ f, unsigned int off) {
-    return __ldg(reinterpret_cast<const float*>(f + off));
+    return __ldg(pto<UNIT>(f, off));
 }
 // flux of a tracer at index i of a line (flux1d_at of tr_flux), and of the vortex force given its
 // velocity (vf_flux); `fast`: i lies where flux1d_at takes its interior branch
+template <int UNIT>
 __device__ __forceinline__ float tr_flux32(const char* __restrict__ f, float u, const LineOff& l, int i, int n, int s,
                                            bool fast) {
     if (fast) {
         float v[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = ldo(f, l.o[k + 1]);
+        for (int k = 0; k < 6; ++k) v[k] = ldo<UNIT>(f, l.o[k + 1]);
         return weno5_upwind(u, v);
     }
-    return tr_flux_closure(reinterpret_cast<const float*>(f + l.o[3]), u, i, n, s);
+    return tr_flux_closure(pto<UNIT>(f, l.o[3]), u, i, n, s);
 }
+template <int UNIT>
 __device__ __forceinline__ float2 vf_flux32_x2(const char* __restrict__ fa, const char* __restrict__ fb, float2 u,
                                                const LineOff& l, int i, int n, int s, bool fast) {
     if (fast) {
         float2 v[6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) v[k] = make_float2(ldo(fa, l.o[k]), ldo(fb, l.o[k]));
+        for (int k = 0; k < 6; ++k) v[k] = make_float2(ldo<UNIT>(fa, l.o[k]), ldo<UNIT>(fb, l.o[k]));
         return weno5_upwind_x2(u, v);
     }
-    return make_float2(vf_flux_closure(reinterpret_cast<const float*>(fa + l.o[3]), u.x, i, n, s),
-                       vf_flux_closure(reinterpret_cast<const float*>(fb + l.o[3]), u.y, i, n, s));
+    return make_float2(vf_flux_closure(pto<UNIT>(fa, l.o[3]), u.x, i, n, s),
+                       vf_flux_closure(pto<UNIT>(fb, l.o[3]), u.y, i, n, s));
 }
 
 // One tracer in a block of RZ_BX x RZ_BY columns: -(flux divergence), summed as TracerMarch::step
 // (x, y, z), with the faces shared as there
+template <int UNIT>
 struct TracerMarch32 {
     float fz_prev;
     // u*: the velocity along each axis at the cell; every thread of the block must call it
@@ -460,18 +469,18 @@ struct TracerMarch32 {
                                           const LineOff& ly, const LineOff& lz, int z, int ys, int xs, int sy, int sz,
                                           int Nz, int Ny, int Nx, float (*sfy)[RZ_BX]) {
         const int tx = threadIdx.x, ty = threadIdx.y;
-        const float fz = tr_flux32(f, u2, lz, z, Nz, sz, z >= 2 && z <= Nz - 4);
-        const float fy = tr_flux32(f, u1, ly, ys, Ny, sy, ys >= 2 && ys <= Ny - 4);
+        const float fz = tr_flux32<UNIT>(f, u2, lz, z, Nz, sz, z >= 2 && z <= Nz - 4);
+        const float fy = tr_flux32<UNIT>(f, u1, ly, ys, Ny, sy, ys >= 2 && ys <= Ny - 4);
         sfy[ty][tx] = fy;
         __syncthreads();
         float fym = (ty > 0) ? sfy[ty - 1][tx] : 0.f;
         __syncthreads();
         if (ty == 0 && ys > 0)   // the face below the block's first row
-            fym = tr_flux32(f, ldo(fU1, ly.o[2]), LineOff(ly.o[2], sy * 4u), ys - 1, Ny, sy, ys - 1 >= 2 && ys - 1 <= Ny - 4);
-        const float fx = tr_flux32(f, u0, lx, xs, Nx, 1, xs >= 2 && xs <= Nx - 4);
+            fym = tr_flux32<UNIT>(f, ldo<UNIT>(fU1, ly.o[2]), LineOff(ly.o[2], sy * (unsigned int)UNIT), ys - 1, Ny, sy, ys - 1 >= 2 && ys - 1 <= Ny - 4);
+        const float fx = tr_flux32<UNIT>(f, u0, lx, xs, Nx, 1, xs >= 2 && xs <= Nx - 4);
         float fxm = __shfl_up_sync(0xffffffffu, fx, 1);
         if (tx == 0 && xs > 0)
-            fxm = tr_flux32(f, ldo(fU0, lx.o[2]), LineOff(lx.o[2], 4u), xs - 1, Nx, 1, xs - 1 >= 2 && xs - 1 <= Nx - 4);
+            fxm = tr_flux32<UNIT>(f, ldo<UNIT>(fU0, lx.o[2]), LineOff(lx.o[2], UNIT), xs - 1, Nx, 1, xs - 1 >= 2 && xs - 1 <= Nx - 4);
         float db = (xs > 0) ? (0.f + fxm) - fx : 0.f - fx;
         db = (ys > 0) ? (db + fym) - fy : db - fy;
         db = (z > 0) ? (db + fz_prev) - fz : db - fz;
@@ -482,6 +491,7 @@ struct TracerMarch32 {
 
 // a block's columns: thread positions, the byte offset of a thread's cell at plane z0, and the
 // distance from a field's start to the point the offsets count from
+template <int UNIT>
 struct Block32 {
     int x, y, xs, ys, z0, z1;
     unsigned int c0;
@@ -497,7 +507,7 @@ struct Block32 {
         // bx, by may lie beyond hi by less than a block: count from the shadowed cells' side
         const int ox = min(bx, hi[2] - 1) - 3, oy = min(by, hi[1] - 1) - 3, oz = z0 - 3;
         org = 4ll * ((long long)oz * sz + (long long)oy * sy + ox);
-        c0 = 4u * (3u * (unsigned int)sz + (unsigned int)(ys - oy) * (unsigned int)sy + (unsigned int)(xs - ox));
+        c0 = (unsigned int)UNIT * (3u * (unsigned int)sz + (unsigned int)(ys - oy) * (unsigned int)sy + (unsigned int)(xs - ox));
     }
 };
 
@@ -505,7 +515,7 @@ struct Block32 {
 // of line; inlined, they took it to 64)
 template <typename T> struct LesMinBlocks { static constexpr int n = 5; };
 
-template <typename T, bool BAT>
+template <typename T, bool BAT, int UNIT>
 __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(const RhsArgs<T> a0, const int zc,
                                                                              const Bat bat = Bat()) {
     __shared__ T sfy[RZ_BY][RZ_BX];
@@ -518,7 +528,7 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(c
     }
     const int Nz = a.g.N[0], Ny = a.g.N[1], Nx = a.g.N[2];
     const int sy = (int)a.g.sy, sz = (int)a.g.sz;
-    const Block32 k(a.lo, a.hi, bz, zc, sy, sz);
+    const Block32<UNIT> k(a.lo, a.hi, bz, zc, sy, sz);
     const int xs = k.xs, ys = k.ys, tx = threadIdx.x;
     const bool valid = k.x < a.hi[2] && k.y < a.hi[1];
     auto fld = [&](const T* p) { return reinterpret_cast<const char*>(p) + k.org; };
@@ -530,47 +540,47 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(c
     const char* __restrict__ W1 = fld(a.W[1]);
     const char* __restrict__ W2 = fld(a.W[2]);
     const char* __restrict__ ke = fld(a.ke);
-    const unsigned int by = 4u * (unsigned int)sy, bzs = 4u * (unsigned int)sz;
+    const unsigned int bx = UNIT, by = UNIT * (unsigned int)sy, bzs = UNIT * (unsigned int)sz;
     // interior vortex-force reconstructions: 3 <= i <= n - 4
     const bool xv = xs >= 3 && xs <= Nx - 4, yv = ys >= 3 && ys <= Ny - 4;
     const bool ylo = ys < Ny - 1, xlo = xs < Nx - 1;
     // carried up the column: the tracer flux through the face below the cell and the
     // two z-fluxes' velocities averaged at that face
-    TracerMarch32 tm;
+    TracerMarch32<UNIT> tm;
     tm.fz_prev = 0.f;
     T uu_zy = T(0), uu_zx = T(0);
     if (k.z0 > 0) {
         const int zm = k.z0 - 1;
         const LineOff lz(k.c0 - bzs, bzs);
-        const T u = ldo(U2, lz.o[3]);
-        tm.fz_prev = tr_flux32(b, u, lz, zm, Nz, sz, zm >= 2 && zm <= Nz - 4);
-        if (ylo) uu_zy = T(0.5) * (u + ldo(U2, lz.o[3] + by));
-        if (xlo) uu_zx = T(0.5) * (u + ldo(U2, lz.o[3] + 4u));
+        const T u = ldo<UNIT>(U2, lz.o[3]);
+        tm.fz_prev = tr_flux32<UNIT>(b, u, lz, zm, Nz, sz, zm >= 2 && zm <= Nz - 4);
+        if (ylo) uu_zy = T(0.5) * (u + ldo<UNIT>(U2, lz.o[3] + by));
+        if (xlo) uu_zx = T(0.5) * (u + ldo<UNIT>(U2, lz.o[3] + bx));
     }
     unsigned int c = k.c0;
     for (int z = k.z0; z < k.z1; ++z, c += bzs) {
         const bool zv = z >= 3 && z <= Nz - 4, zlo = z < Nz - 1;
-        const T u0 = ldo(U0, c), u1 = ldo(U1, c), u2 = ldo(U2, c);
+        const T u0 = ldo<UNIT>(U0, c), u1 = ldo<UNIT>(U1, c), u2 = ldo<UNIT>(U2, c);
         // The vortex-force fluxes are formed direction by direction (one set of offsets live at a
         // time) and summed afterwards in the order of vortex_force_cell.
         T f1 = T(0), f2 = T(0), f3 = T(0), f4 = T(0), f5 = T(0), f6 = T(0);
-        const LineOff lz(c, bzs), ly(c, by), lx(c, 4u);
+        const LineOff lz(c, bzs), ly(c, by), lx(c, bx);
         // f4 (ylo): u_j += U^k w_i along k (U^k averaged along j); f5 (xlo): u_i -= U^k w_j along
         // k (U^k averaged along i)
         {
             float2 u = make_float2(0.f, 0.f);
             if (ylo) {
-                const T uu1 = T(0.5) * (u2 + ldo(U2, c + by)), uu0 = z > 0 ? uu_zy : T(0);
+                const T uu1 = T(0.5) * (u2 + ldo<UNIT>(U2, c + by)), uu0 = z > 0 ? uu_zy : T(0);
                 uu_zy = uu1;
                 u.x = T(0.5) * (uu0 + uu1);
             }
             if (xlo) {
-                const T uu1 = T(0.5) * (u2 + ldo(U2, c + 4u)), uu0 = z > 0 ? uu_zx : T(0);
+                const T uu1 = T(0.5) * (u2 + ldo<UNIT>(U2, c + bx)), uu0 = z > 0 ? uu_zx : T(0);
                 uu_zx = uu1;
                 u.y = T(0.5) * (uu0 + uu1);
             }
             if (ylo || xlo) {
-                const float2 f = vf_flux32_x2(W0, W1, u, lz, z, Nz, sz, zv);
+                const float2 f = vf_flux32_x2<UNIT>(W0, W1, u, lz, z, Nz, sz, zv);
                 f4 = f.x;
                 f5 = f.y;
             }
@@ -580,17 +590,17 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(c
         {
             float2 u = make_float2(0.f, 0.f);
             if (xlo) {
-                const T uu1 = T(0.5) * (u1 + ldo(U1, c + 4u));
-                const T uu0 = ys > 0 ? T(0.5) * (ldo(U1, c - by) + ldo(U1, c - by + 4u)) : T(0);
+                const T uu1 = T(0.5) * (u1 + ldo<UNIT>(U1, c + bx));
+                const T uu0 = ys > 0 ? T(0.5) * (ldo<UNIT>(U1, c - by) + ldo<UNIT>(U1, c - by + bx)) : T(0);
                 u.x = T(0.5) * (uu0 + uu1);
             }
             if (zlo) {
-                const T uu1 = T(0.5) * (u1 + ldo(U1, c + bzs));
-                const T uu0 = ys > 0 ? T(0.5) * (ldo(U1, c - by) + ldo(U1, c - by + bzs)) : T(0);
+                const T uu1 = T(0.5) * (u1 + ldo<UNIT>(U1, c + bzs));
+                const T uu0 = ys > 0 ? T(0.5) * (ldo<UNIT>(U1, c - by) + ldo<UNIT>(U1, c - by + bzs)) : T(0);
                 u.y = T(0.5) * (uu0 + uu1);
             }
             if (xlo || zlo) {
-                const float2 f = vf_flux32_x2(W2, W0, u, ly, ys, Ny, sy, yv);
+                const float2 f = vf_flux32_x2<UNIT>(W2, W0, u, ly, ys, Ny, sy, yv);
                 f2 = f.x;
                 f3 = f.y;
             }
@@ -598,19 +608,19 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(c
         // f1 (ylo): u_j -= U^i w_k along i (U^i averaged along j); f6 (zlo): u_k += U^i w_j along
         // i (U^i averaged along k)
         {
-            const T uy = ylo ? T(0.5) * (u0 + ldo(U0, c + by)) : T(0), uz = zlo ? T(0.5) * (u0 + ldo(U0, c + bzs)) : T(0);
+            const T uy = ylo ? T(0.5) * (u0 + ldo<UNIT>(U0, c + by)) : T(0), uz = zlo ? T(0.5) * (u0 + ldo<UNIT>(U0, c + bzs)) : T(0);
             T my = __shfl_up_sync(0xffffffffu, uy, 1), mz = __shfl_up_sync(0xffffffffu, uz, 1);
             if (tx == 0) {
                 my = mz = T(0);
                 if (xs > 0) {
-                    const T um = ldo(U0, c - 4u);
-                    if (ylo) my = T(0.5) * (um + ldo(U0, c - 4u + by));
-                    if (zlo) mz = T(0.5) * (um + ldo(U0, c - 4u + bzs));
+                    const T um = ldo<UNIT>(U0, c - bx);
+                    if (ylo) my = T(0.5) * (um + ldo<UNIT>(U0, c - bx + by));
+                    if (zlo) mz = T(0.5) * (um + ldo<UNIT>(U0, c - bx + bzs));
                 }
             }
             if (ylo || zlo) {
                 const float2 u = make_float2(ylo ? T(0.5) * (my + uy) : T(0), zlo ? T(0.5) * (mz + uz) : T(0));
-                const float2 f = vf_flux32_x2(W2, W1, u, lx, xs, Nx, 1, xv);
+                const float2 f = vf_flux32_x2<UNIT>(W2, W1, u, lx, xs, Nx, 1, xv);
                 f1 = f.x;
                 f6 = f.y;
             }
@@ -625,12 +635,12 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(c
         if (xlo) dux = dux - f5;
         if (zlo) duz = duz + f6;
         // ---- Bernoulli (core/bernoulli.py:14-23)
-        const T k0 = ldo(ke, c);
-        if (xlo) dux = sub_rn(dux, sub_rn(ldo(ke, c + 4u), k0));
-        if (ylo) duy = sub_rn(duy, sub_rn(ldo(ke, c + by), k0));
+        const T k0 = ldo<UNIT>(ke, c);
+        if (xlo) dux = sub_rn(dux, sub_rn(ldo<UNIT>(ke, c + bx), k0));
+        if (ylo) duy = sub_rn(duy, sub_rn(ldo<UNIT>(ke, c + by), k0));
         if (zlo) {
-            duz = sub_rn(duz, sub_rn(ldo(ke, c + bzs), k0));
-            if (!a.euler) duz = add_rn(duz, mul_rn(a.half_dz, add_rn(ldo(b, c + bzs), ldo(b, c))));
+            duz = sub_rn(duz, sub_rn(ldo<UNIT>(ke, c + bzs), k0));
+            if (!a.euler) duz = add_rn(duz, mul_rn(a.half_dz, add_rn(ldo<UNIT>(b, c + bzs), ldo<UNIT>(b, c))));
         }
         const long long cl = ((long long)z * sz + (long long)ys * sy) + xs;
         if (a.terms & TERM_VISC) {
@@ -653,27 +663,28 @@ __global__ void __launch_bounds__(RZ_BX * RZ_BY, LesMinBlocks<T>::n) k_rhs_les(c
 }
 
 // the same for one passive tracer over the whole arrays (core/tracer.py:59-72)
+template <int UNIT>
 __global__ void __launch_bounds__(RZ_BX * RZ_BY, 5) k_tracer_les(const Geom g, const float* __restrict__ Ux,
                                                                const float* __restrict__ Uy, const float* __restrict__ Uz,
                                                                const float* __restrict__ q, float* __restrict__ dq,
                                                                const int zc) {
     __shared__ float sfy[RZ_BY][RZ_BX];
     const int sy = (int)g.sy, sz = (int)g.sz, lo[3] = {0, 0, 0};
-    const Block32 k(lo, g.N, blockIdx.z, zc, sy, sz);
+    const Block32<UNIT> k(lo, g.N, blockIdx.z, zc, sy, sz);
     const bool valid = k.x < g.N[2] && k.y < g.N[1];
     auto fld = [&](const float* p) { return reinterpret_cast<const char*>(p) + k.org; };
     const char *U0 = fld(Ux), *U1 = fld(Uy), *U2 = fld(Uz), *f = fld(q);
-    const unsigned int by = 4u * (unsigned int)sy, bzs = 4u * (unsigned int)sz;
-    TracerMarch32 tm;
+    const unsigned int bx = UNIT, by = UNIT * (unsigned int)sy, bzs = UNIT * (unsigned int)sz;
+    TracerMarch32<UNIT> tm;
     tm.fz_prev = 0.f;
     if (k.z0 > 0) {
         const int zm = k.z0 - 1;
         const LineOff lz(k.c0 - bzs, bzs);
-        tm.fz_prev = tr_flux32(f, ldo(U2, lz.o[3]), lz, zm, g.N[0], sz, zm >= 2 && zm <= g.N[0] - 4);
+        tm.fz_prev = tr_flux32<UNIT>(f, ldo<UNIT>(U2, lz.o[3]), lz, zm, g.N[0], sz, zm >= 2 && zm <= g.N[0] - 4);
     }
     unsigned int c = k.c0;
     for (int z = k.z0; z < k.z1; ++z, c += bzs) {
-        const float v = tm.step(f, U0, U1, ldo(U0, c), ldo(U1, c), ldo(U2, c), LineOff(c, 4u), LineOff(c, by),
+        const float v = tm.step(f, U0, U1, ldo<UNIT>(U0, c), ldo<UNIT>(U1, c), ldo<UNIT>(U2, c), LineOff(c, bx), LineOff(c, by),
                                 LineOff(c, bzs), z, k.ys, k.xs, sy, sz, g.N[0], g.N[1], g.N[2], sfy);
         if (valid) dq[g.at(z, k.ys, k.xs)] = v;
     }
@@ -769,28 +780,37 @@ __global__ void __launch_bounds__(256) k_tracer_linear(const Geom g, const T* __
     dq[c] = acc;
 }
 
-// k_rhs_les and k_tracer_les serve FP32 arrays whose 7 planes (the reach of a block of one plane) lie within 4 GB;
-// NYLES_GB300_GENERIC_RHS=1 selects k_rhs_march instead (values equal to rounding).
-static bool rhs32_reach(const Geom& g, int zc) { return 4 * ((zc + 6) * g.sz + 16 * g.sy + 64) < (1ll << 32); }
+// k_rhs_les and k_tracer_les serve FP32 arrays whose 7 planes (the reach of a block of one plane) hold fewer than 2^32
+// cells; NYLES_GB300_GENERIC_RHS=1 selects k_rhs_march instead (values equal to rounding).
+static bool rhs32_reach(const Geom& g, int zc, int unit) {
+    return unit * ((zc + 6) * g.sz + 16 * g.sy + 64) < (1ll << 32);
+}
 // Planes per thread of the FP32 marches: 16 where that gives every SM its five blocks, fewer on small
 // grids (each thread starts with the flux below its first plane, a tenth of a plane's work): 16 / 2
-// planes of a 48^3 right-hand side (36 / 288 blocks) 118 / 21 us; fewer too where a block's planes would lie
-// beyond 4 GB, from 48.8 M cells per plane on (8200 x 6144 x 11 with a tracer 53.9 ms on the general march, 34.0 with 8
-// planes; 16400 x 8640 x 5 69.0, 59.2 with one).
-static int rhs32_chunk(const Geom& g, long long columns, int nz) {
+// planes of a 48^3 right-hand side (36 / 288 blocks) 118 / 21 us. The offsets' unit: bytes where a block's planes
+// lie within 4 GB (up to 48.8 M cells per plane with 16), else cells, which cost a widening per load (343 us against 330
+// on 301 x 203 x 97) but keep the planes: 6144 x 8200 x 11 with a tracer 34.1 ms in bytes with 8 planes, 33.6 in cells;
+// 6144 x 16400 x 10, 4 planes, 64.6 / 61.2; 8640 x 16400 x 5, one plane, 59.2 / 44.3; 12800^2 x 5 51.4 in cells (79.8 in
+// k_rhs_march), 16000^2 x 5 80.4 (124.8).
+struct Rhs32Form {
+    int zc, unit;
+};
+static Rhs32Form rhs32_form(const Geom& g, long long columns, int nz) {
     int zc = 16;
     while (zc > 2 && columns * ((nz + zc - 1) / zc) < 152 * 5) zc /= 2;
-    while (zc > 1 && !rhs32_reach(g, zc)) zc /= 2;
-    return zc;
+    const int unit = rhs32_reach(g, zc, 4) ? 4 : 1;
+    while (zc > 1 && !rhs32_reach(g, zc, unit)) zc /= 2;
+    return {zc, unit};
 }
 
 template <typename T, bool BAT>
 static void launch_rhs_les(dim3 grd, dim3 blk, cudaStream_t st, const RhsArgs<T>& a, const Bat& bat) {
     if constexpr (sizeof(T) == sizeof(float)) {
         const int nz = a.hi[0] - a.lo[0], nrun = BAT ? bat.nrun : 1;
-        const int zc = rhs32_chunk(a.g, (long long)grd.x * grd.y * nrun, nz);
-        grd.z = (unsigned)((nz + zc - 1) / zc * nrun);
-        k_rhs_les<T, BAT><<<grd, blk, 0, st>>>(a, zc, bat);
+        const Rhs32Form f = rhs32_form(a.g, (long long)grd.x * grd.y * nrun, nz);
+        grd.z = (unsigned)((nz + f.zc - 1) / f.zc * nrun);
+        if (f.unit == 4) k_rhs_les<T, BAT, 4><<<grd, blk, 0, st>>>(a, f.zc, bat);
+        else k_rhs_les<T, BAT, 1><<<grd, blk, 0, st>>>(a, f.zc, bat);
     }
 }
 
@@ -801,7 +821,7 @@ static bool rhs32_ok(const Geom& g) {
         const char* e = getenv("NYLES_GB300_GENERIC_RHS");
         return e && e[0] == '1';
     }();
-    return !generic && rhs32_reach(g, 1);
+    return !generic && rhs32_reach(g, 1, 1);
 }
 
 bool make_geom(const NylesDesc* d, Geom* g) {
@@ -887,9 +907,10 @@ int launch_rhs(const NylesDesc* d, const Geom& g, const StencilPtrs<T>& s, const
     auto tracer32 = [&](const T* q, T* dq) {   // FP32, no diffusion
         if constexpr (sizeof(T) == sizeof(float)) {
             if (rhs32_ok<T>(g)) {
-                const int zc = rhs32_chunk(g, (long long)grd.x * grd.y, g.N[0]);
-                const dim3 gt(grd.x, grd.y, (unsigned)((g.N[0] + zc - 1) / zc));
-                k_tracer_les<<<gt, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], q, dq, zc);
+                const Rhs32Form f = rhs32_form(g, (long long)grd.x * grd.y, g.N[0]);
+                const dim3 gt(grd.x, grd.y, (unsigned)((g.N[0] + f.zc - 1) / f.zc));
+                if (f.unit == 4) k_tracer_les<4><<<gt, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], q, dq, f.zc);
+                else k_tracer_les<1><<<gt, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], q, dq, f.zc);
             } else {
                 k_tracer_march<T, false><<<grd, blk, 0, st>>>(g, a.U[0], a.U[1], a.U[2], q, dq, T(0), T(0), T(0));
             }

@@ -1,6 +1,6 @@
-"""The FP32 right-hand side on planes so large that a block's columns are cut shorter to stay within its 32-bit
-offsets: equal, bit for bit, to the right-hand side of a small grid of which the large one is the repetition in x and
-y (away from the walls, where every cell's stencil is the small grid's).
+"""The FP32 right-hand side on planes so large that a block's reach in bytes leaves 32 bits (offsets in cells), and in
+cells too (fewer planes per thread): equal, bit for bit, to the right-hand side of a small grid of which the large one is
+the repetition in x and y (away from the walls, where every cell's stencil is the small grid's).
 """
 import ctypes
 
@@ -28,9 +28,10 @@ def _rhs(fields):
     return out
 
 
-@pytest.mark.parametrize("ny,nx,rep_y,rep_x,nz", [(100, 96, 82, 64, 11),      # 50.4 M cells: 8 planes
-                                                  (100, 96, 164, 64, 5),     # 100.8 M cells: 4 planes
-                                                  (100, 96, 164, 90, 5)])    # 141.7 M cells: 1 plane
+@pytest.mark.parametrize("ny,nx,rep_y,rep_x,nz", [(100, 96, 80, 63, 11),      # 48.4 M cells: bytes, 16 planes
+                                                  (100, 96, 82, 64, 11),      # 50.4 M: cells
+                                                  (100, 96, 164, 90, 6),      # 141.7 M
+                                                  (100, 96, 160, 167, 5)])    # 256.5 M: 8 planes
 def test_large_planes_equal_the_small_grid(ny, nx, rep_y, rep_x, nz):
     need = 4 * 15 * nz * ny * nx * rep_y * rep_x
     if torch.cuda.mem_get_info()[0] < 1.2 * need:
